@@ -1622,18 +1622,19 @@ int ovl_ncs_update(ovl_ctx *c, double *delta, double *total) {
         double *out = c->dev_small;
         if (su3(c)) {
             ovl::su3_launch_geodesic(c->u_old, c->U, 0.5, c->u_mid, c->e_mid, c->L, c->stream);
-            ovl::su3_launch_ncsdot(c->u_mid, c->e_mid, c->L, c->partial, out, c->stream);
-            ovl::su3_launch_ncsdot(c->u_old, c->e_mid, c->L, c->partial, out + 1, c->stream);
-            ovl::su3_launch_ncsdot(c->U, c->e_mid, c->L, c->partial, out + 2, c->stream);
+            ovl::su3_launch_ncsdot3(c->u_mid, c->u_old, c->U, c->e_mid, c->L, c->partial, out, c->stream);
         } else {
             ovl::launch_geodesic(c->u_old, c->U, 0.5, c->u_mid, c->e_mid, c->L, c->stream);
-            ovl::launch_ncsdot(c->u_mid, c->e_mid, c->L, c->partial, out, c->stream);
-            ovl::launch_ncsdot(c->u_old, c->e_mid, c->L, c->partial, out + 1, c->stream);
-            ovl::launch_ncsdot(c->U, c->e_mid, c->L, c->partial, out + 2, c->stream);
+            ovl::launch_ncsdot3(c->u_mid, c->u_old, c->U, c->e_mid, c->L, c->partial, out, c->stream);
         }
-        if ((rc = launched(c, 7, "ncs update"))) return rc;
+        if ((rc = launched(c, 3, "ncs update"))) return rc;
         OVL_CUDA(c, cudaMemcpyAsync(c->host_small, out, sizeof(double) * 3, cudaMemcpyDeviceToHost, c->stream));
-        OVL_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    // the links of this call are the next call's old ones; one wait for the values and the copy
+    OVL_CUDA(c, cudaMemcpyAsync(c->u_old, c->U, sizeof(double) * c->link_doubles * 3 * V, cudaMemcpyDeviceToDevice,
+                                c->stream));
+    OVL_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (c->have_u_old) {
         const double *h = c->host_small;
         double value = 0.0, weight = 0.0;
         value += 4.0 * h[0]; weight += 4.0;
@@ -1642,9 +1643,6 @@ int ovl_ncs_update(ovl_ctx *c, double *delta, double *total) {
         d = value / weight;
         c->ncs_total += d;
     }
-    OVL_CUDA(c, cudaMemcpyAsync(c->u_old, c->U, sizeof(double) * c->link_doubles * 3 * V, cudaMemcpyDeviceToDevice,
-                                c->stream));
-    OVL_CUDA(c, cudaStreamSynchronize(c->stream));
     c->have_u_old = true;
     if (delta) *delta = d;
     if (total) *total = c->ncs_total;

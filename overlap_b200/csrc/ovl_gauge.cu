@@ -7,6 +7,7 @@
 
 #include "ovl_device.cuh"
 #include "ovl_internal.h"
+#include "ovl_loops.cuh"
 #include "ovl_su3.cuh"
 
 namespace ovl {
@@ -131,73 +132,71 @@ void launch_update_efield(const double *U, double *E, double * /*unused*/, const
 }
 
 // ----------------------------------------------------------------- NCsDot --
-// Improved E_mu at x: -1/12, 7/12, 7/12, -1/12 of E_mu at x+mu, x, x-mu, x-2mu
-// transported to x (ChernSimonsOperators.cpp:379-401).
-__device__ void improved_e(const double *__restrict__ U, const double *__restrict__ E, const Lattice &L, int x, int y,
-                           int z, int mu, double out[3]) {
-    int c[3] = {x, y, z};
-    const int s0 = site_index(L, c[0], c[1], c[2]);
-    c[mu] += 1;
-    const int sp = site_index(L, c[0], c[1], c[2]);
-    c[mu] -= 2;
-    const int sm = site_index(L, c[0], c[1], c[2]);
-    c[mu] -= 1;
-    const int smm = site_index(L, c[0], c[1], c[2]);
-    const quat um = load_link(U, sm, mu);
-    adj3 Rp = adjoint(load_link(U, s0, mu));
-    adj3 Rm = adjoint(qdag(um));
-    adj3 Rmm = adjoint(qmul(qdag(um), qdag(load_link(U, smm, mu))));
-    const double *ep = E + 3 * (mu + 3 * sp), *e0 = E + 3 * (mu + 3 * s0);
-    const double *em = E + 3 * (mu + 3 * sm), *emm = E + 3 * (mu + 3 * smm);
-    for (int a = 0; a < 3; a++) {
-        double t = (7.0 / 12.0) * e0[a];
-        for (int b = 0; b < 3; b++)
-            t += -(1.0 / 12.0) * Rp.r[a][b] * ep[b] + (7.0 / 12.0) * Rm.r[a][b] * em[b] -
-                 (1.0 / 12.0) * Rmm.r[a][b] * emm[b];
-        out[a] = t;
-    }
-}
+// The improved E.B (ChernSimonsOperators.cpp:128-439): per site and direction
+// E_mu . B_mu with the improved E_mu and B_mu = -2 x the algebra part of 5/12 of
+// the four plaquettes and -1/24 of the eight rectangles of the plane orthogonal
+// to mu, all counter-clockwise and based at x (B_x from yz, B_y from zx, B_z
+// from xy).  Both are sums over four terms, so four lanes share a (site, mu):
+// lane q takes quadrant q of B and term q of E.  One thread per site and
+// direction walked 12 loops of 64 dependent products with dynamically indexed
+// coordinates in local memory and left most of the chip idle (1728 threads at
+// 12^3): three evaluations took 261 us there.  With four lanes and the common
+// sides of the loops shared, an observation (charges, Delta N_CS, bulk) at 12^3
+// with 4096 FP32 modes went from 749 to 466 us, the part of the charges unchanged.
+// blockIdx.y: the field set (links U[y] with the one E), so that the three
+// evaluations of a Delta N_CS step run in one launch.
+constexpr int kNcsThreads = 128;
 
-// Improved B for the (mu, nu) plane: 5/12 of the four plaquettes and -1/24 of
-// the eight 2x1 rectangles with x at a corner, all counter-clockwise and based
-// at x; B^a = 2 Re tr(i t^a avg) (ChernSimonsOperators.cpp:283-421).
-__device__ void improved_b(const double *__restrict__ U, const Lattice &L, int x, int y, int z, int mu, int nu,
-                           double out[3]) {
-    double avg[4] = {0.0, 0.0, 0.0, 0.0};
-    const int sg[4][2] = {{+1, +1}, {-1, +1}, {-1, -1}, {+1, -1}};
-    for (int q = 0; q < 4; q++) {
-        quat box = loop(U, L, x, y, z, mu, nu, sg[q][0], sg[q][1], 1, 1);
-        quat r1 = loop(U, L, x, y, z, mu, nu, sg[q][0], sg[q][1], 2, 1);
-        quat r2 = loop(U, L, x, y, z, mu, nu, sg[q][0], sg[q][1], 1, 2);
-        avg[0] += (5.0 / 12.0) * box.v0 - (1.0 / 24.0) * (r1.v0 + r2.v0);
-        avg[1] += (5.0 / 12.0) * box.v1 - (1.0 / 24.0) * (r1.v1 + r2.v1);
-        avg[2] += (5.0 / 12.0) * box.v2 - (1.0 / 24.0) * (r1.v2 + r2.v2);
-    }
-    for (int a = 0; a < 3; a++) out[a] = -2.0 * avg[a];
-}
+struct NcsSets {
+    const double *U[3];
+};
 
-__global__ void __launch_bounds__(kReduceThreads) ncsdot_kernel(const double *__restrict__ U, const double *__restrict__ E,
-                                                                 Lattice L, double *partial) {
+__global__ void __launch_bounds__(kNcsThreads) ncsdot_kernel(const NcsSets sets, const double *__restrict__ E, Lattice L,
+                                                             double *__restrict__ partial) {
     __shared__ double sh[32];
+    const double *__restrict__ U = sets.U[blockIdx.y];
     CompSum sum;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < L.V; s += gridDim.x * blockDim.x) {
-        int x, y, z;
-        site_coords(L, s, x, y, z);
-        const int plane[3][2] = {{1, 2}, {2, 0}, {0, 1}};  // B_x from yz, B_y from zx, B_z from xy
-        for (int mu = 0; mu < 3; mu++) {
-            double e[3], b[3];
-            improved_e(U, E, L, x, y, z, mu, e);
-            improved_b(U, L, x, y, z, plane[mu][0], plane[mu][1], b);
-            sum.add(e[0] * b[0] + e[1] * b[1] + e[2] * b[2]);
-        }
+    const long long items = 12LL * L.V;
+    const long long stride = (long long)gridDim.x * kNcsThreads;
+    // whole quadrant groups leave the loop together; the shuffles need every
+    // lane of the warp, so the warps that still hold an item run it padded
+    for (long long t0 = (long long)blockIdx.x * kNcsThreads + (threadIdx.x & ~31); t0 < items; t0 += stride) {
+        const long long t = t0 + (threadIdx.x & 31);
+        const bool live = t < items;
+        const int q = (int)(t & 3), sd = live ? (int)(t >> 2) : 0;
+        const int s = sd / 3, mu = sd % 3;
+        int c[3];
+        site_coords(L, s, c[0], c[1], c[2]);
+        int es;
+        quat V;
+        double w;
+        improved_e_term<Su2Ops>(U, L, s, c, mu, q, es, V, w);
+        const adj3 R = adjoint(V);
+        const double *ep = E + 3 * (mu + 3 * (size_t)es);
+        const double e0 = ep[0], e1 = ep[1], e2 = ep[2];
+        double e[3], b[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int a = 0; a < 3; a++) e[a] = w * (R.r[a][0] * e0 + R.r[a][1] * e1 + R.r[a][2] * e2);
+        const Quadrant quad(L, s, c, mu == 2 ? 0 : mu + 1, mu == 0 ? 2 : mu - 1, q);
+        quad.loops<Su2Ops>(U, [&](const quat &p, double f) {
+            b[0] += f * p.v0;
+            b[1] += f * p.v1;
+            b[2] += f * p.v2;
+        });
+        double eb = 0.0;
+#pragma unroll
+        for (int a = 0; a < 3; a++) eb += quad_sum(e[a]) * (-2.0 * quad_sum(b[a]));
+        if (live && q == 0) sum.add(eb);
     }
     double v[1] = {sum.value()};
     block_reduce<1, false>(v, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = v[0];
+    if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = v[0];
 }
 
 template <int NV, bool MAX_LAST>
 __global__ void finish_kernel(const double *__restrict__ partial, int n, double *out, double scale) {
+    partial += (size_t)blockIdx.x * n * NV;  // one CTA per result
+    out += blockIdx.x * NV;
     __shared__ double sh[32 * NV];
     double v[NV];
     CompSum t[NV];
@@ -219,23 +218,29 @@ static int reduce_blocks(int V) {
     return b < 1024 ? b : 1024;
 }
 
-size_t ncsdot_partial_doubles(const Lattice &L) { return (size_t)reduce_blocks(L.V); }
-
-void launch_ncsdot(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream) {
-    const int nb = reduce_blocks(L.V);
-    ncsdot_kernel<<<nb, kReduceThreads, 0, stream>>>(U, E, L, partial);
-    // NCsDot = E.B / (8 pi^2) (ChernSimonsDerivative.cpp:48)
-    finish_kernel<1, false><<<1, kReduceThreads, 0, stream>>>(partial, nb, out, 0.125 / (M_PI * M_PI));
+int ncsdot_blocks(const Lattice &L) {
+    const long long b = (12LL * L.V + kNcsThreads - 1) / kNcsThreads;
+    return b < kNcsMaxBlocks ? (int)b : kNcsMaxBlocks;
 }
 
-// One partial sum per block of kReduceThreads sites, for callers that provide
-// their own partial-sum storage of `blocks` doubles.
-int ncsdot_blocks_exact(const Lattice &L) { return (L.V + kReduceThreads - 1) / kReduceThreads; }
+size_t ncsdot_partial_doubles(const Lattice &L) { return (size_t)3 * ncsdot_blocks(L); }
 
-void launch_ncsdot_into(const double *U, const double *E, const Lattice &L, int blocks, double *partial, double *out,
+// out[k] = NCsDot of links U[k] and E, k < n (at most three).
+// NCsDot = E.B / (8 pi^2) (ChernSimonsDerivative.cpp:48)
+static void ncsdot_sets(const NcsSets &sets, int n, const double *E, const Lattice &L, double *partial, double *out,
                         cudaStream_t stream) {
-    ncsdot_kernel<<<blocks, kReduceThreads, 0, stream>>>(U, E, L, partial);
-    finish_kernel<1, false><<<1, kReduceThreads, 0, stream>>>(partial, blocks, out, 0.125 / (M_PI * M_PI));
+    const int nb = ncsdot_blocks(L);
+    ncsdot_kernel<<<dim3(nb, n), kNcsThreads, 0, stream>>>(sets, E, L, partial);
+    finish_kernel<1, false><<<n, kReduceThreads, 0, stream>>>(partial, nb, out, 0.125 / (M_PI * M_PI));
+}
+
+void launch_ncsdot(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream) {
+    ncsdot_sets(NcsSets{{U, U, U}}, 1, E, L, partial, out, stream);
+}
+
+void launch_ncsdot3(const double *U0, const double *U1, const double *U2, const double *E, const Lattice &L,
+                    double *partial, double *out3, cudaStream_t stream) {
+    ncsdot_sets(NcsSets{{U0, U1, U2}}, 3, E, L, partial, out3, stream);
 }
 
 // ----------------------------------------------------- geodesic interpolation --

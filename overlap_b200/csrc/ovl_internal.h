@@ -86,9 +86,12 @@ void launch_update_efield(const double *U, double *E, double *dE, const Lattice 
 // doubles; out: device array of the result size.
 size_t ncsdot_partial_doubles(const Lattice &L);
 void launch_ncsdot(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream);
-int ncsdot_blocks_exact(const Lattice &L);
-void launch_ncsdot_into(const double *U, const double *E, const Lattice &L, int blocks, double *partial, double *out,
-                        cudaStream_t stream);
+// NCsDot of three link fields with one E (partial holds ncsdot_partial_doubles);
+// a launch writes ncsdot_blocks(L) <= kNcsMaxBlocks partial sums per link field.
+constexpr int kNcsMaxBlocks = 1024;
+int ncsdot_blocks(const Lattice &L);
+void launch_ncsdot3(const double *U0, const double *U1, const double *U2, const double *E, const Lattice &L,
+                    double *partial, double *out3, cudaStream_t stream);
 // Overlap eigenmodes in the U(1) background (ovl_eigen.cu): modes
 // [first_mode, first_mode + count) of the dense, exactly diagonalised h_ov
 // into psi_ref / mid_ref (reference layout, device); 0 on success, 1 library
@@ -323,6 +326,8 @@ void su3_launch_charges(const double *U, const double *u1, const void *psi, cons
 size_t su3_reduce_partial_doubles(const Lattice &L);
 void su3_launch_ncsdot(const double *U, const double *E, const Lattice &L, double *partial, double *out,
                        cudaStream_t stream);
+void su3_launch_ncsdot3(const double *U0, const double *U1, const double *U2, const double *E, const Lattice &L,
+                        double *partial, double *out3, cudaStream_t stream);
 void su3_launch_geodesic(const double *Uold, const double *Unew, double c, double *Umid, double *Emid, const Lattice &L,
                          cudaStream_t stream);
 void su3_launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out,

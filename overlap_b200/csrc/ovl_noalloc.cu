@@ -9,9 +9,10 @@
 // and only needs the reduction.
 //
 // Scratch: the partial sums live in the file-scope device array below, one
-// double per block of 256 sites, at most kNoAllocPartials of them, so the
-// entry point accepts lattices of up to kNoAllocPartials * 256 = 262144 sites
-// (64^3) and rejects larger ones with OVL_E_ARG.  The array is 8 KiB of device
+// double per CTA of the reduction, at most kNoAllocPartials of them
+// (ncsdot_blocks); the entry point accepts lattices of up to
+// kNoAllocPartials * 256 = 262144 sites (64^3) and rejects larger ones with
+// OVL_E_ARG.  The array is 8 KiB of device
 // memory that every GPU loading this library holds until the process exits.
 // Every call overwrites exactly the partial sums it then reads, so nothing has
 // to start at zero; all calls share the one array, so calls whose work
@@ -65,11 +66,11 @@ extern "C" int ovl_ncsdot_noalloc(const double *links, const double *efield, int
         partials = g_partials_addr[dev];
     }
     const ovl::Lattice L{N0, N1, N2, (int)V};
-    const int blocks = ovl::ncsdot_blocks_exact(L);
     // the runtime's last error before and after the launches: a change is this
     // call's failure; an error that was already there belongs to earlier work
     const cudaError_t before = cudaPeekAtLastError();
-    ovl::launch_ncsdot_into(links, efield, L, blocks, partials, out, reinterpret_cast<cudaStream_t>(stream));
+    static_assert(kNoAllocPartials >= ovl::kNcsMaxBlocks, "one partial sum per CTA");
+    ovl::launch_ncsdot(links, efield, L, partials, out, reinterpret_cast<cudaStream_t>(stream));
     const cudaError_t after = cudaPeekAtLastError();
     if (after != before) {
         cudaGetLastError();

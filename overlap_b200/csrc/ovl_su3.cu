@@ -9,6 +9,7 @@
 #include <cmath>
 
 #include "ovl_internal.h"
+#include "ovl_loops.cuh"
 #include "ovl_su3.cuh"
 #include "ovl_su3_packed.cuh"
 
@@ -472,6 +473,8 @@ void su3_launch_currents(const double *U, const double *u1, const void *psi, con
 // sum per thread, then a tree), scaled.
 template <int NV>
 __global__ void su3_sum_rows_kernel(const double *__restrict__ partial, int n, double scale, double *__restrict__ out) {
+    partial += (size_t)blockIdx.x * n * NV;  // one CTA per result
+    out += blockIdx.x * NV;
     __shared__ double sh[256][NV];
     CompSum t[NV];
     for (int i = threadIdx.x; i < n; i += blockDim.x)
@@ -548,66 +551,73 @@ __device__ inline double block_sum(double v, double *sh) {
     return t;
 }
 
-// Improved E.B (ChernSimonsOperators.cpp:128-439; improved_e / improved_b of
-// ovl_gauge.cu), one thread per (site, direction): E_mu . B_mu, B_mu from the
-// plane orthogonal to mu; CTA partial sums.
+// Improved E.B (ChernSimonsOperators.cpp:128-439): four lanes per (site,
+// direction), lane q with quadrant q of B_mu and term q of E_mu, as
+// ncsdot_kernel of ovl_gauge.cu; blockIdx.y: the link field.
+struct NcsSets3 {
+    const double *U[3];
+};
+
 __global__ void __launch_bounds__(kReduce3Threads)
-    su3_ncsdot_kernel(const double *__restrict__ U, const double *__restrict__ E, Lattice L, double *partial) {
+    su3_ncsdot_kernel(const NcsSets3 sets, const double *__restrict__ E, Lattice L, double *__restrict__ partial) {
     __shared__ double sh[32];
-    double v = 0.0;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < 3 * L.V) {
-        const int s = t / 3, mu = t % 3;
-        int x, y, z;
-        site_coords(L, s, x, y, z);
-        const int plane[3][2] = {{1, 2}, {2, 0}, {0, 1}};
-        // improved E_mu: -1/12, 7/12, 7/12, -1/12 of E_mu at x+mu, x, x-mu, x-2mu transported to x
-        int c[3] = {x, y, z};
-        c[mu] += 1;
-        const int sp = site_index(L, c[0], c[1], c[2]);
-        c[mu] -= 2;
-        const int sm = site_index(L, c[0], c[1], c[2]);
-        c[mu] -= 1;
-        const int smm = site_index(L, c[0], c[1], c[2]);
-        const cmat3<double> umd = m3_dag(load_su3(U, sm, mu));
-        double e[8], w[8];
-        for (int a = 0; a < 8; a++) e[a] = (7.0 / 12.0) * E[a + 8 * (mu + 3 * s)];
-        su3_transport(load_su3(U, s, mu), E + 8 * (mu + 3 * sp), w);
-        for (int a = 0; a < 8; a++) e[a] -= (1.0 / 12.0) * w[a];
-        su3_transport(umd, E + 8 * (mu + 3 * sm), w);
-        for (int a = 0; a < 8; a++) e[a] += (7.0 / 12.0) * w[a];
-        su3_transport(m3_mul(umd, m3_dag(load_su3(U, smm, mu))), E + 8 * (mu + 3 * smm), w);
-        for (int a = 0; a < 8; a++) e[a] -= (1.0 / 12.0) * w[a];
-        // improved B: 5/12 of the four plaquettes, -1/24 of the eight 2x1 rectangles
-        const int pm = plane[mu][0], pn = plane[mu][1];
-        cmat3<double> avg;
-        for (int i = 0; i < 3; i++)
-            for (int j = 0; j < 3; j++) avg.m[i][j] = mk<double>(0.0, 0.0);
-        const int sg[4][2] = {{+1, +1}, {-1, +1}, {-1, -1}, {+1, -1}};
-        for (int q = 0; q < 4; q++) {
-            const cmat3<double> box = su3_loop(U, L, x, y, z, pm, pn, sg[q][0], sg[q][1], 1, 1);
-            const cmat3<double> r1 = su3_loop(U, L, x, y, z, pm, pn, sg[q][0], sg[q][1], 2, 1);
-            const cmat3<double> r2 = su3_loop(U, L, x, y, z, pm, pn, sg[q][0], sg[q][1], 1, 2);
-            for (int i = 0; i < 3; i++)
-                for (int j = 0; j < 3; j++)
-                    avg.m[i][j] = avg.m[i][j] + (5.0 / 12.0) * box.m[i][j] - (1.0 / 24.0) * (r1.m[i][j] + r2.m[i][j]);
+    const double *__restrict__ U = sets.U[blockIdx.y];
+    CompSum sum;
+    const long long items = 12LL * L.V, stride = (long long)gridDim.x * kReduce3Threads;
+    for (long long t0 = (long long)blockIdx.x * kReduce3Threads + (threadIdx.x & ~31); t0 < items; t0 += stride) {
+        const long long t = t0 + (threadIdx.x & 31);
+        const bool live = t < items;  // padded lanes repeat site 0: the shuffles need the whole warp
+        const int q = (int)(t & 3), sd = live ? (int)(t >> 2) : 0;
+        const int s = sd / 3, mu = sd % 3;
+        int c[3];
+        site_coords(L, s, c[0], c[1], c[2]);
+        double e[8], b[8];
+        {
+            int es;
+            cmat3<double> V;
+            double w;
+            improved_e_term<Su3Ops>(U, L, s, c, mu, q, es, V, w);
+            su3_transport(V, E + 8 * (mu + 3 * (size_t)es), e);
+#pragma unroll
+            for (int a = 0; a < 8; a++) e[a] *= w;
         }
-        double b[8];
-        su3_retr_ita(avg, b);
-        for (int a = 0; a < 8; a++) v += e[a] * 2.0 * b[a];
+#pragma unroll
+        for (int a = 0; a < 8; a++) b[a] = 0.0;
+        const Quadrant quad(L, s, c, mu == 2 ? 0 : mu + 1, mu == 0 ? 2 : mu - 1, q);
+        quad.loops<Su3Ops>(U, [&](const cmat3<double> &p, double f) {
+            double g[8];
+            su3_retr_ita(p, g);
+#pragma unroll
+            for (int a = 0; a < 8; a++) b[a] += f * g[a];
+        });
+        double eb = 0.0;
+#pragma unroll
+        for (int a = 0; a < 8; a++) eb += quad_sum(e[a]) * (2.0 * quad_sum(b[a]));
+        if (live && q == 0) sum.add(eb);
     }
-    const double tot = block_sum(v, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = tot;
+    const double tot = block_sum(sum.value(), sh);
+    if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
 }
 
 size_t su3_reduce_partial_doubles(const Lattice &L) {
     return (size_t)std::max(11 * ((L.V + kReduce3Threads - 1) / kReduce3Threads), 1);
 }
 
+// partial holds ncsdot_partial_doubles
+static void su3_ncsdot_sets(const NcsSets3 &sets, int n, const double *E, const Lattice &L, double *partial,
+                            double *out, cudaStream_t s) {
+    const int nb = ncsdot_blocks(L);
+    su3_ncsdot_kernel<<<dim3(nb, n), kReduce3Threads, 0, s>>>(sets, E, L, partial);
+    su3_sum_rows_kernel<1><<<n, 256, 0, s>>>(partial, nb, 0.125 / (M_PI * M_PI), out);
+}
+
 void su3_launch_ncsdot(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t s) {
-    const int nb = (3 * L.V + kReduce3Threads - 1) / kReduce3Threads;
-    su3_ncsdot_kernel<<<nb, kReduce3Threads, 0, s>>>(U, E, L, partial);
-    su3_sum_rows_kernel<1><<<1, 256, 0, s>>>(partial, nb, 0.125 / (M_PI * M_PI), out);
+    su3_ncsdot_sets(NcsSets3{{U, U, U}}, 1, E, L, partial, out, s);
+}
+
+void su3_launch_ncsdot3(const double *U0, const double *U1, const double *U2, const double *E, const Lattice &L,
+                        double *partial, double *out3, cudaStream_t s) {
+    su3_ncsdot_sets(NcsSets3{{U0, U1, U2}}, 3, E, L, partial, out3, s);
 }
 
 // ---------------------------------------------------- geodesic interpolation --
