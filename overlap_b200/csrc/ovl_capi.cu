@@ -816,7 +816,7 @@ int ovl_create(const ovl_params *p, ovl_ctx **out) {
     c->partial_doubles = std::max({ovl::currents_partial_doubles(c->L, c->n_mb), ovl::ncsdot_partial_doubles(c->L),
                                    ovl::bulk_partial_doubles(c->L), ovl::charges_partial_doubles(c->L, c->n_mb),
                                    ovl::force_partial_doubles(c->L, c->n_mb), ovl::energy_partial_doubles(),
-                                   ovl::gauss_partial_doubles(c->L), ovl::su3_charges_partial_doubles(c->L, c->n_mb),
+                                   ovl::gauss_partial_doubles(c->L),
                                    ovl::su3_reduce_partial_doubles(c->L),
                                    ovl::su3_force_partial_doubles(c->L, c->n_mb)});
     if ((rc = alloc((void **)&c->partial, sizeof(double) * c->partial_doubles, "reduction scratch")) ||

@@ -256,219 +256,6 @@ void su3_chebyshev_apply(ChebyshevWork &w, const Su3Links &lk, const void *src, 
                              stream, launches);
 }
 
-// ---------------------------------------------------------------- charges --
-// Lattice sums {sum jV^0, N_5, sum PS, sum WA} (Currents.cpp:7-394 for three
-// colours; the bilinears of charges_kernel in ovl_modes.cu).  Bilinears in
-// FP64 for every mode precision.  One CTA per (group of kSites3 sites, slice
-// of mode blocks); partial sums per CTA, summed in a fixed order.
-constexpr int kCharge3Groups = 8;  // mode-block slices per site group
-
-template <typename T>
-__global__ void __launch_bounds__(kModeBlock *kSites3)
-    su3_charges_kernel(const double *__restrict__ U, const double2 *__restrict__ u1, const cpx<T> *__restrict__ psi,
-                       Lattice L, int n_mb, int n_modes, int first_mode, double r, double *__restrict__ partial) {
-    __shared__ double sh[kSites3][4];
-    const int lane = threadIdx.x;
-    const int site = blockIdx.x * kSites3 + threadIdx.y;
-    CompSum sum[4];
-    if (site < L.V) {
-        int x, y, z;
-        site_coords(L, site, x, y, z);
-        int nb[3];
-        for (int mu = 0; mu < 3; mu++) {
-            int c[3] = {x, y, z};
-            c[mu] += 1;
-            nb[mu] = site_index(L, c[0], c[1], c[2]);
-        }
-        const Links3<false, true> lk1{U, u1, L.N0 * L.N1};
-        const Links3<false, false> lk0{U, nullptr, L.N0 * L.N1};
-        cmat3<double> M[3];
-        for (int mu = 0; mu < 3; mu++) M[mu] = u1 ? lk1.get<double>(site, mu) : lk0.get<double>(site, mu);
-        for (int mb = blockIdx.y; mb < n_mb; mb += gridDim.y) {
-            const int mode = mb * kModeBlock + lane;
-            const double w = mode >= n_modes ? 0.0 : (((first_mode + mode) & 1) == 0 ? 1.0 : -1.0);
-            cpx<double> f[3][kSpin];
-            const cpx<T> *p = psi + field_index3(L.V, mb, site, 0, lane);
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-#pragma unroll
-                for (int a = 0; a < kSpin; a++) {
-                    const cpx<T> v = ld(p + (c * kSpin + a) * kModeBlock);
-                    f[c][a] = mk<double>((double)v.re, (double)v.im);
-                }
-            double nv = 0.0;
-            cpx<double> zz = mk<double>(0.0, 0.0);
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-#pragma unroll
-                for (int a = 0; a < kSpin; a++) nv += f[c][a].re * f[c][a].re + f[c][a].im * f[c][a].im;
-                zz = zz + cdot(f[c][0], f[c][2]) + cdot(f[c][1], f[c][3]);
-            }
-            double hop = 0.0;
-            for (int mu = 0; mu < 3; mu++) {
-                const cpx<T> *q = psi + field_index3(L.V, mb, nb[mu], 0, lane);
-                cpx<double> ht[3][kSpin];
-#pragma unroll
-                for (int c = 0; c < 3; c++)
-#pragma unroll
-                    for (int a = 0; a < kSpin; a++) {
-                        const cpx<T> v = ld(q + (c * kSpin + a) * kModeBlock);
-                        ht[c][a] = mk<double>((double)v.re, (double)v.im);
-                    }
-                cpx<double> b = mk<double>(0.0, 0.0);
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    cpx<double> chi[kSpin];
-#pragma unroll
-                    for (int a = 0; a < kSpin; a++)
-                        chi[a] = M[mu].m[i][0] * ht[0][a] + M[mu].m[i][1] * ht[1][a] + M[mu].m[i][2] * ht[2][a];
-                    b = b + cdot(f[i][0], chi[2]) + cdot(f[i][1], chi[3]) - cdot(f[i][2], chi[0]) - cdot(f[i][3], chi[1]);
-                }
-                hop += b.im;
-            }
-            sum[0].add(w * nv);
-            sum[1].add(w * 2.0 * zz.re);
-            sum[2].add(w * -2.0 * zz.im);
-            sum[3].add(w * (r * (-12.0 * zz.im + 2.0 * hop)));
-        }
-    }
-    double acc[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) acc[k] = sum[k].value();
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        double t = acc[k];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        acc[k] = t;
-    }
-    if (lane == 0)
-        for (int k = 0; k < 4; k++) sh[threadIdx.y][k] = acc[k];
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        double *q = partial + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 4;
-        for (int k = 0; k < 4; k++) {
-            double t = 0.0;
-            for (int j = 0; j < kSites3; j++) t += sh[j][k];
-            q[k] = t;
-        }
-    }
-}
-
-// Per-site Wilson currents for three colours (currents_kernel of ovl_modes.cu,
-// Currents.cpp:7-394): per site the 18 vacuum-weighted mode sums jV^0..3,
-// jA^0..3, jVw^1..3, jAw^1..3, PS, WA (slots as kCurrentsPerSite), per group of
-// mode blocks into partial[g][site][18]; launch_currents_finish adds the groups.
-template <typename T>
-__device__ __forceinline__ cpx<double> colour_bilinear3(const mono &G, const cpx<double> (&f)[3][kSpin],
-                                                        const cpx<double> (&h)[3][kSpin]) {
-    return bilinear<double>(G, f[0], h[0]) + bilinear<double>(G, f[1], h[1]) + bilinear<double>(G, f[2], h[2]);
-}
-
-template <typename T>
-__device__ __forceinline__ void load_site3(const cpx<T> *__restrict__ psi, int V, int mb, int site, int lane,
-                                           cpx<double> (&f)[3][kSpin]) {
-    const cpx<T> *p = psi + field_index3(V, mb, site, 0, lane);
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int a = 0; a < kSpin; a++) {
-            const cpx<T> v = ld(p + (c * kSpin + a) * kModeBlock);
-            f[c][a] = mk<double>((double)v.re, (double)v.im);
-        }
-}
-
-template <typename T, bool U1>
-__global__ void __launch_bounds__(kModeBlock *kSites3)
-    su3_currents_kernel(const double *__restrict__ U, const double *__restrict__ u1, const cpx<T> *__restrict__ psi,
-                        Lattice L, int n_mb, int n_modes, int first_mode, int groups, double r,
-                        double *__restrict__ partial) {
-    constexpr mono G1 = {{0, 1, 2, 3}, {0, 0, 0, 0}};
-    constexpr mono G5 = kGamma5;
-    constexpr mono G05 = mono_mul(kGamma0, kGamma5);
-    constexpr mono G0 = kGamma0;
-    constexpr mono GV[3] = {mono_mul(kGamma0, kGammaX), mono_mul(kGamma0, kGammaY), mono_mul(kGamma0, kGammaZ)};
-    constexpr mono GA[3] = {mono_mul(GV[0], kGamma5), mono_mul(GV[1], kGamma5), mono_mul(GV[2], kGamma5)};
-    const int lane = threadIdx.x;
-    const int site = blockIdx.x * kSites3 + threadIdx.y;
-    const int g = blockIdx.y;
-    if (site >= L.V) return;  // whole warps exit together
-    int x, y, z;
-    site_coords(L, site, x, y, z);
-    const int V = L.V;
-    int nb[3][2];
-    for (int mu = 0; mu < 3; mu++) {
-        int cp[3] = {x, y, z}, cm[3] = {x, y, z};
-        cp[mu] += 1;
-        cm[mu] -= 1;
-        nb[mu][0] = site_index(L, cp[0], cp[1], cp[2]);
-        nb[mu][1] = site_index(L, cm[0], cm[1], cm[2]);
-    }
-    const Links3<false, U1> lk{U, u1, L.N0 * L.N1};
-    CompSum acc[kCurrentsPerSite];
-    for (int mb = g; mb < n_mb; mb += groups) {
-        const int mode = mb * kModeBlock + lane;
-        const double w = mode >= n_modes ? 0.0 : (((first_mode + mode) & 1) == 0 ? 1.0 : -1.0);
-        cpx<double> f[3][kSpin];
-        load_site3(psi, V, mb, site, lane, f);
-        double v[kCurrentsPerSite];
-#pragma unroll
-        for (int k = 0; k < kCurrentsPerSite; k++) v[k] = 0.0;
-        v[0] = colour_bilinear3<T>(G1, f, f).re;
-        v[4] = colour_bilinear3<T>(G5, f, f).re;
-        const cpx<double> b05 = colour_bilinear3<T>(G05, f, f);
-        v[16] = -b05.im;
-        double wa = -6.0 * r * b05.im;
-        for (int mu = 0; mu < 3; mu++) {
-            cpx<double> h[3][kSpin], chi[3][kSpin];
-            load_site3(psi, V, mb, nb[mu][0], lane, h);  // forward: chi = U_mu(x) psi(x+mu)
-            {
-                const cmat3<double> M = lk.template get<double>(site, mu);
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int a = 0; a < kSpin; a++)
-                        chi[i][a] = M.m[i][0] * h[0][a] + M.m[i][1] * h[1][a] + M.m[i][2] * h[2][a];
-            }
-            v[1 + mu] = colour_bilinear3<T>(GV[mu], f, chi).re;
-            v[5 + mu] = colour_bilinear3<T>(GA[mu], f, chi).re;
-            v[9 + mu] = r * colour_bilinear3<T>(G0, f, chi).im;
-            const double aw = r * colour_bilinear3<T>(G05, f, chi).im;
-            v[13 + mu] = aw;
-            wa += aw;
-            load_site3(psi, V, mb, nb[mu][1], lane, h);  // backward: chi = U_mu(x-mu)^+ psi(x-mu)
-            {
-                const cmat3<double> M = lk.template get<double>(nb[mu][1], mu);
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int a = 0; a < kSpin; a++)
-                        chi[i][a] = cdot(M.m[0][i], h[0][a]) + cdot(M.m[1][i], h[1][a]) + cdot(M.m[2][i], h[2][a]);
-            }
-            wa += r * colour_bilinear3<T>(G05, f, chi).im;
-        }
-        v[17] = wa;
-#pragma unroll
-        for (int k = 0; k < kCurrentsPerSite; k++) acc[k].add(w * v[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < kCurrentsPerSite; k++) {
-        double t = acc[k].value();
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        if (lane == 0) partial[((size_t)g * V + site) * kCurrentsPerSite + k] = t;
-    }
-}
-
-template <typename T>
-void su3_launch_currents(const double *U, const double *u1, const void *psi, const Lattice &L, int n_mb, int n_modes,
-                         int first_mode, double r, double *partial, double *per_site, cudaStream_t s) {
-    const int groups = currents_groups(n_mb);
-    const dim3 block(kModeBlock, kSites3), grid((L.V + kSites3 - 1) / kSites3, groups);
-    const cpx<T> *p = reinterpret_cast<const cpx<T> *>(psi);
-    if (u1) su3_currents_kernel<T, true><<<grid, block, 0, s>>>(U, u1, p, L, n_mb, n_modes, first_mode, groups, r, partial);
-    else su3_currents_kernel<T, false><<<grid, block, 0, s>>>(U, u1, p, L, n_mb, n_modes, first_mode, groups, r, partial);
-    launch_currents_finish(partial, groups, L, per_site, s);
-}
-
 // Sums `n` partial rows of `nv` values in a fixed order (one CTA: a strided
 // sum per thread, then a tree), scaled.
 template <int NV>
@@ -488,20 +275,6 @@ __global__ void su3_sum_rows_kernel(const double *__restrict__ partial, int n, d
     }
     if (threadIdx.x == 0)
         for (int k = 0; k < NV; k++) out[k] = scale * sh[0][k];
-}
-
-size_t su3_charges_partial_doubles(const Lattice &L, int n_mb) {
-    return (size_t)4 * ((L.V + kSites3 - 1) / kSites3) * std::min(n_mb, kCharge3Groups);
-}
-
-template <typename T>
-void su3_launch_charges(const double *U, const double *u1, const void *psi, const Lattice &L, int n_mb, int n_modes,
-                        int first_mode, double r, double *partial, double *out4, cudaStream_t s) {
-    const dim3 block(kModeBlock, kSites3), grid((L.V + kSites3 - 1) / kSites3, std::min(n_mb, kCharge3Groups));
-    su3_charges_kernel<T><<<grid, block, 0, s>>>(U, reinterpret_cast<const double2 *>(u1),
-                                                 reinterpret_cast<const cpx<T> *>(psi), L, n_mb, n_modes, first_mode, r,
-                                                 partial);
-    su3_sum_rows_kernel<4><<<1, 256, 0, s>>>(partial, (int)(grid.x * grid.y), 1.0 / (2.0 * L.V), out4);
 }
 
 // ----------------------------------------------------------- Wilson loops --
@@ -1118,10 +891,6 @@ void su3_launch_links_to_f32(const double *U, float *U32, const Lattice &L, cuda
     template void su3_chebyshev_apply<T>(ChebyshevWork &, const Su3Links &, const void *, void *, const Lattice &, int, \
                                          const double *, int, double, double, double, double, double, double, bool, int, \
                                          cudaStream_t, uint64_t *);                                                      \
-    template void su3_launch_charges<T>(const double *, const double *, const void *, const Lattice &, int, int, int,   \
-                                        double, double *, double *, cudaStream_t);                                      \
-    template void su3_launch_currents<T>(const double *, const double *, const void *, const Lattice &, int, int, int,  \
-                                         double, double *, double *, cudaStream_t);                                     \
     template void su3_launch_color_force<T>(const double *, const double *, const void *, const Lattice &, int, int,    \
                                             int, double *, double *, double *, double, cudaStream_t);                   \
     template void su3_launch_fermion_energy<T>(const void *, const void *, const Lattice &, int, int, int, double *,    \
