@@ -858,20 +858,24 @@ int ovl_create(const ovl_params *p, ovl_ctx **out) {
         ovl::OverlapWork &w = c->ow;
         const size_t mp = (size_t)c->n_mb * ovl::kModeBlock, np = (size_t)p->zolo_poles;
         if ((rc = alloc(&w.r, field_bytes, "CG residual")) || (rc = alloc(&w.q, field_bytes, "CG direction image")) ||
-            (rc = alloc(&w.t, field_bytes, "CG temporary")) || (rc = alloc(&w.x, field_bytes * np, "shifted solutions")) ||
+            (rc = alloc(&w.t, field_bytes, "CG temporary")) || (rc = alloc(&w.x, field_bytes, "shifted solutions")) ||
             (rc = alloc(&w.p, field_bytes * np, "shifted directions")) ||
-            (rc = alloc((void **)&w.part, sizeof(double) * ovl::kDotChunks * mp, "dot partials")) ||
-            (rc = alloc((void **)&w.rnorm, sizeof(double) * mp * 5, "CG scalars")) ||
+            (rc = alloc((void **)&w.part, sizeof(double) * ovl::cg_partial_chunks(c->L) * mp, "dot partials")) ||
+            (rc = alloc((void **)&w.rnorm, sizeof(double) * mp * 3, "CG scalars")) ||
             (rc = alloc((void **)&w.alpha, sizeof(double) * mp * np * 4, "shift scalars")) ||
-            (rc = alloc((void **)&w.active, sizeof(int) * (mp * 3 + 1), "CG flags")) ||
+            (rc = alloc((void **)&w.active, sizeof(int) * (mp * 5 + 2), "CG flags")) ||
             (rc = alloc((void **)&w.dz, sizeof(double) * 2 * ovl::kMaxPoles, "Zolotarev coefficients")))
             return bail(rc);
-        w.bnorm = w.rnorm + mp; w.betam = w.rnorm + 2 * mp; w.pap = w.rnorm + 3 * mp; w.rr = w.rnorm + 4 * mp;
+        w.bnorm = w.rnorm + mp; w.betam = w.rnorm + 2 * mp;
         w.beta = w.alpha + mp * np; w.z = w.alpha + 2 * mp * np; w.g = w.alpha + 3 * mp * np;
-        w.next = w.active + mp; w.iters = w.active + 2 * mp; w.count = w.active + 3 * mp;
+        w.next = w.active + mp; w.iters = w.active + 2 * mp; w.kact = w.active + 3 * mp;
+        w.knext = w.active + 4 * mp; w.count = w.active + 5 * mp;
         w.bz = w.dz + ovl::kMaxPoles;
-        if (cudaMallocHost(&w.host_count, sizeof(int)) != cudaSuccess)
+        if (cudaMallocHost(&w.host_count, sizeof(int) * 2) != cudaSuccess)
             return bail(fail(c, OVL_E_OOM, "ovl_create: pinned host allocation failed"));
+        for (cudaEvent_t &e : w.counted)
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+                return bail(fail(c, OVL_E_CUDA, "ovl_create: event creation failed"));
     }
     cudaMemsetAsync(c->psi, 0, field_bytes, c->stream);
     cudaMemsetAsync(c->psimid, 0, field_bytes, c->stream);
@@ -899,6 +903,8 @@ int ovl_destroy(ovl_ctx *c) {
                     c->cw.b0, c->cw.b1, c->cw.b2, c->cw.w, c->U32, c->u1_32, c->U_b, c->U32_b,
                     c->psi_lo, c->psimid_lo, c->aux_src_lo, c->aux_dst_lo, c->obs_partial, c->obs_scratch, c->pipe};
     if (c->ow.host_count) cudaFreeHost(c->ow.host_count);
+    for (cudaEvent_t e : c->ow.counted)
+        if (e) cudaEventDestroy(e);
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (c->host_small) cudaFreeHost(c->host_small);

@@ -235,7 +235,9 @@ void launch_blocks_to_ref(const void *blocks, double *ref, const Lattice &L, int
 double zolotarev(double amin, double amax, double errtol, int npoles, double *b, double *d);
 
 constexpr int kMaxPoles = 64;
-constexpr int kDotChunks = 64;  // site chunks per mode in the two-stage dot products
+constexpr int kDotChunks = 64;  // at most, chunks of rows in the CG's vector kernels
+int cg_square_chunks(const Lattice &L);
+size_t cg_partial_chunks(const Lattice &L);
 
 struct OverlapCoeffs {
     int npoles;
@@ -246,13 +248,15 @@ struct OverlapCoeffs {
 
 // Device work space of the batched multi-shift CG (all FP64, mode-block layout).
 struct OverlapWork {
-    void *r = nullptr, *q = nullptr, *t = nullptr;  // one field each
-    void *x = nullptr, *p = nullptr;                // npoles fields each
-    double *part = nullptr;                         // kDotChunks x modes
-    double *rnorm = nullptr, *bnorm = nullptr, *betam = nullptr, *pap = nullptr, *rr = nullptr;
+    void *r = nullptr, *q = nullptr, *t = nullptr, *x = nullptr;  // one field each (x: chi)
+    void *p = nullptr;                              // npoles fields
+    double *part = nullptr;                         // cg_partial_chunks x modes
+    double *rnorm = nullptr, *bnorm = nullptr, *betam = nullptr;
     double *alpha = nullptr, *beta = nullptr, *z = nullptr, *g = nullptr;  // npoles x modes
-    int *active = nullptr, *next = nullptr, *iters = nullptr, *count = nullptr;
-    int *host_count = nullptr;                      // pinned
+    int *active = nullptr, *next = nullptr, *iters = nullptr, *kact = nullptr, *knext = nullptr;
+    int *count = nullptr;                           // two slots, by the iteration's parity
+    int *host_count = nullptr;                      // pinned, two slots
+    cudaEvent_t counted[2] = {nullptr, nullptr};    // host_count[slot] has arrived
     double *dz = nullptr, *bz = nullptr;            // npoles
 };
 
