@@ -287,29 +287,13 @@ __global__ void __launch_bounds__(kRitzThreads)
     }
 }
 
-// The rotation of x in the (x, p) plane (RitzSolver.cpp:176-222), from slot 0:
-// pz = Re <p, z>, xz = Re <x, z>.  Then <x, x>, <x, y> -> slot 1.
-template <int NCOMP>
-__global__ void __launch_bounds__(kRitzThreads)
-    ritz_rotate_kernel(double2 *x, double2 *y, const double2 *__restrict__ p, const double2 *__restrict__ z, int V,
-                       RitzScalars *st, RitzArgs a, double *part) {
-    const int prob = blockIdx.y, site = blockIdx.x * kRitzThreads + threadIdx.x;
-    if (ritz_stopped(st, prob)) return;
-    double r[kRitzParts];
-    reduce_partials(part_of(part, 0, prob, a.nblocks), a.nblocks, 4, r);
-    const double pz = r[0], ccc = r[2];
-    const double xy_re = st[prob].xy_re, xy_im = st[prob].xy_im;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        st[prob].oxy_re = xy_re;
-        st[prob].oxy_im = xy_im;
-        st[prob].ittot += 1;
-    }
-    const double amb = xy_re - pz;  // Re(xy - Re <p, z>)
+// cos and sin of the rotation of x in the (x, p) plane from amb = Re(xy - Re
+// <p, z>) and ccc = Re <x, z> (RitzSolver.cpp:176-222).
+__device__ __forceinline__ void ritz_rotation(double amb, double ccc, double &ct, double &sn) {
     const double cox = 2.0 * ccc / amb;
     const double sig1 = -copysign(1.0, amb);
     const double sig2 = copysign(1.0, cox) * sig1;
     const double c2 = cox * cox;
-    double ct, sn;
     if (c2 <= 1.0e-3) {
         // the reference's series for the rotation, constants as there (:197-200)
         const double sqp = 1.0 - 0.125 * c2 + 0.0859375 * c2 * c2 - 0.0673828125 * c2 * c2 * c2 +
@@ -330,6 +314,27 @@ __global__ void __launch_bounds__(kRitzThreads)
         ct = sqrt((1.0 + sox) * 0.5);
         sn = sqrt((1.0 - sox) * 0.5) * sig2;
     }
+}
+
+// The rotation of x in the (x, p) plane (RitzSolver.cpp:176-222), from slot 0:
+// pz = Re <p, z>, xz = Re <x, z>.  Then <x, x>, <x, y> -> slot 1.
+template <int NCOMP>
+__global__ void __launch_bounds__(kRitzThreads)
+    ritz_rotate_kernel(double2 *x, double2 *y, const double2 *__restrict__ p, const double2 *__restrict__ z, int V,
+                       RitzScalars *st, RitzArgs a, double *part) {
+    const int prob = blockIdx.y, site = blockIdx.x * kRitzThreads + threadIdx.x;
+    if (ritz_stopped(st, prob)) return;
+    double r[kRitzParts];
+    reduce_partials(part_of(part, 0, prob, a.nblocks), a.nblocks, 4, r);
+    const double pz = r[0], ccc = r[2];
+    const double xy_re = st[prob].xy_re, xy_im = st[prob].xy_im;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st[prob].oxy_re = xy_re;
+        st[prob].oxy_im = xy_im;
+        st[prob].ittot += 1;
+    }
+    double ct, sn;
+    ritz_rotation(xy_re - pz, ccc, ct, sn);
     double v[kRitzParts] = {0.0, 0.0, 0.0, 0.0};
     if (site < V) {
         const size_t o = ((size_t)prob * V + site) * NCOMP;
@@ -421,6 +426,349 @@ __global__ void __launch_bounds__(kRitzThreads)
     block_partials(v, 1, part_of(part, 1, prob, a.nblocks) + (size_t)blockIdx.x * kRitzParts);
 }
 
+// ------------------------------------------------- one launch per solve --
+// The whole two-colour iteration in one cooperative launch.  The kernels above
+// take a step in six launches of a few CTAs each, and at the sizes of the
+// spectral bounds a launch is all latency (8^3: 37 us per step, 6.3 us per
+// kernel).  Here two threads own a site, half h the spins h and 3 - h of both
+// colours, and keep x, y = A x, p, z = A p and g of it in registers for the
+// whole solve; only the vectors the stencil reads from neighbours (the raw
+// direction, or x at a restart, and t = D p) go through memory, component by
+// component over the sites.  A step is five phases, each ending in a barrier
+// of the problem's CTAs that also delivers the phase's sums: t = D p; z = -s D t;
+// the rotation; the residual; the new direction (normalised on the way into
+// the next step).  The arithmetic is that of the kernels above, except that D
+// is applied to the raw direction and its result scaled.
+// One overlap leapfrog step with its two pairs of bounds at 8^3, 256 modes:
+// 91 ms with six launches per Ritz step, 50 ms with one launch per solve.
+// The CTAs wait for one another, so the launch is cooperative (all resident)
+// and every wait is bounded (1 s of %globaltimer): on expiry the error word is
+// set, every CTA leaves at its next wait, and the host reports the solve as failed.
+constexpr int kRitzSites = 32;               // sites per CTA
+constexpr int kRitzOneThreads = 2 * kRitzSites;
+constexpr int kRitzTabStride = 50;           // doubles per site of the link table: 6 x 8 and 2 to spread the banks
+
+struct RitzOne {
+    const double2 *start;  // [V][8]
+    double2 *v, *t;        // [problem][8][V]: the exchanged vectors
+    double *part;          // [2 slots][problem][CTAs][kRitzParts]
+    int *count, *err;      // arrivals per problem; error word
+    RitzScalars *st;
+    double amass, delitr;
+    int max_iter, nrestart;
+};
+
+// One thread waits for the count, polling without a pause (the phases are a
+// few hundred nanoseconds apart); bounded as wait_count.
+__device__ __forceinline__ bool ritz_wait(const int *counter, int target, int *err) {
+    if (ld_acquire(counter) >= target) return true;
+    const unsigned long long t0 = global_ns();
+    for (long long polls = 1; ld_acquire(counter) < target; polls++) {
+        if ((polls & 255) == 0 &&
+            (polls > kWaitPolls || (long long)(global_ns() - t0) > kWaitNs || *(volatile int *)err)) {
+            atomicExch(err, 1);
+            return false;
+        }
+    }
+    return true;
+}
+
+struct RitzBarrier {
+    double *part;  // this problem's partials of slot 0; slot 1 at + slot_stride
+    size_t slot_stride;
+    int *count, *err;
+    int nblocks, phase;
+};
+
+// Sums nv values over the problem's CTAs (in the order of the CTAs; every
+// thread gets the same totals) behind a barrier of them: what the CTAs wrote
+// before it is visible after it.  False when a wait ran out.
+__device__ __forceinline__ bool ritz_sum(RitzBarrier &b, int nv, const double (&v)[kRitzParts], double (&out)[kRitzParts]) {
+    __shared__ double sh[kRitzOneThreads / 32][kRitzParts], tot[kRitzParts];
+    __shared__ int ok;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = 0; k < nv; k++) {
+        double t = v[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sh[warp][k] = t;
+    }
+    __syncthreads();
+    double *slot = b.part + (b.phase & 1) * b.slot_stride;
+    b.phase++;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < nv; k++) {
+            double t = 0.0;
+            for (int w = 0; w < kRitzOneThreads / 32; w++) t += sh[w][k];
+            __stcg(slot + (size_t)blockIdx.x * kRitzParts + k, t);
+        }
+        red_release_add(b.count, 1);
+        ok = ritz_wait(b.count, b.nblocks * b.phase, b.err) ? 1 : 0;
+    }
+    __syncthreads();
+    if (!ok) return false;
+    if (nv > 0) {
+        if (threadIdx.x < 32) {
+            double t[kRitzParts] = {0.0, 0.0, 0.0, 0.0};
+            for (int i = lane; i < b.nblocks; i += 32)
+                for (int k = 0; k < nv; k++) t[k] += __ldcg(slot + (size_t)i * kRitzParts + k);
+            for (int k = 0; k < nv; k++) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+                if (lane == 0) tot[k] = t[k];
+            }
+        }
+        __syncthreads();
+        for (int k = 0; k < nv; k++) out[k] = tot[k];
+    }
+    __syncthreads();  // sh, tot and ok are reused by the next phase
+    return true;
+}
+
+// Component (colour c, upper 0 / lower 1) of half h: spin h or 3 - h.
+__device__ __forceinline__ int ritz_comp(int c, int lower, int h) { return c * kSpin + (lower ? 3 - h : h); }
+
+// The half spinor of D src at the thread's site: own[c][0] spin h, own[c][1]
+// spin 3 - h of src there; the neighbours' components from src [8][V].
+// The projections and reconstruction of hop() (ovl_stencil.cuh), half by half:
+// h0 and its products belong to half 0, h1 to half 1; in the z hops the lower
+// component rebuilt from one half's product belongs to the other half.
+__device__ __forceinline__ void ritz_half_d(const double *__restrict__ tab, const double2 *src, int V, const Nbrs &n,
+                                            int h, bool live, double amass, const cpx<double> (&own)[2][2],
+                                            cpx<double> (&out)[2][2]) {
+    const double sg = h ? -1.0 : 1.0;
+    cpx<double> acc[2][2];
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+        for (int k = 0; k < 2; k++) acc[c][k] = amass * own[c][k];
+    auto at = [&](int site, int comp) {
+        const double2 u = __ldcg(src + (size_t)comp * V + site);
+        return mk<double>(u.x, u.y);
+    };
+    auto link = [&](int dir) {
+        const double2 *q = reinterpret_cast<const double2 *>(tab + 8 * dir);
+        const double2 a = q[0], b = q[1], c = q[2], d = q[3];
+        return cmat2<double>{{a.x, a.y}, {b.x, b.y}, {c.x, c.y}, {d.x, d.y}};
+    };
+#pragma unroll
+    for (int dir = 0; dir < 6; dir++) {  // +x, +y, +z, -x, -y, -z as in the link table
+        const int mu = dir % 3;
+        const bool fwd = dir < 3;
+        const int nb = mu == 0 ? (fwd ? n.xp : n.xm) : (mu == 1 ? (fwd ? n.yp : n.ym) : (fwd ? n.zp : n.zm));
+        const double s = fwd ? 1.0 : -1.0;
+        cpx<double> hh[2], k[2];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const cpx<double> up = at(nb, c * kSpin + h);
+            const cpx<double> lo = at(nb, c * kSpin + (mu == 2 ? 2 + h : 3 - h));
+            if (mu == 0) hh[c] = mk<double>(fma(-s, lo.im, up.re), fma(s, lo.re, up.im));              // p_h +- i p_{3-h}
+            else if (mu == 1) hh[c] = mk<double>(fma(s * sg, lo.re, up.re), fma(s * sg, lo.im, up.im));  // p_h +- sg p_{3-h}
+            else hh[c] = mk<double>(fma(-s * sg, lo.im, up.re), fma(s * sg, lo.re, up.im));            // p_h +- sg i p_{2+h}
+        }
+        const cmat2<double> M = link(dir);
+        if (fwd) mul(M, hh[0], hh[1], k[0], k[1]);
+        else mul_dag(M, hh[0], hh[1], k[0], k[1]);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            acc[c][0] = acc[c][0] - k[c];
+            if (mu == 0) {  // lower -= -+ i k
+                acc[c][1] = acc[c][1] - s * times_mi(k[c]);
+            } else if (mu == 1) {  // lower -= +- sg k
+                acc[c][1] = acc[c][1] - (s * sg) * k[c];
+            } else {  // the other half's product: lower -= +- sg i k'
+                const cpx<double> o = mk<double>(__shfl_xor_sync(0xffffffffu, k[c].re, 1), __shfl_xor_sync(0xffffffffu, k[c].im, 1));
+                acc[c][1] = acc[c][1] - (s * sg) * times_i(o);
+            }
+        }
+    }
+    (void)live;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {  // -i gamma_0 / 2
+        out[c][0] = 0.5 * times_mi(acc[c][0]);
+        out[c][1] = 0.5 * times_i(acc[c][1]);
+    }
+}
+
+template <bool U1>
+__global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> lk, Lattice L, RitzOne a) {
+    __shared__ double tab_s[kRitzSites * kRitzTabStride];
+    const int prob = blockIdx.y, V = L.V;
+    const int sl = threadIdx.x >> 1, h = threadIdx.x & 1;
+    const int want = blockIdx.x * kRitzSites + sl;
+    const bool live = want < V;
+    const int site = live ? want : 0;  // a padded pair repeats site 0 and adds nothing
+    for (int i = threadIdx.x; i < kRitzSites * 6; i += kRitzOneThreads) {
+        const int s = blockIdx.x * kRitzSites + i / 6, dir = i % 6, mu = dir % 3;
+        if (s < V) {
+            int ls = s;
+            if (dir >= 3) {
+                const Nbrs n = neighbours(L, s);
+                ls = mu == 0 ? n.xm : (mu == 1 ? n.ym : n.zm);
+            }
+            const cmat2<double> M = lk.template get<double>(ls, mu);
+            double2 *o = reinterpret_cast<double2 *>(tab_s + (i / 6) * kRitzTabStride + 8 * dir);
+            o[0] = make_double2(M.m00.re, M.m00.im);
+            o[1] = make_double2(M.m01.re, M.m01.im);
+            o[2] = make_double2(M.m10.re, M.m10.im);
+            o[3] = make_double2(M.m11.re, M.m11.im);
+        }
+    }
+    __syncthreads();
+    const double *tab = tab_s + (live ? sl : 0) * kRitzTabStride;
+    const Nbrs n = neighbours(L, site);
+    const double sign = prob == 0 ? 1.0 : -1.0;
+    double2 *v = a.v + (size_t)prob * kComp * V, *t = a.t + (size_t)prob * kComp * V;
+    RitzBarrier bar;
+    bar.nblocks = gridDim.x;
+    bar.slot_stride = (size_t)2 * gridDim.x * kRitzParts;
+    bar.part = a.part + (size_t)prob * gridDim.x * kRitzParts;
+    bar.count = a.count + prob;
+    bar.err = a.err;
+    bar.phase = 0;
+    using Half = cpx<double>[2][2];
+    auto store = [&](double2 *dst, const Half &f) {
+        if (!live) return;
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) __stcg(dst + (size_t)ritz_comp(c, k, h) * V + site, make_double2(f[c][k].re, f[c][k].im));
+    };
+    auto dot = [&](const Half &u, const Half &w, double &re, double &im) {
+        if (!live) return;
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                re += u[c][k].re * w[c][k].re + u[c][k].im * w[c][k].im;
+                im += u[c][k].re * w[c][k].im - u[c][k].im * w[c][k].re;
+            }
+    };
+#define OVL_RITZ_EACH for (int c = 0; c < 2; c++) for (int k = 0; k < 2; k++)
+    Half x, y, p, z, g, raw;
+    double s[kRitzParts], r[kRitzParts];
+    auto clear = [&]() { s[0] = s[1] = s[2] = s[3] = 0.0; };
+    // x = start / |start|
+#pragma unroll
+    OVL_RITZ_EACH {
+        const double2 u = a.start[(size_t)site * kComp + ritz_comp(c, k, h)];
+        x[c][k] = mk<double>(u.x, u.y);
+        y[c][k] = p[c][k] = z[c][k] = g[c][k] = raw[c][k] = mk<double>(0.0, 0.0);
+    }
+    clear();
+    dot(x, x, s[0], s[3]);
+    if (!ritz_sum(bar, 1, s, r)) return;
+    {
+        const double inv = 1.0 / sqrt(r[0]);
+#pragma unroll
+        OVL_RITZ_EACH x[c][k] = inv * x[c][k];
+    }
+    double xy_re = 0.0, xy_im = 0.0, gnorm = 0.0, raw2 = 0.0;
+    int ittot = 0;
+    bool stop = false;
+    while (!stop) {
+        // restart (RitzSolver.cpp:138-166): y = s A x, xy = <x, y>, g = raw direction = y - xy x
+        store(v, x);
+        if (!ritz_sum(bar, 0, s, r)) return;
+        Half w;
+        ritz_half_d(tab, v, V, n, h, live, a.amass, x, w);
+        store(t, w);
+        if (!ritz_sum(bar, 0, s, r)) return;
+        ritz_half_d(tab, t, V, n, h, live, a.amass, w, y);
+#pragma unroll
+        OVL_RITZ_EACH y[c][k] = (-sign) * y[c][k];
+        clear();
+        dot(x, y, s[0], s[1]);
+        if (!ritz_sum(bar, 2, s, r)) return;
+        xy_re = r[0];
+        xy_im = r[1];
+        clear();
+#pragma unroll
+        OVL_RITZ_EACH {
+            g[c][k] = mk<double>(y[c][k].re - (xy_re * x[c][k].re - xy_im * x[c][k].im),
+                                 y[c][k].im - (xy_re * x[c][k].im + xy_im * x[c][k].re));
+            raw[c][k] = g[c][k];
+        }
+        dot(g, g, s[0], s[3]);
+        store(v, raw);
+        if (!ritz_sum(bar, 1, s, r)) return;
+        raw2 = r[0];
+        double gnormim = raw2;
+        for (int itt = 1; itt <= a.nrestart && !stop; itt++) {
+            // p = raw / |raw|; t = D p
+            const double pnorm = sqrt(raw2), inv = 1.0 / pnorm;
+#pragma unroll
+            OVL_RITZ_EACH p[c][k] = mk<double>(raw[c][k].re / pnorm, raw[c][k].im / pnorm);
+            ritz_half_d(tab, v, V, n, h, live, a.amass, raw, w);
+#pragma unroll
+            OVL_RITZ_EACH w[c][k] = inv * w[c][k];
+            store(t, w);
+            if (!ritz_sum(bar, 0, s, r)) return;
+            // z = s A p; <p, z>, <x, z>
+            ritz_half_d(tab, t, V, n, h, live, a.amass, w, z);
+#pragma unroll
+            OVL_RITZ_EACH z[c][k] = (-sign) * z[c][k];
+            clear();
+            dot(p, z, s[0], s[1]);
+            dot(x, z, s[2], s[3]);
+            if (!ritz_sum(bar, 4, s, r)) return;
+            // the rotation in the (x, p) plane (RitzSolver.cpp:176-222)
+            const double oxy_re = xy_re;
+            double ct, sn;
+            ritz_rotation(xy_re - r[0], r[2], ct, sn);
+            ittot++;
+#pragma unroll
+            OVL_RITZ_EACH {
+                x[c][k] = mk<double>(x[c][k].re * ct + p[c][k].re * sn, x[c][k].im * ct + p[c][k].im * sn);
+                y[c][k] = mk<double>(y[c][k].re * ct + z[c][k].re * sn, y[c][k].im * ct + z[c][k].im * sn);
+            }
+            clear();
+            dot(x, x, s[0], s[3]);
+            dot(x, y, s[1], s[2]);
+            if (!ritz_sum(bar, 3, s, r)) return;
+            // x normalised, xy, g (RitzSolver.cpp:224-243)
+            const double xnorm = 1.0 / sqrt(r[0]);
+            xy_re = r[1] * xnorm;
+            xy_im = r[2] * xnorm;
+            clear();
+#pragma unroll
+            OVL_RITZ_EACH {
+                x[c][k] = xnorm * x[c][k];
+                g[c][k] = mk<double>(y[c][k].re - (xy_re * x[c][k].re - xy_im * x[c][k].im),
+                                     y[c][k].im - (xy_re * x[c][k].im + xy_im * x[c][k].re));
+            }
+            dot(g, g, s[0], s[3]);
+            s[3] = 0.0;
+            dot(x, p, s[1], s[2]);
+            if (!ritz_sum(bar, 3, s, r)) return;
+            // stopping tests and the new direction (RitzSolver.cpp:245-284)
+            gnorm = r[0];
+            const double xpr = r[1], xpi = r[2];
+            stop = xy_re > oxy_re || gnorm < a.delitr * sign * xy_re || ittot >= a.max_iter;
+            if (stop) break;
+            const double beta = gnorm / gnormim * pnorm;
+            clear();
+#pragma unroll
+            OVL_RITZ_EACH {
+                const cpx<double> xxp = mk<double>(x[c][k].re * xpr - x[c][k].im * xpi, x[c][k].re * xpi + x[c][k].im * xpr);
+                raw[c][k] = mk<double>(g[c][k].re + beta * (p[c][k].re - xxp.re), g[c][k].im + beta * (p[c][k].im - xxp.im));
+            }
+            dot(raw, raw, s[0], s[3]);
+            store(v, raw);
+            if (!ritz_sum(bar, 1, s, r)) return;
+            raw2 = r[0];
+            gnormim = gnorm;
+        }
+    }
+#undef OVL_RITZ_EACH
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.st[prob].xy_re = xy_re;
+        a.st[prob].xy_im = xy_im;
+        a.st[prob].ittot = ittot;
+        a.st[prob].done = 1;
+    }
+}
+
 // Start vector with the reference's distribution (Re, Im uniform in [0, 1),
 // OverlapUpdate.cpp:69-84) from a counter-based generator: SplitMix64
 // (Steele, Lea and Flood, "Fast splittable pseudorandom number generators",
@@ -465,32 +813,29 @@ struct RitzWork {
     double2 *x = nullptr, *y = nullptr, *z = nullptr, *t = nullptr, *p = nullptr, *praw = nullptr, *g = nullptr;
     double2 *start = nullptr;
     double *part = nullptr;
+    int *count = nullptr;         // one-launch solve: arrivals of the two problems, error word
     RitzScalars *st = nullptr;
-    RitzScalars *host = nullptr;  // pinned
+    RitzScalars *host = nullptr;  // pinned, two and the error word
     int V = 0;
     int nc = 2;  // colours: vectors of 4 nc components per site
     RitzGraphs graphs;
 };
-
-size_t ritz_work_bytes(int V, int nc) {
-    const int nblocks = (V + kRitzThreads - 1) / kRitzThreads;
-    return sizeof(double2) * 4 * nc * (size_t)V * (7 * 2 + 1) + sizeof(double) * 4 * nblocks * kRitzParts +
-           2 * sizeof(RitzScalars);
-}
 
 void *ritz_create(int V, int nc) {
     RitzWork *w = new RitzWork;
     w->V = V;
     w->nc = nc;
     const size_t vec = sizeof(double2) * 4 * nc * (size_t)V * 2;
-    const int nblocks = (V + kRitzThreads - 1) / kRitzThreads;
+    // partials of the kernel-by-kernel iteration or of the one-launch solve (smaller CTAs)
+    const int nblocks = (V + kRitzSites - 1) / kRitzSites;
     double2 **bufs[] = {&w->x, &w->y, &w->z, &w->t, &w->p, &w->praw, &w->g};
     bool ok = true;
     for (double2 **b : bufs) ok = ok && cudaMalloc(b, vec) == cudaSuccess;
     ok = ok && cudaMalloc(&w->start, vec / 2) == cudaSuccess;
     ok = ok && cudaMalloc(&w->part, sizeof(double) * 4 * nblocks * kRitzParts) == cudaSuccess;
+    ok = ok && cudaMalloc(&w->count, sizeof(int) * 3) == cudaSuccess;
     ok = ok && cudaMalloc(&w->st, 2 * sizeof(RitzScalars)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&w->host, 2 * sizeof(RitzScalars)) == cudaSuccess;
+    ok = ok && cudaMallocHost(&w->host, 3 * sizeof(RitzScalars)) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         ritz_destroy(w);
@@ -502,7 +847,7 @@ void *ritz_create(int V, int nc) {
 void ritz_destroy(void *work) {
     RitzWork *w = static_cast<RitzWork *>(work);
     if (!w) return;
-    void *bufs[] = {w->x, w->y, w->z, w->t, w->p, w->praw, w->g, w->start, w->part, w->st};
+    void *bufs[] = {w->x, w->y, w->z, w->t, w->p, w->praw, w->g, w->start, w->part, w->count, w->st};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (w->host) cudaFreeHost(w->host);
@@ -667,6 +1012,58 @@ static cudaError_t ritz_run_nc(RitzWork &w, const double *U, const double *u1, c
     return cudaSuccess;
 }
 
+// Whether the one-launch solve serves a lattice of V sites: its CTAs all fit
+// the GPU at once.  (up to 9472 sites on 148 SMs; beyond that, and for
+// three colours, whose vectors do not fit the registers, the iteration above.)
+template <bool U1> static bool ritz_one_fits(int V) {
+    int dev = 0, sms = 0, coop = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ritz_one_kernel<U1>, kRitzOneThreads, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return coop && 2LL * ((V + kRitzSites - 1) / kRitzSites) <= (long long)sms * per_sm;
+}
+
+template <bool U1>
+static cudaError_t ritz_run_one(RitzWork &w, const double *U, const double *u1, const Lattice &L, double amass,
+                                int max_iter, int nrestart, double delitr, double out[2], int iters[2],
+                                cudaStream_t stream, uint64_t *launches) {
+    RitzOne a;
+    a.start = w.start;
+    a.v = w.praw;
+    a.t = w.t;
+    a.part = w.part;
+    a.count = w.count;
+    a.err = w.count + 2;
+    a.st = w.st;
+    a.amass = amass;
+    a.delitr = delitr;
+    a.max_iter = max_iter;
+    a.nrestart = nrestart;
+    LinksF64<U1> lk{U, reinterpret_cast<const double2 *>(u1), L.N0 * L.N1};
+    Lattice lat = L;
+    cudaError_t e = cudaMemsetAsync(w.count, 0, sizeof(int) * 3, stream);
+    if (e != cudaSuccess) return e;
+    void *args[] = {&lk, &lat, &a};
+    const dim3 grid((L.V + kRitzSites - 1) / kRitzSites, 2);
+    e = cudaLaunchCooperativeKernel(ritz_one_kernel<U1>, grid, dim3(kRitzOneThreads), args, 0, stream);
+    if (e != cudaSuccess) return e;
+    int *err = reinterpret_cast<int *>(w.host + 2);
+    if ((e = cudaMemcpyAsync(w.host, w.st, 2 * sizeof(RitzScalars), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(err, a.err, sizeof(int), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(stream)) != cudaSuccess)
+        return e;
+    if (*err) return cudaErrorLaunchTimeout;  // a wait between the CTAs ran out
+    for (int k = 0; k < 2; k++) {
+        out[k] = w.host[k].xy_re;
+        if (iters) iters[k] = w.host[k].ittot;
+    }
+    if (launches) *launches += 1;
+    return cudaSuccess;
+}
+
 // Runs both Ritz problems from the start vector already in the start buffer
 // (compact [V][4 nc] double2; links of the work space's colour count).  out:
 // {lambda_min, -lambda_max as returned by the sign = -1 problem}; iters: steps
@@ -677,6 +1074,9 @@ cudaError_t ritz_run(void *work, const double *U, const double *u1, const Lattic
     RitzWork &w = *static_cast<RitzWork *>(work);
     if (w.nc == 3)
         return ritz_run_nc<3>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
+    if (u1 ? ritz_one_fits<true>(L.V) : ritz_one_fits<false>(L.V))
+        return u1 ? ritz_run_one<true>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches)
+                  : ritz_run_one<false>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
     return ritz_run_nc<2>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
 }
 
