@@ -117,6 +117,54 @@ __device__ __forceinline__ double warp_sum16(double (&v)[16]) {
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// The same for 32 values: lane i returns the total of v[i] (31 shuffles for 160).
+__device__ __forceinline__ double warp_sum32(double (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 16; n >= 1; n >>= 1) {
+        const bool up = lane & n;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const double send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+        }
+    }
+    return v[0];
+}
+
+// The colour force's link-independent bilinears of one hop direction,
+// C_ij += psi_i^+ g0 (1 - G_mu) psi'_j with psi' the neighbour.  1 - G_mu = 1 + i
+// g_mu is twice a rank-2 projector: (1 + i g_mu) psi' is rebuilt from its two
+// upper spin components h0, h1 (the forward projection of hop()), so that
+// psi^+ g0 (1 + i g_mu) psi' = q0^+ h0 + q1^+ h1 with q0, q1 the backward projection
+// of psi: two dot products per colour pair instead of the eight terms of two
+// full spinor bilinears.  f carries the vacuum weight.
+template <int NC, int MU, class RAW>
+__device__ __forceinline__ void add_colour_pairs(const cpx<double> (&f)[NC][kSpin], const RAW &raw, double *acc) {
+    cpx<double> h0[NC], h1[NC];
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+        const cpx<double> p0 = raw.get(kSpin * j), p1 = raw.get(kSpin * j + 1), p2 = raw.get(kSpin * j + 2),
+                          p3 = raw.get(kSpin * j + 3);
+        h0[j] = MU == 0 ? p0 + times_i(p3) : (MU == 1 ? p0 + p3 : p0 + times_i(p2));
+        h1[j] = MU == 0 ? p1 + times_i(p2) : (MU == 1 ? p1 - p2 : p1 - times_i(p3));
+    }
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        const cpx<double> *p = f[i];
+        const cpx<double> q0 = MU == 0 ? p[0] - times_i(p[3]) : (MU == 1 ? p[0] - p[3] : p[0] - times_i(p[2]));
+        const cpx<double> q1 = MU == 0 ? p[1] - times_i(p[2]) : (MU == 1 ? p[1] + p[2] : p[1] + times_i(p[3]));
+#pragma unroll
+        for (int j = 0; j < NC; j++) {
+            double *a = acc + 2 * (NC * i + j);
+            add_part<false>(a[0], 0, q0, h0[j]);
+            add_part<false>(a[0], 0, q1, h1[j]);
+            add_part<true>(a[1], 0, q0, h0[j]);
+            add_part<true>(a[1], 0, q1, h1[j]);
+        }
+    }
+}
+
 // Vacuum weight of a mode: +-1 by the parity of its global index, 0 for padding.
 __device__ __forceinline__ double vacuum_weight(int mode, int n_modes, int first_mode) {
     return mode >= n_modes ? 0.0 : (((first_mode + mode) & 1) == 0 ? 1.0 : -1.0);

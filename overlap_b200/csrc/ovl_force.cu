@@ -15,102 +15,67 @@
 // with M the (U(1)-dressed) link.  The link update U <- exp(-i dt E^a t^a) U of
 // the reference makes d theta / dt = -E, so dE/dt = dH/dtheta conserves
 // H_gauge + g^2 H_F.
+#include "ovl_bilinears.cuh"
 #include "ovl_device.cuh"
 #include "ovl_fp40.cuh"
 #include "ovl_internal.h"
 
 namespace ovl {
 
-constexpr int kForceThreadsY = kSitesPerCta;
-
-// One site's spinor of the lane's mode as complex doubles, from a field view
-// (SrcPlain<T> or Src40, ovl_fp40.cuh).
-template <class SRC>
-__device__ __forceinline__ void force_load(const SRC &f, int V, int mb, int site, int lane,
-                                           cpx<double> (&s)[kColours][kSpin]) {
-    const size_t base = field_index(V, mb, site, 0, lane);
-#pragma unroll
-    for (int c = 0; c < kColours; c++)
-#pragma unroll
-        for (int a = 0; a < kSpin; a++) s[c][a] = f(base + (c * kSpin + a) * kModeBlock);
-}
+constexpr int kForceSites = 4;
 
 // partial[(g V + site) kForcePerSite + 8 mu + 2 (2 i + j) + {re, im}] = C_ij of
 // mode-block group g (a warp is one site, its lanes the 32 modes of a block).
+// Four coupled steps at 8^3, 1024 FP64 modes: 645 us with the eight-term
+// bilinears and one thread per link in the finish and the staple force, 539 us so.
 template <class SRC>
-__global__ void __launch_bounds__(kModeBlock *kForceThreadsY)
+__global__ void __launch_bounds__(kModeBlock *kForceSites, 3)
     color_force_modes_kernel(SRC psi, Lattice L, int n_mb, int n_modes, int first_mode, int groups,
                              double *__restrict__ partial) {
-    constexpr mono G0 = kGamma0;
-    constexpr mono G0M[3] = {mono_mul(kGamma0, kGammaX), mono_mul(kGamma0, kGammaY), mono_mul(kGamma0, kGammaZ)};
     const int lane = threadIdx.x;
-    const int site = blockIdx.x * kForceThreadsY + threadIdx.y;
+    const int site = blockIdx.x * kForceSites + threadIdx.y;
     const int g = blockIdx.y;
     if (site >= L.V) return;  // whole warps exit together
-    int x, y, z;
-    site_coords(L, site, x, y, z);
-    int nb[3];
+    const Nbrs nb = neighbours(L, site);
+    double acc[32];  // kForcePerSite used
 #pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-        int c[3] = {x, y, z};
-        c[mu] += 1;
-        nb[mu] = site_index(L, c[0], c[1], c[2]);
-    }
-    double acc[kForcePerSite];
-#pragma unroll
-    for (int k = 0; k < kForcePerSite; k++) acc[k] = 0.0;
+    for (int k = 0; k < 32; k++) acc[k] = 0.0;
     for (int mb = g; mb < n_mb; mb += groups) {
-        const int mode = mb * kModeBlock + lane;
-        const double w = mode >= n_modes ? 0.0 : (((first_mode + mode) & 1) == 0 ? 1.0 : -1.0);
+        const double w = vacuum_weight(mb * kModeBlock + lane, n_modes, first_mode);
+        SiteRaw<2, SRC> raw;
+        raw.load(psi, L.V, mb, site, lane);
         cpx<double> f[kColours][kSpin];
-        force_load(psi, L.V, mb, site, lane, f);
 #pragma unroll
-        for (int mu = 0; mu < 3; mu++) {
-            cpx<double> h[kColours][kSpin];
-            force_load(psi, L.V, mb, nb[mu], lane, h);
-#pragma unroll
-            for (int i = 0; i < kColours; i++)
-#pragma unroll
-                for (int j = 0; j < kColours; j++) {
-                    const cpx<double> b0 = bilinear<double>(G0, f[i], h[j]);
-                    const cpx<double> b1 = bilinear<double>(G0M[mu], f[i], h[j]);
-                    // g0 (1 + i g_mu) = g0 + i g0 g_mu
-                    const int k = 8 * mu + 2 * (2 * i + j);
-                    acc[k] += w * (b0.re - b1.im);
-                    acc[k + 1] += w * (b0.im + b1.re);
-                }
-        }
+        for (int k = 0; k < kComp; k++) f[k / kSpin][k % kSpin] = w * raw.get(k);
+        raw.load(psi, L.V, mb, nb.xp, lane);
+        add_colour_pairs<2, 0>(f, raw, acc);
+        raw.load(psi, L.V, mb, nb.yp, lane);
+        add_colour_pairs<2, 1>(f, raw, acc + 8);
+        raw.load(psi, L.V, mb, nb.zp, lane);
+        add_colour_pairs<2, 2>(f, raw, acc + 16);
     }
-#pragma unroll
-    for (int k = 0; k < kForcePerSite; k++) {
-        double t = acc[k];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        acc[k] = t;
-    }
-    if (lane == 0) {
-        double *p = partial + ((size_t)g * L.V + site) * kForcePerSite;
-#pragma unroll
-        for (int k = 0; k < kForcePerSite; k++) p[k] = acc[k];
-    }
+    const double total = warp_sum32(acc);
+    if (lane < kForcePerSite) partial[((size_t)g * L.V + site) * kForcePerSite + lane] = total;
 }
 
-// One thread per (site, mu): sum the groups' C, contract with the dressed link.
-// out != null: out[a + 3 (mu + 3 site)] = dH_F/dtheta^a; otherwise
+// One warp per (site, mu): lane k + 8 s sums C's value k over the groups s, s + 4,
+// ..., then every lane contracts C with the dressed link and lane a < 3 writes
+// dH_F/dtheta^a: out[a + 3 (mu + 3 site)] when out is set, otherwise
 // E[a + 3 (mu + 3 site)] += coef dH_F/dtheta^a.
 __global__ void color_force_finish_kernel(const double *__restrict__ partial, int groups, const double *__restrict__ U,
                                           const double2 *__restrict__ u1, Lattice L, double *__restrict__ out,
                                           double *__restrict__ E, double coef) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * L.V) return;
+    const int t = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (t >= 3 * L.V) return;  // whole warps exit together
     const int site = t / 3, mu = t % 3;
+    double v = 0.0;
+    for (int g = lane >> 3; g < groups; g += 4)
+        v += partial[((size_t)g * L.V + site) * kForcePerSite + 8 * mu + (lane & 7)];
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
     double c[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) c[k] = 0.0;
-    for (int g = 0; g < groups; g++) {
-        const double *p = partial + ((size_t)g * L.V + site) * kForcePerSite + 8 * mu;
-#pragma unroll
-        for (int k = 0; k < 8; k++) c[k] += p[k];
-    }
+    for (int k = 0; k < 8; k++) c[k] = __shfl_sync(0xffffffffu, v, k);
     const cpx<double> C00 = mk<double>(c[0], c[1]), C01 = mk<double>(c[2], c[3]);
     const cpx<double> C10 = mk<double>(c[4], c[5]), C11 = mk<double>(c[6], c[7]);
     const cmat2<double> M = dressed_link<double>(U, u1, site, mu, L.N0 * L.N1);
@@ -119,21 +84,14 @@ __global__ void color_force_finish_kernel(const double *__restrict__ partial, in
     const cpx<double> m0c1 = M.m00 * C10 + M.m01 * C11;  // sum_j M_0j C_1j
     const cpx<double> m0c0 = M.m00 * C00 + M.m01 * C01;
     const cpx<double> m1c1 = M.m10 * C10 + M.m11 * C11;
+    if (lane >= 3) return;
     const double sx = m1c0.im + m0c1.im;
     const double sy = -m1c0.re + m0c1.re;  // Im(-i m1c0 + i m0c1)
     const double sz = m0c0.im - m1c1.im;
-    const double s = 1.0 / (4.0 * L.V);
-    const double f[3] = {s * sx, s * sy, s * sz};
-    const size_t o = 3 * ((size_t)mu + 3 * (size_t)site);
-    if (out) {
-        out[o] = f[0];
-        out[o + 1] = f[1];
-        out[o + 2] = f[2];
-    } else {
-        E[o] += coef * f[0];
-        E[o + 1] += coef * f[1];
-        E[o + 2] += coef * f[2];
-    }
+    const double f = 1.0 / (4.0 * L.V) * (lane == 0 ? sx : (lane == 1 ? sy : sz));
+    const size_t o = 3 * (size_t)t + lane;
+    if (out) out[o] = f;
+    else E[o] += coef * f;
 }
 
 int force_groups(int n_mb) { return n_mb < 16 ? n_mb : 16; }
@@ -145,13 +103,11 @@ static void color_force_from(const SRC &src, const double *U, const double *u1, 
                              int n_modes, int first_mode, double *partial, double *out, double *E, double coef,
                              cudaStream_t stream) {
     const int groups = force_groups(n_mb);
-    dim3 block(kModeBlock, kForceThreadsY);
-    dim3 grid((L.V + kForceThreadsY - 1) / kForceThreadsY, groups);
+    const dim3 block(kModeBlock, kForceSites), grid((L.V + kForceSites - 1) / kForceSites, groups);
     color_force_modes_kernel<SRC><<<grid, block, 0, stream>>>(src, L, n_mb, n_modes, first_mode, groups, partial);
-    const int n = 3 * L.V;
-    color_force_finish_kernel<<<(n + 127) / 128, 128, 0, stream>>>(partial, groups, U,
-                                                                   reinterpret_cast<const double2 *>(u1), L, out, E,
-                                                                   coef);
+    const int links_per_cta = 8;  // a warp each
+    color_force_finish_kernel<<<(3 * L.V + links_per_cta - 1) / links_per_cta, 32 * links_per_cta, 0, stream>>>(
+        partial, groups, U, reinterpret_cast<const double2 *>(u1), L, out, E, coef);
 }
 
 template <typename T>

@@ -99,36 +99,20 @@ __device__ quat loop(const double *__restrict__ U, const Lattice &L, int x, int 
 // E^a_mu(x) += -2 dt sum_{nu != mu} [Re tr(i t^a U_{mu,nu}) + Re tr(i t^a U_{mu,-nu})],
 // both staples written to start with U_mu(x) (Dynamics.cpp:145-197).
 // Re tr(i t^a q) = -q_a.
+// Four lanes share a link, a plaquette each (two transverse directions, both
+// sides); their sums are added by shuffles.
 __global__ void update_efield_kernel(const double *__restrict__ U, double *E, Lattice L, double gamma) {
-    int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= 3 * L.V) return;
-    const int site = l / 3, mu = l % 3;
-    int x, y, z;
-    site_coords(L, site, x, y, z);
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int nu = 0; nu < 3; nu++) {
-        if (nu == mu) continue;
-        int c[3] = {x, y, z};
-        quat up = {0.0, 0.0, 0.0, 1.0};
-        up = path_step(U, L, c, mu, +1, up);
-        up = path_step(U, L, c, nu, +1, up);
-        up = path_step(U, L, c, mu, -1, up);
-        up = path_step(U, L, c, nu, -1, up);
-        int d[3] = {x, y, z};
-        quat dn = {0.0, 0.0, 0.0, 1.0};
-        dn = path_step(U, L, d, mu, +1, dn);
-        dn = path_step(U, L, d, nu, -1, dn);
-        dn = path_step(U, L, d, mu, -1, dn);
-        dn = path_step(U, L, d, nu, +1, dn);
-        for (int a = 0; a < 3; a++) f[a] += -qcomp(up, a) - qcomp(dn, a);
-    }
-    for (int a = 0; a < 3; a++) E[3 * l + a] += gamma * f[a];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t & 3;
+    const bool live = t < 12 * L.V;  // padded lanes repeat link 0: the shuffles need the whole warp
+    const int l = live ? t >> 2 : 0;
+    const quat p = staple_plaquette<Su2Ops>(U, L, l, q);
+    const double f0 = quad_sum(p.v0), f1 = quad_sum(p.v1), f2 = quad_sum(p.v2);
+    if (live && q < 3) E[3 * (size_t)l + q] -= gamma * (q == 0 ? f0 : (q == 1 ? f1 : f2));
 }
 
 void launch_update_efield(const double *U, double *E, double * /*unused*/, const Lattice &L, double dt_step,
                           cudaStream_t stream) {
-    const int n = 3 * L.V;
-    update_efield_kernel<<<(n + 127) / 128, 128, 0, stream>>>(U, E, L, -2.0 * dt_step);
+    update_efield_kernel<<<(12 * L.V + 127) / 128, 128, 0, stream>>>(U, E, L, -2.0 * dt_step);
 }
 
 // ----------------------------------------------------------------- NCsDot --

@@ -78,6 +78,26 @@ struct Quadrant {
     }
 };
 
+// Plaquette q of the staple force of link l = 3 site + mu (Dynamics.cpp:145-197),
+// starting with U_mu(x): q >> 1 picks the transverse direction nu, q & 1 the
+// side: x -> x+mu -> x+mu+nu -> x+nu, or the same towards -nu.
+template <class OPS>
+__device__ __forceinline__ typename OPS::M staple_plaquette(const double *__restrict__ U, const Lattice &L, int l, int q) {
+    const int site = l / 3, mu = l % 3, nu = (mu + 1 + (q >> 1)) % 3;
+    int c[3];
+    site_coords(L, site, c[0], c[1], c[2]);
+    const int cm = mu == 0 ? c[0] : (mu == 1 ? c[1] : c[2]), cn = nu == 0 ? c[0] : (nu == 1 ? c[1] : c[2]);
+    const int om = wrap_offset(cm, extent_of(L, mu), stride_of(L, mu), 1);
+    const int on = wrap_offset(cn, extent_of(L, nu), stride_of(L, nu), (q & 1) ? -1 : 1);
+    const typename OPS::M u0 = OPS::load(U, site, mu), u2 = OPS::load(U, site + on, mu);
+    if (q & 1) {
+        const typename OPS::M u1 = OPS::load(U, site + om + on, nu), u3 = OPS::load(U, site + on, nu);
+        return OPS::mul(OPS::mul(OPS::mul(u0, OPS::dag(u1)), OPS::dag(u2)), u3);
+    }
+    const typename OPS::M u1 = OPS::load(U, site + om, nu), u3 = OPS::load(U, site, nu);
+    return OPS::mul(OPS::mul(u0, u1), OPS::mul(OPS::dag(u2), OPS::dag(u3)));
+}
+
 // The improved electric field (ChernSimonsOperators.cpp:379-401) is the sum of
 // -1/12, 7/12, 7/12, -1/12 of E_mu at x+mu, x, x-mu, x-2mu transported to x.
 // Term q (0: x, 1: x+mu, 2: x-mu, 3: x-2mu): its site, transporter and weight.

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "ovl_bilinears.cuh"
 #include "ovl_internal.h"
 #include "ovl_loops.cuh"
 #include "ovl_su3.cuh"
@@ -590,39 +591,24 @@ void su3_launch_bulk(const double *U, const double *E, const Lattice &L, double 
 // ------------------------------------------------------------ staple force --
 // E^a_mu(x) += -2 dt sum_{nu != mu} [Re tr(i t^a U_{mu,nu}) + Re tr(i t^a U_{mu,-nu})]
 // (Dynamics.cpp:145-197; update_efield_kernel of ovl_gauge.cu for three colours).
+// Four lanes per link, a plaquette each (update_efield_kernel of ovl_gauge.cu).
 __global__ void su3_efield_kernel(const double *__restrict__ U, double *E, Lattice L, double gamma) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= 3 * L.V) return;
-    const int site = l / 3, mu = l % 3;
-    int x, y, z;
-    site_coords(L, site, x, y, z);
-    double f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int nu = 0; nu < 3; nu++) {
-        if (nu == mu) continue;
-        int c[3] = {x, y, z};
-        cmat3<double> up = m3_unit<double>();
-        up = su3_step(U, L, c, mu, +1, up);
-        up = su3_step(U, L, c, nu, +1, up);
-        up = su3_step(U, L, c, mu, -1, up);
-        up = su3_step(U, L, c, nu, -1, up);
-        int d[3] = {x, y, z};
-        cmat3<double> dn = m3_unit<double>();
-        dn = su3_step(U, L, d, mu, +1, dn);
-        dn = su3_step(U, L, d, nu, -1, dn);
-        dn = su3_step(U, L, d, mu, -1, dn);
-        dn = su3_step(U, L, d, nu, +1, dn);
-        double a[8], b[8];
-        su3_retr_ita(up, a);
-        su3_retr_ita(dn, b);
-        for (int k = 0; k < 8; k++) f[k] += a[k] + b[k];
-    }
-    for (int k = 0; k < 8; k++) E[8 * (size_t)l + k] += gamma * f[k];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t & 3;
+    const bool live = t < 12 * L.V;  // padded lanes repeat link 0: the shuffles need the whole warp
+    const int l = live ? t >> 2 : 0;
+    double f[8];
+    su3_retr_ita(staple_plaquette<Su3Ops>(U, L, l, q), f);
+#pragma unroll
+    for (int k = 0; k < 8; k++) f[k] = quad_sum(f[k]);
+    if (!live) return;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if ((k & 3) == q) E[8 * (size_t)l + k] += gamma * f[k];
 }
 
 // The force of every link reads the links only, so one pass updates E in place.
 void su3_launch_update_efield(const double *U, double *E, const Lattice &L, double dt_step, cudaStream_t s) {
-    const int n = 3 * L.V;
-    su3_efield_kernel<<<(n + 127) / 128, 128, 0, s>>>(U, E, L, -2.0 * dt_step);
+    su3_efield_kernel<<<(12 * L.V + 127) / 128, 128, 0, s>>>(U, E, L, -2.0 * dt_step);
 }
 
 // ------------------------------------------------------ Gauss restoration --
@@ -712,97 +698,70 @@ void su3_launch_gauss_update(const double *U, const double *G, double *E, const 
 // then dH_F/dtheta^a = (1/2V) Im tr(t^a Q), Q = M C^T, M the dressed link.
 constexpr int kForce3PerSite = 3 * 18;  // mu, (i, j), (re, im)
 
-template <typename T>
-__global__ void __launch_bounds__(kModeBlock *kSites3)
-    su3_force_modes_kernel(const cpx<T> *__restrict__ psi, Lattice L, int n_mb, int n_modes, int first_mode,
-                           double *__restrict__ partial) {
-    constexpr mono G0 = kGamma0;
-    constexpr mono G0M[3] = {mono_mul(kGamma0, kGammaX), mono_mul(kGamma0, kGammaY), mono_mul(kGamma0, kGammaZ)};
-    const int lane = threadIdx.x;
-    const int site = blockIdx.x * kSites3 + threadIdx.y;
-    const int g = blockIdx.y, groups = gridDim.y;
-    if (site >= L.V) return;  // whole warps exit together
-    int x, y, z;
-    site_coords(L, site, x, y, z);
-    int nb[3];
-    for (int mu = 0; mu < 3; mu++) {
-        int c[3] = {x, y, z};
-        c[mu] += 1;
-        nb[mu] = site_index(L, c[0], c[1], c[2]);
-    }
-    double acc[kForce3PerSite];
+// One direction mu per blockIdx.z: the 18 sums of one mu beside the spinor fit
+// the registers, the 54 of all three do not.
+template <typename T, int MU>
+__device__ __forceinline__ void su3_force_modes(const SrcPlain<T> &psi, const Lattice &L, int n_mb, int n_modes,
+                                                int first_mode, int site, double *__restrict__ partial) {
+    const int lane = threadIdx.x, g = blockIdx.y, groups = gridDim.y;
+    const Nbrs n = neighbours(L, site);
+    const int nb = MU == 0 ? n.xp : (MU == 1 ? n.yp : n.zp);
+    double acc[32];  // 18 used
 #pragma unroll
-    for (int k = 0; k < kForce3PerSite; k++) acc[k] = 0.0;
+    for (int k = 0; k < 32; k++) acc[k] = 0.0;
     for (int mb = g; mb < n_mb; mb += groups) {
-        const int mode = mb * kModeBlock + lane;
-        const double w = mode >= n_modes ? 0.0 : (((first_mode + mode) & 1) == 0 ? 1.0 : -1.0);
+        const double w = vacuum_weight(mb * kModeBlock + lane, n_modes, first_mode);
+        SiteRaw<3, SrcPlain<T>> raw;
+        raw.load(psi, L.V, mb, site, lane);
         cpx<double> f[3][kSpin];
-        const cpx<T> *pf = psi + field_index3(L.V, mb, site, 0, lane);
 #pragma unroll
-        for (int c = 0; c < 3; c++)
-#pragma unroll
-            for (int a = 0; a < kSpin; a++) {
-                const cpx<T> v = ld(pf + (c * kSpin + a) * kModeBlock);
-                f[c][a] = mk<double>((double)v.re, (double)v.im);
-            }
-#pragma unroll
-        for (int mu = 0; mu < 3; mu++) {
-            cpx<double> h[3][kSpin];
-            const cpx<T> *ph = psi + field_index3(L.V, mb, nb[mu], 0, lane);
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-#pragma unroll
-                for (int a = 0; a < kSpin; a++) {
-                    const cpx<T> v = ld(ph + (c * kSpin + a) * kModeBlock);
-                    h[c][a] = mk<double>((double)v.re, (double)v.im);
-                }
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    const cpx<double> b0 = bilinear<double>(G0, f[i], h[j]);
-                    const cpx<double> b1 = bilinear<double>(G0M[mu], f[i], h[j]);
-                    const int k = 18 * mu + 2 * (3 * i + j);  // g0 (1 - G_mu) = g0 + i g0 g_mu
-                    acc[k] += w * (b0.re - b1.im);
-                    acc[k + 1] += w * (b0.im + b1.re);
-                }
-        }
+        for (int k = 0; k < kComp3; k++) f[k / kSpin][k % kSpin] = w * raw.get(k);
+        raw.load(psi, L.V, mb, nb, lane);
+        add_colour_pairs<3, MU>(f, raw, acc);
     }
-#pragma unroll
-    for (int k = 0; k < kForce3PerSite; k++) {
-        double t = acc[k];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-        acc[k] = t;
-    }
-    if (lane == 0) {
-        double *q = partial + ((size_t)g * L.V + site) * kForce3PerSite;
-#pragma unroll
-        for (int k = 0; k < kForce3PerSite; k++) q[k] = acc[k];
-    }
+    const double total = warp_sum32(acc);
+    if (lane < 18) partial[((size_t)g * L.V + site) * kForce3PerSite + 18 * MU + lane] = total;
 }
 
-// One thread per (site, mu).  out != null: out[a + 8 (mu + 3 site)] =
-// dH_F/dtheta^a; otherwise E[a + 8 (mu + 3 site)] += coef dH_F/dtheta^a.
+template <typename T>
+__global__ void __launch_bounds__(kModeBlock *kSites3, 3)
+    su3_force_modes_kernel(SrcPlain<T> psi, Lattice L, int n_mb, int n_modes, int first_mode,
+                           double *__restrict__ partial) {
+    const int site = blockIdx.x * kSites3 + threadIdx.y;
+    if (site >= L.V) return;  // whole warps exit together
+    if (blockIdx.z == 0) su3_force_modes<T, 0>(psi, L, n_mb, n_modes, first_mode, site, partial);
+    else if (blockIdx.z == 1) su3_force_modes<T, 1>(psi, L, n_mb, n_modes, first_mode, site, partial);
+    else su3_force_modes<T, 2>(psi, L, n_mb, n_modes, first_mode, site, partial);
+}
+
+// One warp per (site, mu): lane k < 18 sums C's value k over the groups, every
+// lane contracts C with the dressed link, and lane a < 8 writes.  out != null:
+// out[a + 8 (mu + 3 site)] = dH_F/dtheta^a; otherwise
+// E[a + 8 (mu + 3 site)] += coef dH_F/dtheta^a.
 template <bool U1>
 __global__ void su3_force_finish_kernel(const double *__restrict__ partial, int groups, const double *__restrict__ U,
                                         const double *__restrict__ u1, Lattice L, double *__restrict__ out,
                                         double *__restrict__ E, double coef) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * L.V) return;
+    const int t = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (t >= 3 * L.V) return;  // whole warps exit together
     const int site = t / 3, mu = t % 3;
+    double v = 0.0;
+    if (lane < 18)
+        for (int g = 0; g < groups; g++) v += partial[((size_t)g * L.V + site) * kForce3PerSite + 18 * mu + lane];
     cmat3<double> C;
+#pragma unroll
     for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) C.m[i][j] = mk<double>(0.0, 0.0);
-    for (int g = 0; g < groups; g++) {
-        const double *p = partial + ((size_t)g * L.V + site) * kForce3PerSite + 18 * mu;
-        for (int i = 0; i < 3; i++)
-            for (int j = 0; j < 3; j++) C.m[i][j] = C.m[i][j] + mk<double>(p[2 * (3 * i + j)], p[2 * (3 * i + j) + 1]);
-    }
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            C.m[i][j] = mk<double>(__shfl_sync(0xffffffffu, v, 2 * (3 * i + j)), __shfl_sync(0xffffffffu, v, 2 * (3 * i + j) + 1));
     const Links3<false, U1> lk{U, u1, L.N0 * L.N1};
     const cmat3<double> M = lk.template get<double>(site, mu);
     cmat3<double> Q;  // M C^T
+#pragma unroll
     for (int k = 0; k < 3; k++)
+#pragma unroll
         for (int i = 0; i < 3; i++) Q.m[k][i] = M.m[k][0] * C.m[i][0] + M.m[k][1] * C.m[i][1] + M.m[k][2] * C.m[i][2];
+    if (lane >= 8) return;
     // Im tr(t^a Q) per generator (t^a = lambda^a / 2)
     const double r3 = 0.57735026918962576451;
     double f[8];
@@ -814,12 +773,13 @@ __global__ void su3_force_finish_kernel(const double *__restrict__ partial, int 
     f[5] = 0.5 * (Q.m[2][1].im + Q.m[1][2].im);
     f[6] = 0.5 * (Q.m[1][2].re - Q.m[2][1].re);
     f[7] = 0.5 * r3 * (Q.m[0][0].im + Q.m[1][1].im - 2.0 * Q.m[2][2].im);
-    const double sc = 1.0 / (2.0 * L.V);
-    const size_t o = 8 * (size_t)t;
-    for (int a = 0; a < 8; a++) {
-        if (out) out[o + a] = sc * f[a];
-        else E[o + a] += coef * sc * f[a];
-    }
+    double fa = f[0];
+#pragma unroll
+    for (int a = 1; a < 8; a++) fa = lane == a ? f[a] : fa;
+    fa *= 1.0 / (2.0 * L.V);
+    const size_t o = 8 * (size_t)t + lane;
+    if (out) out[o] = fa;
+    else E[o] += coef * fa;
 }
 
 int su3_force_groups(int n_mb) { return n_mb < 16 ? n_mb : 16; }
@@ -832,12 +792,12 @@ template <typename T>
 void su3_launch_color_force(const double *U, const double *u1, const void *psi, const Lattice &L, int n_mb, int n_modes,
                             int first_mode, double *partial, double *out, double *E, double coef, cudaStream_t s) {
     const int groups = su3_force_groups(n_mb);
-    const dim3 block(kModeBlock, kSites3), grid((L.V + kSites3 - 1) / kSites3, groups);
-    su3_force_modes_kernel<T><<<grid, block, 0, s>>>(reinterpret_cast<const cpx<T> *>(psi), L, n_mb, n_modes,
-                                                      first_mode, partial);
-    const int n = 3 * L.V;
-    if (u1) su3_force_finish_kernel<true><<<(n + 127) / 128, 128, 0, s>>>(partial, groups, U, u1, L, out, E, coef);
-    else su3_force_finish_kernel<false><<<(n + 127) / 128, 128, 0, s>>>(partial, groups, U, u1, L, out, E, coef);
+    const dim3 block(kModeBlock, kSites3), grid((L.V + kSites3 - 1) / kSites3, groups, 3);
+    su3_force_modes_kernel<T><<<grid, block, 0, s>>>(SrcPlain<T>{reinterpret_cast<const cpx<T> *>(psi)}, L, n_mb, n_modes,
+                                                     first_mode, partial);
+    const int n = (3 * L.V + 3) / 4;  // four links (warps) per CTA
+    if (u1) su3_force_finish_kernel<true><<<n, 128, 0, s>>>(partial, groups, U, u1, L, out, E, coef);
+    else su3_force_finish_kernel<false><<<n, 128, 0, s>>>(partial, groups, U, u1, L, out, E, coef);
 }
 
 // sum_m w_m Re <psi_m, i (D psi)_m> / 2V from psi and D psi (ovl_force.cu's
