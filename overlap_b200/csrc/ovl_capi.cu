@@ -1452,16 +1452,17 @@ static int step_observe(ovl_ctx *c, int nsteps, double *out, bool async) {
             return fail(c, OVL_E_OOM, "ovl_step_observe: partial sums");
         }
     }
+    int nl = 0;
     if (pipe_obs) {
         if ((rc = grouped_step(c, c->obs_partial))) return rc;
         c->tsteps++;
         if ((rc = coupled_efield(c))) return rc;
         {
             ProfScope ps(c, OVL_PROF_OBS);
-            ovl::launch_obs_finish(c->obs_partial, ovl::pipeline_obs_rows(c->L, c->n_mb, c->mode_group),
-                                   c->obs_scratch, 1.0 / (2.0 * c->L.V), c->dev_small + 32, c->stream);
+            nl = ovl::launch_obs_finish(c->obs_partial, ovl::pipeline_obs_rows(c->L, c->n_mb, c->mode_group),
+                                        c->obs_scratch, 1.0 / (2.0 * c->L.V), c->dev_small + 32, c->stream);
         }
-        if ((rc = launched(c, 2, "charges (observing step)"))) return rc;
+        if ((rc = launched(c, nl, "charges (observing step)"))) return rc;
         OVL_CUDA(c, cudaMemcpyAsync(async ? out : c->host_small + 32, c->dev_small + 32, sizeof(double) * 3,
                                     cudaMemcpyDeviceToHost, c->stream));
         if (async) return OVL_OK;  // a timed-out wait is reported by ovl_synchronize
@@ -1506,10 +1507,10 @@ static int step_observe(ovl_ctx *c, int nsteps, double *out, bool async) {
     if ((rc = coupled_efield(c))) return rc;
     {
         ProfScope ps(c, OVL_PROF_OBS);
-        ovl::launch_obs_finish(c->obs_partial, obs_rows, c->obs_scratch,
-                               1.0 / (2.0 * c->L.V), c->dev_small + 32, c->stream);
+        nl = ovl::launch_obs_finish(c->obs_partial, obs_rows, c->obs_scratch, 1.0 / (2.0 * c->L.V), c->dev_small + 32,
+                                    c->stream);
     }
-    if ((rc = launched(c, 2, "charges (observing step)"))) return rc;
+    if ((rc = launched(c, nl, "charges (observing step)"))) return rc;
     OVL_CUDA(c, cudaMemcpyAsync(async ? out : c->host_small + 32, c->dev_small + 32, sizeof(double) * 3,
                                 cudaMemcpyDeviceToHost, c->stream));
     if (async) return OVL_OK;
@@ -1694,8 +1695,7 @@ int cool_record(CoolRun &r, bool after_step) {
     ovl_ctx *c = r.c;
     if (r.rows >= r.max_rows) return fail(c, OVL_E_ARG, "ovl_cool: log rows");
     double *v = r.vals + (size_t)kCoolVals * r.rows;
-    if (su3(c)) ovl::su3_launch_bulk(r.U, r.E, r.L, c->partial, v + 2, c->stream);
-    else ovl::launch_bulk(r.U, r.E, r.L, c->partial, v + 2, c->stream);
+    ovl::launch_bulk(r.U, r.E, r.L, c->partial, v + 2, c->stream, c->nc);
     ovl::launch_vacuum_ncs(r.U, r.L, c->nc, c->partial, v + 12, c->stream);
     r.row_a.push_back(r.a);
     r.row_tau.push_back(r.tau);
@@ -2098,8 +2098,7 @@ int ovl_bulk(ovl_ctx *c, double out[10]) {
     if (!c || !out) return OVL_E_ARG;
     int rc = set_device(c);
     if (rc) return rc;
-    if (su3(c)) ovl::su3_launch_bulk(c->U, c->E, c->L, c->partial, c->dev_small, c->stream);
-    else ovl::launch_bulk(c->U, c->E, c->L, c->partial, c->dev_small, c->stream);
+    ovl::launch_bulk(c->U, c->E, c->L, c->partial, c->dev_small, c->stream, c->nc);
     if ((rc = launched(c, 2, "bulk"))) return rc;
     OVL_CUDA(c, cudaMemcpyAsync(c->host_small, c->dev_small, sizeof(double) * 10, cudaMemcpyDeviceToHost, c->stream));
     OVL_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -53,8 +53,33 @@ struct CompSum {
         c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
         s = t;
     }
+    // Adds another compensated sum: its rounding part and the rounding of the
+    // two leading parts' sum go into c.
+    __host__ __device__ void merge(double os, double oc) {
+        add(os);
+        c += oc;
+    }
     __host__ __device__ double value() const { return s + c; }
 };
+#ifdef __CUDACC__
+// Merges t over the warp's lanes in a fixed tree; every lane returns the total.
+__device__ __forceinline__ void warp_merge(CompSum &t) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double os = __shfl_xor_sync(0xffffffffu, t.s, o), oc = __shfl_xor_sync(0xffffffffu, t.c, o);
+        // the same pair order in both lanes, so that both hold the same bits
+        CompSum a = t;
+        if (threadIdx.x & o) {
+            a.s = os;
+            a.c = oc;
+            a.merge(t.s, t.c);
+        } else {
+            a.merge(os, oc);
+        }
+        t = a;
+    }
+}
+#endif
 
 // ----------------------------------------------------------------- complex --
 // The GPU's global nanosecond timer (bounds for waits on other CTAs).

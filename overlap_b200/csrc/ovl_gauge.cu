@@ -69,32 +69,6 @@ void launch_update_links(double *U, const double *E, const Lattice &L, double dt
                                                              reunit ? 1 : 0);
 }
 
-// ------------------------------------------------------- Wilson loops ------
-__device__ inline quat path_step(const double *__restrict__ U, const Lattice &L, int c[3], int mu, int dir, quat acc) {
-    if (dir > 0) {
-        quat u = load_link(U, site_index(L, c[0], c[1], c[2]), mu);
-        c[mu] += 1;
-        return qmul(acc, u);
-    }
-    c[mu] -= 1;
-    return qmul(acc, qdag(load_link(U, site_index(L, c[0], c[1], c[2]), mu)));
-}
-
-// Counter-clockwise lmu x lnu loop in the (mu, nu) plane with (x, y, z) at its
-// corner in quadrant (smu, snu), holonomy based at that corner.
-__device__ quat loop(const double *__restrict__ U, const Lattice &L, int x, int y, int z, int mu, int nu, int smu,
-                     int snu, int lmu, int lnu) {
-    const int dmu[4] = {mu, nu, mu, nu}, ddir[4] = {+1, +1, -1, -1}, dlen[4] = {lmu, lnu, lmu, lnu};
-    const int start = (smu > 0 && snu > 0) ? 0 : (smu < 0 && snu > 0) ? 1 : (smu < 0 && snu < 0) ? 2 : 3;
-    int c[3] = {x, y, z};
-    quat acc = {0.0, 0.0, 0.0, 1.0};
-    for (int k = 0; k < 4; k++) {
-        const int j = (start + k) & 3;
-        for (int n = 0; n < dlen[j]; n++) acc = path_step(U, L, c, dmu[j], ddir[j], acc);
-    }
-    return acc;
-}
-
 // ------------------------------------------------------------ staple force --
 // E^a_mu(x) += -2 dt sum_{nu != mu} [Re tr(i t^a U_{mu,nu}) + Re tr(i t^a U_{mu,-nu})],
 // both staples written to start with U_mu(x) (Dynamics.cpp:145-197).
@@ -310,85 +284,139 @@ void launch_sphaleron(double *U, double *E, double *Ufinal, const Lattice &L, do
 }
 
 // ------------------------------------------------------------------- bulk --
-// Per-thread sums: E^2 per direction (3), B^2 per direction (3), Gauss
-// violation squares, unitarity squares, unitarity max, Gauss max (last, max-reduced).
+// E^2 per direction (3), B^2_k = 4 Re tr(1 - U_plaq) of the plaquette orthogonal
+// to k (3, BulkObservables.cpp:72-77), Gauss violation squares, unitarity
+// squares, and the maxima of the Gauss violation (signed, from 0,
+// GaussLawViolation.cpp:44) and of the unitarity violation.  Four lanes per site,
+// lane q < 3 with direction and plane q; the Gauss vector is summed over them.
 constexpr int kBulkVals = 10;
+constexpr int kBulkThreads = 128;
 
-__global__ void __launch_bounds__(kReduceThreads) bulk_kernel(const double *__restrict__ U, const double *__restrict__ E,
-                                                               Lattice L, double *partial) {
-    __shared__ double sh[32 * kBulkVals];
+// V (t^b e^b) V^+ as components.
+__device__ __forceinline__ void transport(const quat &V, const double *__restrict__ e, double *out) {
+    const adj3 R = adjoint(V);
+    const double e0 = e[0], e1 = e[1], e2 = e[2];
+#pragma unroll
+    for (int a = 0; a < 3; a++) out[a] = R.r[a][0] * e0 + R.r[a][1] * e1 + R.r[a][2] * e2;
+}
+__device__ __forceinline__ void transport(const cmat3<double> &V, const double *__restrict__ e, double *out) {
+    su3_components(m3_mul(m3_mul(V, su3_form(e)), m3_dag(V)), out);
+}
+// 4 Re tr(1 - P)
+__device__ __forceinline__ double plaquette_action(const quat &p) { return 4.0 * 2.0 * (1.0 - p.s); }
+__device__ __forceinline__ double plaquette_action(const cmat3<double> &p) {
+    return 4.0 * (3.0 - (p.m[0][0].re + p.m[1][1].re + p.m[2][2].re));
+}
+// The unitarity violation of a link and its square.
+__device__ __forceinline__ void unitarity(const quat &u, double &dev, double &dev2) {
+    dev = fabs(u.v0 * u.v0 + u.v1 * u.v1 + u.v2 * u.v2 + u.s * u.s - 1.0);
+    dev2 = dev * dev;
+}
+__device__ __forceinline__ void unitarity(const cmat3<double> &u, double &dev, double &dev2) {
+    const cmat3<double> cc = m3_mul(u, m3_dag(u));
+    dev2 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const double re = cc.m[i][j].re - (i == j ? 1.0 : 0.0), im = cc.m[i][j].im;
+            dev2 += re * re + im * im;
+        }
+    dev = sqrt(dev2);
+}
+
+template <class OPS, int NA>
+__global__ void __launch_bounds__(kBulkThreads) bulk_kernel(const double *__restrict__ U, const double *__restrict__ E,
+                                                            Lattice L, double *__restrict__ partial) {
+    __shared__ double sh[kBulkThreads / 32][kBulkVals];
     double v[kBulkVals];
+#pragma unroll
     for (int k = 0; k < kBulkVals; k++) v[k] = 0.0;
-    double umax = 0.0, gmax = 0.0;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < L.V; s += gridDim.x * blockDim.x) {
-        int x, y, z;
-        site_coords(L, s, x, y, z);
-        for (int mu = 0; mu < 3; mu++)
-            for (int a = 0; a < 3; a++) {
-                double e = E[a + 3 * (mu + 3 * s)];
-                v[mu] += e * e;
+    const long long items = 4LL * L.V, stride = (long long)gridDim.x * kBulkThreads;
+    for (long long t0 = (long long)blockIdx.x * kBulkThreads + (threadIdx.x & ~31); t0 < items; t0 += stride) {
+        const long long t = t0 + (threadIdx.x & 31);
+        const int q = (int)(t & 3), mu = q < 3 ? q : 0;
+        const bool site_live = t < items, live = site_live && q < 3;  // the shuffles need every lane
+        const int s = site_live ? (int)(t >> 2) : 0;
+        int c[3];
+        site_coords(L, s, c[0], c[1], c[2]);
+        double g[NA];
+        {
+            const double *e = E + NA * (mu + 3 * (size_t)s);
+            const int cm = mu == 0 ? c[0] : (mu == 1 ? c[1] : c[2]);
+            const int sm = s + wrap_offset(cm, extent_of(L, mu), stride_of(L, mu), -1);
+            double w[NA], e2 = 0.0;
+            transport(OPS::dag(OPS::load(U, sm, mu)), E + NA * (mu + 3 * (size_t)sm), w);
+#pragma unroll
+            for (int a = 0; a < NA; a++) {
+                const double ea = e[a];
+                e2 += ea * ea;
+                g[a] = live ? ea - w[a] : 0.0;
             }
-        // B^2_k = 4 Re tr(1 - U_plaq) of the plaquette orthogonal to k (BulkObservables.cpp:72-77)
-        const int plane[3][2] = {{1, 2}, {2, 0}, {0, 1}};
-        for (int k = 0; k < 3; k++) {
-            quat pl = loop(U, L, x, y, z, plane[k][0], plane[k][1], +1, +1, 1, 1);
-            v[3 + k] += 4.0 * 2.0 * (1.0 - pl.s);
-        }
-        // G^a = sum_mu E_mu(x) - (U^+ E U)(x - mu)
-        double g[3] = {0.0, 0.0, 0.0};
-        for (int mu = 0; mu < 3; mu++) {
-            int c[3] = {x, y, z};
-            c[mu] -= 1;
-            const int sm = site_index(L, c[0], c[1], c[2]);
-            adj3 R = adjoint(qdag(load_link(U, sm, mu)));
-            for (int a = 0; a < 3; a++) {
-                double t = E[a + 3 * (mu + 3 * s)];
-                for (int b = 0; b < 3; b++) t -= R.r[a][b] * E[b + 3 * (mu + 3 * sm)];
-                g[a] += t;
+            const Quadrant quad(L, s, c, mu == 2 ? 0 : mu + 1, mu == 0 ? 2 : mu - 1, 0);
+            const double b2 = plaquette_action(OPS::mul(OPS::mul(quad.a<OPS>(U, 0, 0), quad.b<OPS>(U, 1, 0)),
+                                                        OPS::dag(OPS::mul(quad.b<OPS>(U, 0, 0), quad.a<OPS>(U, 0, 1)))));
+            double dev, dev2;
+            unitarity(OPS::load(U, s, mu), dev, dev2);
+            if (live) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    v[k] += k == q ? e2 : 0.0;
+                    v[3 + k] += k == q ? b2 : 0.0;
+                }
+                v[7] += dev2;
+                v[9] = fmax(v[9], dev);
             }
         }
-        for (int a = 0; a < 3; a++) {
-            gmax = fmax(gmax, g[a]);  // signed maximum, as GaussLawViolation.cpp:44
-            v[6] += g[a] * g[a];
-        }
-        for (int mu = 0; mu < 3; mu++) {
-            quat u = load_link(U, s, mu);
-            double dev = fabs(u.v0 * u.v0 + u.v1 * u.v1 + u.v2 * u.v2 + u.s * u.s - 1.0);
-            umax = fmax(umax, dev);
-            v[7] += dev * dev;
+#pragma unroll
+        for (int a = 0; a < NA; a++) {
+            const double ga = quad_sum(g[a]);
+            if (site_live && q == 0) {
+                v[6] += ga * ga;
+                v[8] = fmax(v[8], ga);
+            }
         }
     }
-    v[8] = umax;
-    v[9] = gmax;
-    // max-reduce slot 8 by hand; block_reduce max-reduces only the last slot
-    double vm[1] = {v[8]};
-    v[8] = 0.0;
-    block_reduce<kBulkVals, true>(v, sh);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < kBulkVals; k++) {
+        double t = v[k];
+        for (int o = 16; o > 0; o >>= 1) {
+            const double u = __shfl_down_sync(0xffffffffu, t, o);
+            t = k >= 8 ? fmax(t, u) : t + u;
+        }
+        if (lane == 0) sh[warp][k] = t;
+    }
     __syncthreads();
-    double t = vm[0];
-    for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_down_sync(0xffffffffu, t, o));
-    __shared__ double shm[32];
-    if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) t = fmax(t, shm[w]);
-        for (int k = 0; k < kBulkVals; k++) partial[(size_t)blockIdx.x * (kBulkVals + 1) + k] = v[k];
-        partial[(size_t)blockIdx.x * (kBulkVals + 1) + kBulkVals] = t;
+    if (threadIdx.x < kBulkVals) {
+        const int k = threadIdx.x;
+        double t = sh[0][k];
+        for (int w = 1; w < kBulkThreads / 32; w++) t = k >= 8 ? fmax(t, sh[w][k]) : t + sh[w][k];
+        partial[(size_t)blockIdx.x * kBulkVals + k] = t;
     }
 }
 
-__global__ void bulk_finish_kernel(const double *__restrict__ partial, int n, Lattice L, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One warp: lanes over the CTAs' rows, compensated sums merged over the lanes.
+__global__ void bulk_finish_kernel(const double *__restrict__ partial, int n, Lattice L, int na, double *out) {
+    const int lane = threadIdx.x;
     CompSum cs[8];
     double gmax = 0.0, umax = 0.0;
-    for (int i = 0; i < n; i++) {
-        const double *p = partial + (size_t)i * (kBulkVals + 1);
+    for (int i = lane; i < n; i += 32) {
+        const double *p = partial + (size_t)i * kBulkVals;
         for (int k = 0; k < 8; k++) cs[k].add(p[k]);
-        gmax = fmax(gmax, p[9]);
-        umax = fmax(umax, p[10]);
+        gmax = fmax(gmax, p[8]);
+        umax = fmax(umax, p[9]);
     }
     double s[8];
-    for (int k = 0; k < 8; k++) s[k] = cs[k].value();
+    for (int k = 0; k < 8; k++) {
+        warp_merge(cs[k]);
+        s[k] = cs[k].value();
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        gmax = fmax(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+        umax = fmax(umax, __shfl_xor_sync(0xffffffffu, umax, o));
+    }
+    if (lane != 0) return;
     const double V = (double)L.V;
     double e2[3], b2[3];
     for (int k = 0; k < 3; k++) { e2[k] = s[k] / V; b2[k] = s[3 + k] / V; }
@@ -399,7 +427,7 @@ __global__ void bulk_finish_kernel(const double *__restrict__ partial, int n, La
     out[4] = 0.5 * (e2[0] + e2[1] + e2[2]);
     out[5] = 0.5 * (b2[0] + b2[1] + b2[2]);
     out[6] = gmax;
-    out[7] = sqrt(s[6] / (3.0 * V));
+    out[7] = sqrt(s[6] / (na * V));  // over the Nc^2 - 1 components (GaussLawViolation.cpp:64)
     out[8] = umax;
     out[9] = sqrt(s[7] / (3.0 * V));
 }
@@ -476,12 +504,19 @@ void launch_gauss_update(const double *U, const double *G, double *E, const Latt
     gauss_update_kernel<<<(n + 127) / 128, 128, 0, stream>>>(U, G, E, L, gamma);
 }
 
-size_t bulk_partial_doubles(const Lattice &L) { return (size_t)reduce_blocks(L.V) * (kBulkVals + 1); }
+static int bulk_blocks(const Lattice &L) {
+    const long long b = (4LL * L.V + kBulkThreads - 1) / kBulkThreads;
+    return b < 1024 ? (int)b : 1024;
+}
 
-void launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream) {
-    const int nb = reduce_blocks(L.V);
-    bulk_kernel<<<nb, kReduceThreads, 0, stream>>>(U, E, L, partial);
-    bulk_finish_kernel<<<1, 32, 0, stream>>>(partial, nb, L, out);
+size_t bulk_partial_doubles(const Lattice &L) { return (size_t)bulk_blocks(L) * kBulkVals; }
+
+void launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream,
+                 int nc) {
+    const int nb = bulk_blocks(L);
+    if (nc == 3) bulk_kernel<Su3Ops, 8><<<nb, kBulkThreads, 0, stream>>>(U, E, L, partial);
+    else bulk_kernel<Su2Ops, 3><<<nb, kBulkThreads, 0, stream>>>(U, E, L, partial);
+    bulk_finish_kernel<<<1, 32, 0, stream>>>(partial, nb, L, nc * nc - 1, out);
 }
 
 // ------------------------------------------------------------- cooling ----

@@ -49,8 +49,9 @@ size_t launch_wilson_observe(const HopConfig &hc, const void *src, void *dst, co
 void launch_wilson40_observe(const HopConfig &hc, const void *src, const void *src_lo, void *dst, void *dst_lo,
                              const Lattice &L, int n_mb, double amass, double dt, int n_modes, int first_mode,
                              double *partial, cudaStream_t stream);
-void launch_obs_finish(const double *partial, size_t rows, double *scratch, double scale, double *out3,
-                       cudaStream_t stream);
+// Returns the kernels launched.
+int launch_obs_finish(const double *partial, size_t rows, double *scratch, double scale, double *out3,
+                      cudaStream_t stream);
 // The grouped fused step in one persistent launch (FP32 packed pairs, hop
 // variant 3): b += dt D a with links h1 and then c += dt D b with links h2,
 // group by group of `group` mode blocks, each group's second half step while
@@ -124,7 +125,8 @@ void launch_gauss_violation(const double *U, const double *E, const Lattice &L, 
                             double *out, cudaStream_t stream);
 void launch_gauss_update(const double *U, const double *G, double *E, const Lattice &L, double gamma,
                          cudaStream_t stream);
-void launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream);
+void launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t stream,
+                 int nc = 2);
 
 // Currents: 16 doubles per site (jV[4], jA[4], jVw[4], jAw[4]) + PS + WA = 18.
 constexpr int kCurrentsPerSite = 18;
@@ -333,8 +335,6 @@ void su3_launch_ncsdot3(const double *U0, const double *U1, const double *U2, co
                         double *partial, double *out3, cudaStream_t stream);
 void su3_launch_geodesic(const double *Uold, const double *Unew, double c, double *Umid, double *Emid, const Lattice &L,
                          cudaStream_t stream);
-void su3_launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out,
-                     cudaStream_t stream);
 // out2 = {sum of G^2, signed maximum}; G holds 8 components per site.
 void su3_launch_gauss_violation(const double *U, const double *E, const Lattice &L, double *G, double *partial,
                                 double *out2, cudaStream_t stream);

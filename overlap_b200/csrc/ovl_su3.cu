@@ -278,34 +278,6 @@ __global__ void su3_sum_rows_kernel(const double *__restrict__ partial, int n, d
         for (int k = 0; k < NV; k++) out[k] = scale * sh[0][k];
 }
 
-// ----------------------------------------------------------- Wilson loops --
-__device__ inline cmat3<double> su3_step(const double *__restrict__ U, const Lattice &L, int c[3], int mu, int dir,
-                                         const cmat3<double> &acc) {
-    if (dir > 0) {
-        const cmat3<double> u = load_su3(U, site_index(L, c[0], c[1], c[2]), mu);
-        c[mu] += 1;
-        return m3_mul(acc, u);
-    }
-    c[mu] -= 1;
-    return m3_mul(acc, m3_dag(load_su3(U, site_index(L, c[0], c[1], c[2]), mu)));
-}
-
-// Counter-clockwise lmu x lnu loop in the (mu, nu) plane with (x, y, z) at its
-// corner in quadrant (smu, snu), holonomy based at that corner (loop() in
-// ovl_gauge.cu).
-__device__ cmat3<double> su3_loop(const double *__restrict__ U, const Lattice &L, int x, int y, int z, int mu, int nu,
-                                  int smu, int snu, int lmu, int lnu) {
-    const int dmu[4] = {mu, nu, mu, nu}, ddir[4] = {+1, +1, -1, -1}, dlen[4] = {lmu, lnu, lmu, lnu};
-    const int start = (smu > 0 && snu > 0) ? 0 : (smu < 0 && snu > 0) ? 1 : (smu < 0 && snu < 0) ? 2 : 3;
-    int c[3] = {x, y, z};
-    cmat3<double> acc = m3_unit<double>();
-    for (int k = 0; k < 4; k++) {
-        const int j = (start + k) & 3;
-        for (int n = 0; n < dlen[j]; n++) acc = su3_step(U, L, c, dmu[j], ddir[j], acc);
-    }
-    return acc;
-}
-
 // V (t^b e^b) V^+ as components: the adjoint transport R(V) e, R_ab = 2 tr(t^a V t^b V^+).
 __device__ inline void su3_transport(const cmat3<double> &V, const double *e, double *out) {
     const cmat3<double> A = su3_form(e);
@@ -482,110 +454,6 @@ void su3_launch_geodesic(const double *Uold, const double *Unew, double c, doubl
                          cudaStream_t s) {
     const int n = 3 * L.V;
     su3_geodesic_kernel<<<(n + 127) / 128, 128, 0, s>>>(Uold, Unew, c, Umid, Emid, n);
-}
-
-// ------------------------------------------------------------------- bulk --
-// E^2 (3), B^2 = 4 Re tr(1 - U_plaq) (3), Gauss squares, unitarity squares,
-// Gauss max, unitarity max per CTA (bulk_kernel of ovl_gauge.cu for three colours).
-__global__ void __launch_bounds__(kReduce3Threads)
-    su3_bulk_kernel(const double *__restrict__ U, const double *__restrict__ E, Lattice L, double *partial) {
-    __shared__ double sh[32];
-    double v[10];
-    for (int k = 0; k < 10; k++) v[k] = 0.0;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < L.V) {
-        int x, y, z;
-        site_coords(L, s, x, y, z);
-        for (int mu = 0; mu < 3; mu++)
-            for (int a = 0; a < 8; a++) {
-                const double e = E[a + 8 * (mu + 3 * s)];
-                v[mu] += e * e;
-            }
-        const int plane[3][2] = {{1, 2}, {2, 0}, {0, 1}};
-        for (int k = 0; k < 3; k++) {
-            const cmat3<double> pl = su3_loop(U, L, x, y, z, plane[k][0], plane[k][1], +1, +1, 1, 1);
-            v[3 + k] = 4.0 * (3.0 - (pl.m[0][0].re + pl.m[1][1].re + pl.m[2][2].re));
-        }
-        double g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int mu = 0; mu < 3; mu++) {
-            int c[3] = {x, y, z};
-            c[mu] -= 1;
-            const int sm = site_index(L, c[0], c[1], c[2]);
-            double t[8];
-            su3_transport(m3_dag(load_su3(U, sm, mu)), E + 8 * (mu + 3 * sm), t);
-            for (int a = 0; a < 8; a++) g[a] += E[a + 8 * (mu + 3 * s)] - t[a];
-        }
-        double gmax = -1e300;
-        for (int a = 0; a < 8; a++) {
-            gmax = fmax(gmax, g[a]);
-            v[6] += g[a] * g[a];
-        }
-        v[8] = gmax;
-        double umax = 0.0;
-        for (int mu = 0; mu < 3; mu++) {
-            const cmat3<double> u = load_su3(U, s, mu), cc = m3_mul(u, m3_dag(u));
-            double n = 0.0;
-            for (int i = 0; i < 3; i++)
-                for (int j = 0; j < 3; j++) {
-                    const double re = cc.m[i][j].re - (i == j ? 1.0 : 0.0), im = cc.m[i][j].im;
-                    n += re * re + im * im;
-                }
-            umax = fmax(umax, sqrt(n));
-            v[7] += n;
-        }
-        v[9] = umax;
-    } else {
-        v[8] = -1e300;
-    }
-    // sums of slots 0..7, maxima of 8 (Gauss, signed) and 9 (unitarity)
-    double out[10];
-    for (int k = 0; k < 8; k++) out[k] = block_sum(v[k], sh);
-    for (int k = 8; k < 10; k++) {
-        double t = v[k];
-        for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_down_sync(0xffffffffu, t, o));
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
-        __syncthreads();
-        t = -1e300;
-        if (threadIdx.x == 0)
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) t = fmax(t, sh[w]);
-        __syncthreads();
-        out[k] = t;
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 10; k++) partial[(size_t)blockIdx.x * 10 + k] = out[k];
-}
-
-__global__ void su3_bulk_finish_kernel(const double *__restrict__ partial, int n, Lattice L, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    CompSum cs[8];
-    double gmax = -1e300, umax = 0.0;
-    for (int i = 0; i < n; i++) {
-        const double *p = partial + (size_t)i * 10;
-        for (int k = 0; k < 8; k++) cs[k].add(p[k]);
-        gmax = fmax(gmax, p[8]);
-        umax = fmax(umax, p[9]);
-    }
-    double s[8];
-    for (int k = 0; k < 8; k++) s[k] = cs[k].value();
-    const double V = (double)L.V;
-    double e2[3], b2[3];
-    for (int k = 0; k < 3; k++) { e2[k] = s[k] / V; b2[k] = s[3 + k] / V; }
-    out[0] = 0.5 * (e2[0] + e2[1] + e2[2] + b2[0] + b2[1] + b2[2]);
-    out[1] = 0.5 * ((e2[1] + e2[2] + b2[1] + b2[2]) - (e2[0] + b2[0]));
-    out[2] = 0.5 * ((e2[0] + e2[2] + b2[0] + b2[2]) - (e2[1] + b2[1]));
-    out[3] = 0.5 * ((e2[0] + e2[1] + b2[0] + b2[1]) - (e2[2] + b2[2]));
-    out[4] = 0.5 * (e2[0] + e2[1] + e2[2]);
-    out[5] = 0.5 * (b2[0] + b2[1] + b2[2]);
-    out[6] = fmax(gmax, 0.0);
-    out[7] = sqrt(s[6] / (8.0 * V));  // over the Nc^2 - 1 components (GaussLawViolation.cpp:64)
-    out[8] = umax;
-    out[9] = sqrt(s[7] / (3.0 * V));
-}
-
-void su3_launch_bulk(const double *U, const double *E, const Lattice &L, double *partial, double *out, cudaStream_t s) {
-    const int nb = (L.V + kReduce3Threads - 1) / kReduce3Threads;
-    su3_bulk_kernel<<<nb, kReduce3Threads, 0, s>>>(U, E, L, partial);
-    su3_bulk_finish_kernel<<<1, 32, 0, s>>>(partial, nb, L, out);
 }
 
 // ------------------------------------------------------------ staple force --
