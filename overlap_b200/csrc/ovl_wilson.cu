@@ -167,40 +167,62 @@ __device__ __forceinline__ void cta_partial(double (&o)[kObsVals], double *__res
 constexpr int kPkWarps = 4, kPkDepth = 2, kPkMinBlocks = 3;
 constexpr int kPkCtaSites = 2 * kPkWarps;
 
-template <int MODE, bool U1, bool OBS>
+// MBLK: mode blocks per CTA (kPkBlocks, or kPkFewBlocks for launches too small to
+// give most SMs a CTA, packed_mblk).
+constexpr int kPkFewBlocks = 2;
+
+template <int MODE, bool U1, bool OBS, int MBLK>
 __global__ void __launch_bounds__(kModeBlock *kPkWarps, kPkMinBlocks)
     wilson_packed_kernel(const float4 *__restrict__ U32, const float2 *__restrict__ u1, const float4 *__restrict__ src,
                          float4 *__restrict__ dst, Lattice L, int n_mb, float amass, float hdt, int n_modes,
                          int first_mode, double *__restrict__ partial) {
     __shared__ float4 rec[kPkCtaSites][6][kPkRecVec];
-    const int mb0 = blockIdx.y * kPkBlocks;
+    const int mb0 = blockIdx.y * MBLK;
     double o[kObsVals] = {0.0, 0.0, 0.0};
     packed_tile<MODE, U1, OBS, kPkWarps, kPkDepth>(rec, U32, u1, src, dst, L, blockIdx.x * kPkCtaSites, mb0,
-                                                   min(n_mb, mb0 + kPkBlocks), amass, hdt, n_modes, first_mode, o);
+                                                   min(n_mb, mb0 + MBLK), amass, hdt, n_modes, first_mode, o);
     if (OBS) cta_partial(o, partial);
 }
 
 
-// Rows of kObsVals partial sums the packed observing launch writes.
-size_t packed_obs_rows(const Lattice &L, int n_mb) {
-    return (size_t)((L.V + kPkCtaSites - 1) / kPkCtaSites) * ((n_mb + kPkBlocks - 1) / kPkBlocks);
+// CTAs of the packed launch along the sites, and mode blocks per CTA.
+static int packed_tiles(const Lattice &L) { return (L.V + kPkCtaSites - 1) / kPkCtaSites; }
+static int packed_mblk(const Lattice &L, int n_mb) {
+    // three quarters of a CTA per SM, of the three that run on one: at 8^3 x 256
+    // modes 64 CTAs with 8 took 15.9 us per step, 256 with 2 12.0 (three contexts in
+    // turn); at 12^3 x 256 216 with 8 33.0, 432 with 4 33.6
+    return mode_blocks_per_cta(packed_tiles(L), n_mb, 3 * current_sm_count() / 4) == kPkBlocks ? kPkBlocks : kPkFewBlocks;
 }
 
-template <int MODE, bool OBS>
-static void launch_packed(const HopConfig &hc, const void *src, void *dst, const Lattice &L, int n_mb, double amass,
-                          double dt, int n_modes, int first_mode, double *partial, cudaStream_t stream) {
-    const dim3 block(kModeBlock, kPkWarps),
-        grid((L.V + kPkCtaSites - 1) / kPkCtaSites, (n_mb + kPkBlocks - 1) / kPkBlocks);
+// Rows of kObsVals partial sums the packed observing launch writes.
+size_t packed_obs_rows(const Lattice &L, int n_mb) {
+    const int m = packed_mblk(L, n_mb);
+    return (size_t)packed_tiles(L) * ((n_mb + m - 1) / m);
+}
+
+template <int MODE, bool OBS, int MBLK>
+static void launch_packed_m(const HopConfig &hc, const void *src, void *dst, const Lattice &L, int n_mb, double amass,
+                            double dt, int n_modes, int first_mode, double *partial, cudaStream_t stream) {
+    const dim3 block(kModeBlock, kPkWarps), grid(packed_tiles(L), (n_mb + MBLK - 1) / MBLK);
     const float4 *U = reinterpret_cast<const float4 *>(hc.U32);
     const float4 *s = reinterpret_cast<const float4 *>(src);
     float4 *d = reinterpret_cast<float4 *>(dst);
     const float a = (float)amass, h = (float)(0.5 * dt);
     if (hc.u1_32)
-        wilson_packed_kernel<MODE, true, OBS><<<grid, block, 0, stream>>>(
+        wilson_packed_kernel<MODE, true, OBS, MBLK><<<grid, block, 0, stream>>>(
             U, reinterpret_cast<const float2 *>(hc.u1_32), s, d, L, n_mb, a, h, n_modes, first_mode, partial);
     else
-        wilson_packed_kernel<MODE, false, OBS><<<grid, block, 0, stream>>>(U, nullptr, s, d, L, n_mb, a, h, n_modes,
-                                                                          first_mode, partial);
+        wilson_packed_kernel<MODE, false, OBS, MBLK><<<grid, block, 0, stream>>>(U, nullptr, s, d, L, n_mb, a, h, n_modes,
+                                                                                first_mode, partial);
+}
+
+template <int MODE, bool OBS>
+static void launch_packed(const HopConfig &hc, const void *src, void *dst, const Lattice &L, int n_mb, double amass,
+                          double dt, int n_modes, int first_mode, double *partial, cudaStream_t stream) {
+    if (packed_mblk(L, n_mb) == kPkBlocks)
+        launch_packed_m<MODE, OBS, kPkBlocks>(hc, src, dst, L, n_mb, amass, dt, n_modes, first_mode, partial, stream);
+    else
+        launch_packed_m<MODE, OBS, kPkFewBlocks>(hc, src, dst, L, n_mb, amass, dt, n_modes, first_mode, partial, stream);
 }
 
 // ---------------------------------------------- pipelined grouped step --
