@@ -28,23 +28,24 @@ namespace ovl {
 // finishing kernel adds it per site.  That leaves four spinor reads and 128
 // FP64 multiply-adds per hop and mode (two colours) of the seven reads and 208.
 // What bounds the kernel is FP64 arithmetic (and, for FP32 modes, the FP32 to
-// FP64 conversions beside it): the links sit in shared memory, so that 128
-// registers hold two CTAs per SM instead of one.
-// ovl_currents at 16^3, 4096 FP32 modes: 1715 us with the seven reads (254
-// registers, FP64 pipe 52 % busy at 12 % of the warps), 924 us so.
+// FP64 conversions beside it): the links sit in shared memory instead of
+// registers, and a neighbour is converted as a whole so that the next one's
+// loads are in flight while it is used.  ovl_currents at 16^3, 4096 FP32 modes:
+// 1715 us with the seven reads (254 registers, 8 warps per SM), 924 us with four
+// reads at 128 registers (16 warps) without the loads in flight, 845 us so (168
+// registers, 12 warps), 913 us so squeezed into 128 registers.
 constexpr int kCurrentVals = 16;  // partial sums per site and group: jV0, jA0, PS, then jV, jA, jVw, jAw by mu; one spare
 
 // Slot k of the per-site output is partial value kCurrentSlot[k] (-1: zero, -2: WA).
 __constant__ int kCurrentSlot[kCurrentsPerSite] = {0, 3, 4, 5, 1, 6, 7, 8, -1, 9, 10, 11, -1, 12, 13, 14, 2, -2};
 
-// CTAs of 8 (two colours) or 4 (three) sites.
-template <int NC> struct CurrentShape { static constexpr int kSites = NC == 2 ? 8 : 4, kMinBlocks = NC == 2 ? 2 : 2; };
+constexpr int kCurrentSites = 4;  // per CTA, a warp each
 
 template <int NC, class SRC>
-__global__ void __launch_bounds__(kModeBlock *CurrentShape<NC>::kSites, CurrentShape<NC>::kMinBlocks)
+__global__ void __launch_bounds__(kModeBlock *kCurrentSites, NC == 2 ? 3 : 2)
     currents_kernel(const double *__restrict__ U, const double *__restrict__ u1, SRC psi, Lattice L, int n_mb,
                     int n_modes, int first_mode, int groups, double r, double *__restrict__ partial) {
-    constexpr int S = CurrentShape<NC>::kSites;
+    constexpr int S = kCurrentSites;
     constexpr mono G05 = mono_mul(kGamma0, kGamma5);
     constexpr mono GV[3] = {mono_mul(kGamma0, kGammaX), mono_mul(kGamma0, kGammaY), mono_mul(kGamma0, kGammaZ)};
     constexpr mono GA[3] = {mono_mul(GV[0], kGamma5), mono_mul(GV[1], kGamma5), mono_mul(GV[2], kGamma5)};
@@ -82,12 +83,18 @@ __global__ void __launch_bounds__(kModeBlock *CurrentShape<NC>::kSites, CurrentS
         }
 #pragma unroll
         for (int mu = 0; mu < 3; mu++) {
+            // the neighbour in FP64, and the next one's loads in flight while it is used
+            cpx<double> nbr[4 * NC];
+#pragma unroll
+            for (int k = 0; k < 4 * NC; k++) nbr[k] = raw.get(k);
+            if (mu == 0) raw.load(psi, V, mb, nb.yp, lane);
+            if (mu == 1) raw.load(psi, V, mb, nb.zp, lane);
             double v[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int b = 0; b < kSpin; b++) {  // chi = U_mu(x) psi(x+mu), one spin component at a time
                 cpx<double> h[NC], chi[NC];
 #pragma unroll
-                for (int j = 0; j < NC; j++) h[j] = raw.get(kSpin * j + b);
+                for (int j = 0; j < NC; j++) h[j] = nbr[kSpin * j + b];
                 link_times<NC>(tab[threadIdx.y][mu], h, chi);
                 // component b meets the row a with perm[a] = b; the permutations are involutions
                 const mono Gs[4] = {GV[mu], GA[mu], kGamma0, G05};
@@ -101,8 +108,6 @@ __global__ void __launch_bounds__(kModeBlock *CurrentShape<NC>::kSites, CurrentS
                     }
                 }
             }
-            if (mu == 0) raw.load(psi, V, mb, nb.yp, lane);
-            if (mu == 1) raw.load(psi, V, mb, nb.zp, lane);
             acc[3 + mu].add(w * v[0]);
             acc[6 + mu].add(w * v[1]);
             acc[9 + mu].add(w * (r * v[2]));
@@ -168,7 +173,7 @@ size_t currents_partial_doubles(const Lattice &L, int n_mb) {
 template <int NC, class SRC>
 static void currents_from(const SRC &src, const double *U, const double *u1, const Lattice &L, int n_mb, int n_modes,
                           int first_mode, double r_wilson, double *partial, double *per_site, cudaStream_t stream) {
-    constexpr int S = CurrentShape<NC>::kSites;
+    constexpr int S = kCurrentSites;
     const int groups = currents_groups(n_mb);
     currents_kernel<NC, SRC><<<dim3((L.V + S - 1) / S, groups), dim3(kModeBlock, S), 0, stream>>>(
         U, u1, src, L, n_mb, n_modes, first_mode, groups, r_wilson, partial);

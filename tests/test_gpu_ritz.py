@@ -60,6 +60,39 @@ def test_ritz_random_start_and_u1_background_match_oracle():
     assert r1["iters"] != r2["iters"] or r1["raw"] != r2["raw"]  # different start vectors
 
 
+# One-launch solves: clusters of 8 CTAs (64 and 990 sites, the second not filling
+# its CTAs) and of 16 (1716), the cooperative launch (2197), and the iteration
+# kernel by kernel (9600 sites, more than fit the GPU at once; the largest
+# eigenvalue only, the smallest takes the CPU half a minute).
+@pytest.mark.parametrize("N, u1", [((4, 4, 4), True), ((9, 11, 10), False), ((11, 12, 13), True), ((13, 13, 13), False),
+                                   ((24, 20, 20), False)])
+def test_ritz_at_the_edges_of_its_launch_shapes(N, u1):
+    V = volume(N)
+    U = random_links(N, 0.3, 421)
+    p = oracle_params(N, m=0.05, mdw=1.4)
+    rng = np.random.default_rng(422)
+    start = rng.uniform(0, 1, (V, 2, 4)) + 1j * rng.uniform(0, 1, (V, 2, 4))
+    ph = np.ascontiguousarray(np.exp(1j * rng.uniform(-0.3, 0.3, (N[1], N[0], 2)))) if u1 else None
+    oracle().orc_set_u1(ptr(ph.view(np.float64).ravel()) if u1 else None)
+    try:
+        it = C.c_int(0)
+        hi = -oracle().orc_ritz(C.byref(p), ptr(U), ptr(start.view(np.float64)), -1.0, 2000, 100, 1e-16, C.byref(it))
+        lo = None
+        if V < 9000:
+            lo = oracle().orc_ritz(C.byref(p), ptr(U), ptr(start.view(np.float64)), 1.0, 2000, 100, 1e-16, C.byref(it))
+    finally:
+        oracle().orc_set_u1(None)
+    with Context(N=N, n_modes=1, fermion="overlap", sign_method="chebyshev", m_fermion=0.05, m_dw=1.4) as ctx:
+        ctx.set_links(U)
+        ctx.set_u1(ph)
+        r = ctx.ritz_bounds(start)
+        again = ctx.ritz_bounds(start)
+    # the iteration stops at round-off (the start-vector independence of the test above)
+    assert abs(r["raw"][1] - hi) <= 1e-11 * hi
+    assert lo is None or abs(r["raw"][0] - lo) <= 1e-11 * lo
+    assert r["raw"] == again["raw"] and r["iters"] == again["iters"]  # fixed summation order
+
+
 @pytest.mark.skipif(not have_reference("overlap"), reason="reference overlap build not present")
 def test_overlap_leapfrog_with_gpu_ritz_bounds_matches_reference():
     N = (4, 4, 4)

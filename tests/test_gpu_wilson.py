@@ -569,3 +569,20 @@ def test_step_observe_equals_step_then_charges(precision, variant):
     assert np.array_equal(p0, p1) and np.array_equal(u0, u1)
     for k in ("NV", "N5", "PS"):
         assert abs(c0[k] - c1[k]) <= 1e-13 * max(1.0, abs(c0[k])), k
+
+
+@pytest.mark.parametrize("modes", [31, 257, 300])
+def test_observing_step_sums_one_and_two_launches(modes):
+    """ovl_step_observe adds its partial rows in one launch up to 4096 rows and in
+    two beyond: 512, 4608 and 5120 rows here (16^3, FP64)."""
+    N = (16, 16, 16)
+    with Context(N=N, n_modes=modes, first_mode=1, precision="fp64", form="fused", m_fermion=0.1, m_dw=0.0, dt=0.05,
+                 t_sphaleron=1e9, hop_variant=0) as ctx:
+        ctx.set_links(random_links(N, 0.5, 3))
+        ctx.set_free_fermions()
+        o = ctx.step_observe(2)
+        c = ctx.charges()
+    # FP64 sums of 16^3 x modes terms of size 1 / 2V, in another order
+    for k in ("NV", "N5", "PS"):
+        assert abs(o[k] - c[k]) < 1e-13 * modes
+
