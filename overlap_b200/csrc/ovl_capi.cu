@@ -857,19 +857,16 @@ int ovl_create(const ovl_params *p, ovl_ctx **out) {
     if (p->fermion == OVL_FERMION_OVERLAP && p->sign_method == OVL_SIGN_ZOLOTAREV) {
         ovl::OverlapWork &w = c->ow;
         const size_t mp = (size_t)c->n_mb * ovl::kModeBlock, np = (size_t)p->zolo_poles;
-        if ((rc = alloc(&w.r, field_bytes, "CG residual")) || (rc = alloc(&w.q, field_bytes, "CG direction image")) ||
+        if ((rc = alloc(&w.r, field_bytes * ovl::kCgBatchSlots, "CG residuals")) ||
+            (rc = alloc(&w.q, field_bytes, "CG direction image")) || (rc = alloc(&w.p0, field_bytes, "CG direction")) ||
             (rc = alloc(&w.t, field_bytes, "CG temporary")) || (rc = alloc(&w.x, field_bytes, "shifted solutions")) ||
             (rc = alloc(&w.p, field_bytes * np, "shifted directions")) ||
             (rc = alloc((void **)&w.part, sizeof(double) * ovl::cg_partial_chunks(c->L) * mp, "dot partials")) ||
-            (rc = alloc((void **)&w.rnorm, sizeof(double) * mp * 3, "CG scalars")) ||
-            (rc = alloc((void **)&w.alpha, sizeof(double) * mp * np * 4, "shift scalars")) ||
-            (rc = alloc((void **)&w.active, sizeof(int) * (mp * 5 + 2), "CG flags")) ||
+            (rc = alloc((void **)&w.scalars, sizeof(double) * mp * ovl::kCgModeScalars, "CG scalars")) ||
+            (rc = alloc((void **)&w.shifts, sizeof(double) * mp * np * (2 + 3 * ovl::kCgBatchSlots), "shift scalars")) ||
+            (rc = alloc((void **)&w.flags, sizeof(int) * (mp * ovl::kCgModeFlags + 2), "CG flags")) ||
             (rc = alloc((void **)&w.dz, sizeof(double) * 2 * ovl::kMaxPoles, "Zolotarev coefficients")))
             return bail(rc);
-        w.bnorm = w.rnorm + mp; w.betam = w.rnorm + 2 * mp;
-        w.beta = w.alpha + mp * np; w.z = w.alpha + 2 * mp * np; w.g = w.alpha + 3 * mp * np;
-        w.next = w.active + mp; w.iters = w.active + 2 * mp; w.kact = w.active + 3 * mp;
-        w.knext = w.active + 4 * mp; w.count = w.active + 5 * mp;
         w.bz = w.dz + ovl::kMaxPoles;
         if (cudaMallocHost(&w.host_count, sizeof(int) * 2) != cudaSuccess)
             return bail(fail(c, OVL_E_OOM, "ovl_create: pinned host allocation failed"));
@@ -898,8 +895,8 @@ int ovl_destroy(ovl_ctx *c) {
     cudaSetDevice(c->p.device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     void *bufs[] = {c->psi, c->psimid, c->U, c->E, c->deriv, c->per_site, c->partial, c->dev_small, c->dev_int,
-                    c->aux_src, c->aux_dst, c->ow.r, c->ow.q, c->ow.t, c->ow.x, c->ow.p, c->ow.part, c->ow.rnorm,
-                    c->ow.alpha, c->ow.active, c->ow.dz, c->u_old, c->u_mid, c->e_mid, c->u1,
+                    c->aux_src, c->aux_dst, c->ow.r, c->ow.q, c->ow.t, c->ow.x, c->ow.p0, c->ow.p, c->ow.part, c->ow.scalars,
+                    c->ow.shifts, c->ow.flags, c->ow.dz, c->u_old, c->u_mid, c->e_mid, c->u1,
                     c->cw.b0, c->cw.b1, c->cw.b2, c->cw.w, c->U32, c->u1_32, c->U_b, c->U32_b,
                     c->psi_lo, c->psimid_lo, c->aux_src_lo, c->aux_dst_lo, c->obs_partial, c->obs_scratch, c->pipe};
     if (c->ow.host_count) cudaFreeHost(c->ow.host_count);

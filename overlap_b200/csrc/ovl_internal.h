@@ -249,18 +249,20 @@ struct OverlapCoeffs {
 };
 
 // Device work space of the batched multi-shift CG (all FP64, mode-block layout).
+constexpr int kCgBatchSlots = 8;  // iterations between two updates of the shifted vectors
 struct OverlapWork {
-    void *r = nullptr, *q = nullptr, *t = nullptr, *x = nullptr;  // one field each (x: chi)
+    void *r = nullptr;                              // kCgBatchSlots fields: the residuals of a batch
+    void *q = nullptr, *t = nullptr, *p0 = nullptr, *x = nullptr;  // one field each (x: chi)
     void *p = nullptr;                              // npoles fields
     double *part = nullptr;                         // cg_partial_chunks x modes
-    double *rnorm = nullptr, *bnorm = nullptr, *betam = nullptr;
-    double *alpha = nullptr, *beta = nullptr, *z = nullptr, *g = nullptr;  // npoles x modes
-    int *active = nullptr, *next = nullptr, *iters = nullptr, *kact = nullptr, *knext = nullptr;
-    int *count = nullptr;                           // two slots, by the iteration's parity
+    double *scalars = nullptr;                      // kCgModeScalars x modes
+    double *shifts = nullptr;                       // (2 + 3 kCgBatchSlots) x npoles x modes
+    int *flags = nullptr;                           // kCgModeFlags x modes, then two counts by the iteration's parity
     int *host_count = nullptr;                      // pinned, two slots
     cudaEvent_t counted[2] = {nullptr, nullptr};    // host_count[slot] has arrived
     double *dz = nullptr, *bz = nullptr;            // npoles
 };
+constexpr int kCgModeScalars = 6, kCgModeFlags = 6;
 
 struct OverlapStats {
     uint64_t launches = 0;

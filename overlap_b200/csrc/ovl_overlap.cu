@@ -50,11 +50,11 @@ __device__ __forceinline__ void cg_partial(double v, double *__restrict__ part, 
     }
 }
 
-// r = phi, p_k = phi, chi = 0 and the partial sums of |phi|^2.
+// r = p0 = p_k = phi, chi = 0 and the partial sums of |phi|^2.
 __global__ void __launch_bounds__(kModeBlock *kCgWarps)
-    mscg_init_vectors_kernel(const cpx<double> *__restrict__ phi, cpx<double> *__restrict__ r, cpx<double> *__restrict__ p,
-                             cpx<double> *__restrict__ chi, int V, size_t n, int npoles, double *__restrict__ part,
-                             int modes_padded) {
+    mscg_init_vectors_kernel(const cpx<double> *__restrict__ phi, cpx<double> *__restrict__ r, cpx<double> *__restrict__ p0,
+                             cpx<double> *__restrict__ p, cpx<double> *__restrict__ chi, int V, size_t n, int npoles,
+                             double *__restrict__ part, int modes_padded) {
     const int lane = threadIdx.x, mb = blockIdx.x, rows = V * kComp;
     const size_t base = (size_t)mb * rows * kModeBlock + lane;
     double t = 0.0;
@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(kModeBlock *kCgWarps)
         const size_t e = base + (size_t)j * kModeBlock;
         const cpx<double> v = ld(phi + e);
         st(r + e, v);
+        st(p0 + e, v);
         st(chi + e, mk<double>(0.0, 0.0));
         for (int k = 0; k < npoles; k++) st(p + (size_t)k * n + e, v);
         t += v.re * v.re + v.im * v.im;
@@ -127,71 +128,245 @@ static void launch_cg_square(const double *U, const double *u1, const void *t, c
     else go(LinksF64<false>{U, nullptr, L.N0 * L.N1});
 }
 
-// r -= beta0 q for active modes, and the partial sums of |r|^2.
+// The sum of a mode's partial sums over the chunks, in a fixed order; every
+// thread of the CTA (32 modes x kCgWarps) gets its mode's.
+__device__ __forceinline__ double cg_total(const double *__restrict__ part, int chunks, int m, int modes_padded) {
+    __shared__ double sh[kCgWarps][kModeBlock];
+    double t = 0.0;
+    for (int c = threadIdx.y; c < chunks; c += kCgWarps) t += part[(size_t)c * modes_padded + m];
+    sh[threadIdx.y][threadIdx.x] = t;
+    __syncthreads();
+    t = 0.0;
+#pragma unroll
+    for (int w = 0; w < kCgWarps; w++) t += sh[w][threadIdx.x];
+    return t;
+}
+
+// Sums the chunks' partial sums down to kDotChunks chunks (lattices of many
+// site CTAs, so that the kernels that read them add few).
 __global__ void __launch_bounds__(kModeBlock *kCgWarps)
-    residual_kernel(cpx<double> *r, const cpx<double> *__restrict__ q, const double *__restrict__ beta0,
-                    const int *__restrict__ active, int V, double *__restrict__ part, int modes_padded) {
+    cg_fold_kernel(const double *__restrict__ part, int chunks, double *__restrict__ out, int modes_padded) {
+    const int m = blockIdx.x * kModeBlock + threadIdx.x;
+    for (int o = blockIdx.y * kCgWarps + threadIdx.y; o < kDotChunks; o += gridDim.y * kCgWarps) {
+        const int c0 = (int)((long long)chunks * o / kDotChunks), c1 = (int)((long long)chunks * (o + 1) / kDotChunks);
+        double t = 0.0;
+        for (int c = c0; c < c1; c++) t += part[(size_t)c * modes_padded + m];
+        out[(size_t)o * modes_padded + m] = t;
+    }
+}
+
+// ---------------------------------------------------------- CG scalars --
+// The CG of the smallest shift runs iteration by iteration; the other shifts'
+// vectors only follow it (x_k += beta_k p_k, p_k = alpha_k p_k + g_k r), so they
+// are brought up to date once per kCgBatch iterations from the residuals and
+// the scalars of those iterations: their 2 x 25 fields are moved once per
+// batch.  Slot j of a batch: its residual r[j] and its scalars.
+constexpr int kCgBatch = kCgBatchSlots;
+
+struct CgScalars {
+    double *rnorm[2];              // |r|^2 before / after an iteration, by its parity
+    double *bnorm, *betam, *alpha0, *beta0;
+    double *z, *g;                 // [npoles][modes_padded]
+    double *cb, *al, *gg;          // [kCgBatch][npoles][modes_padded]: b_k beta_k, alpha_k, g_k of a slot
+    int *active, *next, *iters;    // active this iteration / after it
+    int *kact, *knext;             // unfinished shifts of a mode, k < kact: in this batch / by the last iteration
+    int *steps;                    // iterations of this batch that a mode took part in
+    int *count;                    // number of modes active after the iteration
+};
+
+// rnorm = |phi|^2, bnorm = sqrt(rnorm), betam = 1, alpha_0 = 0, z_k = g_k = 1 (OverlapU.cpp:39-54)
+__global__ void __launch_bounds__(kModeBlock *kCgWarps)
+    cg_init_scalars_kernel(CgScalars s, const double *__restrict__ part, int chunks, int n_modes, int modes_padded,
+                           int npoles, double cgerr) {
+    const int m = blockIdx.x * kModeBlock + threadIdx.x;
+    const double rn = cg_total(part, chunks, m, modes_padded);
+    for (int k = threadIdx.y; k < npoles; k += kCgWarps) {
+        const size_t i = (size_t)k * modes_padded + m;
+        s.z[i] = 1.0;
+        s.g[i] = 1.0;
+    }
+    if (threadIdx.y != 0) return;
+    s.rnorm[0][m] = rn;
+    s.bnorm[m] = sqrt(rn);
+    s.betam[m] = 1.0;
+    s.alpha0[m] = 0.0;
+    s.iters[m] = 0;
+    s.kact[m] = npoles;
+    s.knext[m] = npoles;
+    s.steps[m] = 0;
+    const int act = (m < n_modes) && (rn > cgerr * sqrt(rn));
+    s.active[m] = act;
+    s.next[m] = act;
+    if (act) atomicAdd(s.count, 1);
+}
+
+// beta_0 = rnorm / <p0, q> (OverlapU.cpp:71-75) from the partial sums of <p0, q>,
+// rout = rin - beta_0 q for active modes, and the partial sums of |rout|^2.
+// Clears this iteration's count.
+__global__ void __launch_bounds__(kModeBlock *kCgWarps)
+    residual_kernel(CgScalars s, int parity, const double *__restrict__ pap_part, int pap_chunks,
+                    const cpx<double> *__restrict__ rin, cpx<double> *__restrict__ rout, const cpx<double> *__restrict__ q,
+                    int V, double *__restrict__ part, int modes_padded) {
     const int lane = threadIdx.x, mb = blockIdx.x, rows = V * kComp, m = mb * kModeBlock + lane;
+    const double pap = cg_total(pap_part, pap_chunks, m, modes_padded);
     const size_t base = (size_t)mb * rows * kModeBlock + lane;
-    const bool act = active[m] != 0;
-    const double b = act ? beta0[m] : 0.0;
+    const bool act = s.active[m] != 0;
+    const double b = act ? s.rnorm[parity][m] / pap : 0.0;
+    if (blockIdx.y == 0 && threadIdx.y == 0) {
+        s.beta0[m] = b;
+        if (m == 0) *s.count = 0;
+    }
     double t = 0.0;
     if (act)
         for (int j = blockIdx.y * kCgWarps + threadIdx.y; j < rows; j += gridDim.y * kCgWarps) {
             const size_t e = base + (size_t)j * kModeBlock;
-            const cpx<double> a = r[e], y = ld(q + e);
+            const cpx<double> a = ld(rin + e), y = ld(q + e);
             const cpx<double> v = mk<double>(a.re - b * y.re, a.im - b * y.im);
-            st(r + e, v);
+            st(rout + e, v);
             t += v.re * v.re + v.im * v.im;
         }
     cg_partial(t, part, blockIdx.y, m, modes_padded);
 }
 
-// For active modes and their unfinished shifts k < kact: chi += b_k beta_k p_k
-// (the step x_k += beta_k p_k of OverlapU.cpp:95-108 and the combination
-// chi = sum_k b_k x_k of :129-133 in one), then p_k = p_k alpha_k + r g_k.
-// Only the combination of the shifted solutions is wanted, so the 25 x_k are
-// not kept: per iteration the kernel moves 2 kact + 3 fields instead of 4 x 25 + 1
-// and the work space is half as large.  A thread holds kShiftRows rows so that
-// the scalars of a shift are read once for all of them.
-// One overlap leapfrog step at 8^3, 256 modes, 25 poles: 125 ms with the x_k,
-// separate dot products and a host wait per iteration, 91 ms with this CG (the
-// rest are the Ritz solves).
-constexpr int kShiftRows = 4;
+// Finished shifts: g_k r is the residual of the shifted system k, so what its
+// further steps could still add to chi is at most b_k |g_k r| / (lambda_min +
+// d_k).  sum_k b_k / (lambda + d_k) approximates lambda^(-1/2), every term is
+// positive, and |chi| >= |phi| lambda_max^(-1/2): relative to chi that is at
+// most sqrt(lambda_max / lambda_min) |g_k r| / |phi|.  A shift is left alone
+// once |g_k r| <= kShiftDone |phi| = 1e-20 |phi|, which bounds it by 1e-18 at a
+// condition number of 1e4, below the rounding of chi.  Poles come in
+// ascending order and the larger ones finish first; kact is the last
+// unfinished one + 1 and never grows.
+constexpr double kShiftDone = 1e-20;
 
+// The end of an iteration (slot j of its batch).  CTAs with blockIdx.y > 0:
+// alpha_0 = |r|^2 / rnorm and p0 = alpha_0 p0 + r for active modes.  The CTA
+// with blockIdx.y = 0: the iteration's scalars of every unfinished shift, shared
+// out over its warps -- z_k, beta_k from the previous alpha_0, z_k, betam
+// (OverlapU.cpp:71-88), alpha_k and g_k as the shift loop of :95-106 computes
+// them (alpha_0 is rewritten at k = 0 before the other shifts read it) -- then
+// betam = beta_0, the iteration count and the stopping test (:56, 110-117).
 __global__ void __launch_bounds__(kModeBlock *kCgWarps)
-    shift_update_kernel(cpx<double> *__restrict__ chi, cpx<double> *__restrict__ p, const cpx<double> *__restrict__ r,
-                        const double *__restrict__ beta, const double *__restrict__ alpha, const double *__restrict__ g,
-                        const double *__restrict__ bz, const int *__restrict__ active, const int *__restrict__ kact,
-                        int V, size_t n, int modes_padded) {
+    cg_advance_kernel(CgScalars s, int parity, int slot, const double *__restrict__ part, int chunks,
+                      const double *__restrict__ dz, const double *__restrict__ bz, int npoles, double cgerr, int max_iter,
+                      cpx<double> *__restrict__ p0, const cpx<double> *__restrict__ r, int V, int modes_padded) {
+    const int lane = threadIdx.x, mb = blockIdx.x, m = mb * kModeBlock + lane;
+    const double rr = cg_total(part, chunks, m, modes_padded);
+    const bool active = s.active[m] != 0;
+    const double b0 = s.beta0[m];
+    // z_0 = 1 and beta_0 = b0, in the reference's order of operations
+    const double a0 = active ? rr / s.rnorm[parity][m] * 1.0 * b0 / b0 : 0.0;
+    if (blockIdx.y > 0) {
+        if (!active) return;
+        const int rows = V * kComp;
+        const size_t base = (size_t)mb * rows * kModeBlock + lane;
+        for (int j = (blockIdx.y - 1) * kCgWarps + threadIdx.y; j < rows; j += (gridDim.y - 1) * kCgWarps) {
+            const size_t e = base + (size_t)j * kModeBlock;
+            const cpx<double> pv = p0[e], rv = ld(r + e);
+            st(p0 + e, mk<double>(pv.re * a0 + rv.re, pv.im * a0 + rv.im));
+        }
+        return;
+    }
+    __shared__ int last[kCgWarps][kModeBlock];
+    const int nk = slot == 0 ? s.knext[m] : s.kact[m];
+    int unfinished = 0;
+    if (active) {
+        const double ap = s.alpha0[m], bm = s.betam[m], bnorm = s.bnorm[m];
+        for (int k = threadIdx.y; k < nk; k += kCgWarps) {
+            const size_t i = (size_t)k * modes_padded + m, o = (size_t)slot * npoles * modes_padded + i;
+            double zk = 1.0, bk = b0, ak = a0;
+            if (k > 0) {
+                const double dr = b0 * ap * (1.0 - s.z[i]) + bm * (1.0 + (dz[k] - dz[0]) * b0);
+                zk = bm / dr;
+                bk = b0 * zk;
+                ak = a0 * zk * bk / b0;
+                s.z[i] = zk;
+            }
+            const double gk = s.g[i] * zk;
+            s.g[i] = gk;
+            s.cb[o] = bz[k] * bk;
+            s.al[o] = ak;
+            s.gg[o] = gk;
+            // bnorm = |phi|; compared as squares
+            if (gk * gk * rr > kShiftDone * kShiftDone * bnorm * bnorm) unfinished = k + 1;
+        }
+    }
+    last[threadIdx.y][lane] = unfinished;
+    __syncthreads();  // every warp has read kact, knext, alpha0 and betam
+    if (threadIdx.y != 0) return;
+    if (slot == 0) {
+        s.kact[m] = nk;
+        s.steps[m] = 0;
+    }
+    if (!active) {
+        s.next[m] = 0;
+        return;
+    }
+    for (int w = 1; w < kCgWarps; w++) unfinished = max(unfinished, last[w][lane]);
+    s.knext[m] = unfinished;
+    s.steps[m] = slot + 1;
+    s.rnorm[parity ^ 1][m] = rr;
+    s.betam[m] = b0;
+    s.alpha0[m] = a0;
+    const int it = s.iters[m] + 1;
+    s.iters[m] = it;
+    const int act = (it < max_iter) && (rr > cgerr * s.bnorm[m]);
+    s.next[m] = act;
+    if (act) atomicAdd(s.count, 1);
+}
+
+// Brings the unfinished shifts of a batch up to date: for each of the mode's
+// iterations of the batch chi += b_k beta_k p_k (the step x_k += beta_k p_k of
+// OverlapU.cpp:95-108 and the combination chi = sum_k b_k x_k of :129-133 in
+// one), then p_k = p_k alpha_k + r g_k.  Only the combination of the shifted
+// solutions is wanted, so the 25 x_k are not kept; per batch the kernel moves
+// 2 kact fields, the residuals of the batch and chi (HBM bound), against 4 x 25 + 1
+// fields per iteration for separate x_k and p_k.
+// One overlap leapfrog step with its two pairs of bounds at 8^3, 256 modes:
+// 50 ms with the shifts updated in every iteration, 42.9 ms in batches of eight.
+constexpr int kShiftRows = 2, kShiftWarps = 4;
+
+__global__ void __launch_bounds__(kModeBlock *kShiftWarps, 3)
+    shift_update_kernel(CgScalars s, cpx<double> *__restrict__ chi, cpx<double> *__restrict__ p,
+                        const cpx<double> *__restrict__ r, int V, size_t n, int npoles, int modes_padded) {
     const int lane = threadIdx.x, mb = blockIdx.x, rows = V * kComp, m = mb * kModeBlock + lane;
-    if (!active[m]) return;
-    const int nk = kact[m];
+    const int nj = s.steps[m];
+    if (nj == 0) return;
+    const int nk = s.kact[m];
     const size_t base = (size_t)mb * rows * kModeBlock + lane;
-    const int step = gridDim.y * kCgWarps;
-    for (int j0 = blockIdx.y * kCgWarps + threadIdx.y; j0 < rows; j0 += step * kShiftRows) {
-        cpx<double> rv[kShiftRows], x[kShiftRows];
+    const int step = gridDim.y * kShiftWarps;
+    for (int j0 = blockIdx.y * kShiftWarps + threadIdx.y; j0 < rows; j0 += step * kShiftRows) {
+        cpx<double> rv[kCgBatch][kShiftRows], x[kShiftRows];
         size_t e[kShiftRows];
 #pragma unroll
         for (int u = 0; u < kShiftRows; u++) {
-            const int j = j0 + u * step;
-            e[u] = base + (size_t)min(j, rows - 1) * kModeBlock;
-            rv[u] = ld(r + e[u]);
+            e[u] = base + (size_t)min(j0 + u * step, rows - 1) * kModeBlock;
             x[u] = chi[e[u]];
         }
+#pragma unroll
+        for (int j = 0; j < kCgBatch; j++)
+#pragma unroll
+            for (int u = 0; u < kShiftRows; u++) rv[j][u] = j < nj ? ld(r + (size_t)j * n + e[u]) : mk<double>(0.0, 0.0);
         for (int k = 0; k < nk; k++) {
-            const size_t s = (size_t)k * modes_padded + m;
-            const double cb = bz[k] * beta[s], ak = alpha[s], gk = g[s];
             cpx<double> *pk = p + (size_t)k * n;
             cpx<double> pv[kShiftRows];
 #pragma unroll
             for (int u = 0; u < kShiftRows; u++) pv[u] = pk[e[u]];
 #pragma unroll
-            for (int u = 0; u < kShiftRows; u++) {
-                x[u] = mk<double>(x[u].re + cb * pv[u].re, x[u].im + cb * pv[u].im);
-                if (j0 + u * step < rows)
-                    st(pk + e[u], mk<double>(pv[u].re * ak + rv[u].re * gk, pv[u].im * ak + rv[u].im * gk));
+            for (int j = 0; j < kCgBatch; j++) {
+                if (j < nj) {
+                    const size_t o = ((size_t)j * npoles + k) * modes_padded + m;
+                    const double cb = s.cb[o], ak = s.al[o], gk = s.gg[o];
+#pragma unroll
+                    for (int u = 0; u < kShiftRows; u++) {
+                        x[u] = mk<double>(x[u].re + cb * pv[u].re, x[u].im + cb * pv[u].im);
+                        pv[u] = mk<double>(pv[u].re * ak + rv[j][u].re * gk, pv[u].im * ak + rv[j][u].im * gk);
+                    }
+                }
             }
+#pragma unroll
+            for (int u = 0; u < kShiftRows; u++)
+                if (j0 + u * step < rows) st(pk + e[u], pv[u]);
         }
 #pragma unroll
         for (int u = 0; u < kShiftRows; u++)
@@ -216,138 +391,6 @@ __global__ void overlap_finish_kernel(const cpx<double> *__restrict__ phi, const
             st(dst + e, o);
         }
     }
-}
-
-// ---------------------------------------------------------- scalar kernels --
-// One CTA of 32 x kCgWarps threads per mode block: the chunks' partial sums of
-// the dot product are added (in a fixed order), then the shifts of a mode are
-// shared out over the CTA's warps.  One thread per mode walking the chunks and
-// the 25 shifts alone took 16-20 us per launch, all of it load latency.
-struct CgScalars {
-    double *rnorm, *bnorm, *betam;
-    double *alpha, *beta, *z, *g;  // [npoles][modes_padded]
-    int *active, *next, *iters;    // active this iteration / after it
-    int *kact, *knext;             // unfinished shifts of a mode, k < kact: this iteration / after it
-    int *count;                    // number of modes active after the update
-};
-
-__device__ __forceinline__ double cg_total(const double *__restrict__ part, int chunks, int m, int modes_padded) {
-    __shared__ double sh[kCgWarps][kModeBlock];
-    double t = 0.0;
-    for (int c = threadIdx.y; c < chunks; c += kCgWarps) t += part[(size_t)c * modes_padded + m];
-    sh[threadIdx.y][threadIdx.x] = t;
-    __syncthreads();
-    t = 0.0;
-#pragma unroll
-    for (int w = 0; w < kCgWarps; w++) t += sh[w][threadIdx.x];
-    return t;
-}
-
-// rnorm = |phi|^2, bnorm = sqrt(rnorm), betam = 1, alpha_0 = 0, z_k = g_k = 1 (OverlapU.cpp:39-54)
-__global__ void __launch_bounds__(kModeBlock *kCgWarps)
-    cg_init_scalars_kernel(CgScalars s, const double *__restrict__ part, int chunks, int n_modes, int modes_padded,
-                           int npoles, double cgerr) {
-    const int m = blockIdx.x * kModeBlock + threadIdx.x;
-    const double rn = cg_total(part, chunks, m, modes_padded);
-    for (int k = threadIdx.y; k < npoles; k += kCgWarps) {
-        const size_t i = (size_t)k * modes_padded + m;
-        s.alpha[i] = 0.0;
-        s.z[i] = 1.0;
-        s.g[i] = 1.0;
-        s.beta[i] = 0.0;
-    }
-    if (threadIdx.y != 0) return;
-    s.rnorm[m] = rn;
-    s.bnorm[m] = sqrt(rn);
-    s.betam[m] = 1.0;
-    s.iters[m] = 0;
-    s.kact[m] = npoles;
-    s.knext[m] = npoles;
-    const int act = (m < n_modes) && (rn > cgerr * sqrt(rn));
-    s.active[m] = act;
-    s.next[m] = act;
-    if (act) atomicAdd(s.count, 1);
-}
-
-// beta_0 = rnorm / <p0, q>; for k >= 1: z_k, beta_k from the previous alpha_0,
-// z_k, betam (OverlapU.cpp:71-88).  Clears this iteration's count.
-__global__ void __launch_bounds__(kModeBlock *kCgWarps)
-    cg_scalars_beta_kernel(CgScalars s, const double *__restrict__ part, int chunks, const double *__restrict__ dz,
-                           int modes_padded) {
-    const int m = blockIdx.x * kModeBlock + threadIdx.x;
-    const double pap = cg_total(part, chunks, m, modes_padded);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) *s.count = 0;
-    if (!s.active[m]) return;
-    const double b0 = s.rnorm[m] / pap, a0 = s.alpha[m], bm = s.betam[m];
-    const int nk = s.kact[m];
-    for (int k = threadIdx.y; k < nk; k += kCgWarps) {
-        const size_t i = (size_t)k * modes_padded + m;
-        if (k == 0) {
-            s.beta[i] = b0;
-            continue;
-        }
-        const double dr = b0 * a0 * (1.0 - s.z[i]) + bm * (1.0 + (dz[k] - dz[0]) * b0);
-        s.z[i] = bm / dr;
-        s.beta[i] = b0 * s.z[i];
-    }
-}
-
-// alpha_0 = |r|^2 / rnorm, rnorm = |r|^2; per shift alpha_k and g_k as the
-// shift loop of OverlapU.cpp:95-106 computes them (alpha_0 is rewritten at
-// k = 0 before the other shifts read it); betam = beta_0; iteration count and
-// the stopping test (OverlapU.cpp:56, 110-117).
-//
-// Finished shifts: g_k r is the residual of the shifted system k, so what its
-// further steps could still add to chi is at most b_k |g_k r| / (lambda_min +
-// d_k).  sum_k b_k / (lambda + d_k) approximates lambda^(-1/2), every term is
-// positive, and |chi| >= |phi| lambda_max^(-1/2): relative to chi that is at
-// most sqrt(lambda_max / lambda_min) |g_k r| / |phi|.  A shift is left alone
-// once |g_k r| <= kShiftDone |phi| = 1e-20 |phi|, which bounds it by 1e-18 at a
-// condition number of 1e4, below the rounding of chi.  Poles come in
-// ascending order and the larger ones finish first; kact is the last
-// unfinished one + 1 and never grows; the step that finishes a shift is still
-// applied (knext is the next iteration's kact).
-constexpr double kShiftDone = 1e-20;
-
-__global__ void __launch_bounds__(kModeBlock *kCgWarps)
-    cg_scalars_alpha_kernel(CgScalars s, const double *__restrict__ part, int chunks, int modes_padded, double cgerr,
-                            int max_iter) {
-    __shared__ int last[kCgWarps][kModeBlock];
-    const int m = blockIdx.x * kModeBlock + threadIdx.x;
-    const double rr = cg_total(part, chunks, m, modes_padded);
-    const bool active = s.active[m] != 0;
-    int unfinished = 0;
-    double b0 = 0.0;
-    if (active) {
-        const int nk = s.kact[m];
-        const double bnorm = s.bnorm[m], a00 = rr / s.rnorm[m];
-        b0 = s.beta[m];
-        const double a0 = a00 * s.z[m] * s.beta[m] / b0;  // shift 0
-        for (int k = threadIdx.y; k < nk; k += kCgWarps) {
-            const size_t i = (size_t)k * modes_padded + m;
-            const double zk = s.z[i], gk = s.g[i] * zk;
-            s.alpha[i] = k == 0 ? a0 : a0 * zk * s.beta[i] / b0;
-            s.g[i] = gk;
-            // bnorm = |phi|; compared as squares
-            if (gk * gk * rr > kShiftDone * kShiftDone * bnorm * bnorm) unfinished = k + 1;
-        }
-    }
-    last[threadIdx.y][threadIdx.x] = unfinished;
-    __syncthreads();  // every warp has read rnorm, z, beta of shift 0 and kact
-    if (threadIdx.y != 0) return;
-    if (!active) {
-        s.next[m] = 0;
-        return;
-    }
-    for (int w = 1; w < kCgWarps; w++) unfinished = max(unfinished, last[w][threadIdx.x]);
-    s.knext[m] = max(1, unfinished);  // shift 0 carries the iteration
-    s.rnorm[m] = rr;
-    s.betam[m] = b0;
-    const int it = s.iters[m] + 1;
-    s.iters[m] = it;
-    const int act = (it < max_iter) && (rr > cgerr * s.bnorm[m]);
-    s.next[m] = act;
-    if (act) atomicAdd(s.count, 1);
 }
 
 // --------------------------------------------------------- overlap currents --
@@ -452,7 +495,8 @@ static int cg_chunks(const Lattice &L, int n_mb, int sm_count) {
     return std::max(1, std::min(most, (8 * sm_count + n_mb - 1) / n_mb));
 }
 
-size_t cg_partial_chunks(const Lattice &L) { return (size_t)std::max(kDotChunks, cg_square_chunks(L)); }
+// chunks of |r|^2, of <p0, q>, and of the latter folded
+size_t cg_partial_chunks(const Lattice &L) { return (size_t)2 * kDotChunks + cg_square_chunks(L); }
 
 void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void *src, void *dst, const Lattice &L, int n_mb,
                    int n_modes, const OverlapCoeffs &co, double amass, double mdw, double mf, double dt,
@@ -463,49 +507,81 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
     const int grid = elem_grid(n, sm_count);
     const cpx<double> *phi = reinterpret_cast<const cpx<double> *>(src);
     cpx<double> *r = reinterpret_cast<cpx<double> *>(w.r), *q = reinterpret_cast<cpx<double> *>(w.q);
-    cpx<double> *t = reinterpret_cast<cpx<double> *>(w.t);
+    cpx<double> *t = reinterpret_cast<cpx<double> *>(w.t), *p0 = reinterpret_cast<cpx<double> *>(w.p0);
     cpx<double> *chi = reinterpret_cast<cpx<double> *>(w.x), *p = reinterpret_cast<cpx<double> *>(w.p);
-    CgScalars s{w.rnorm, w.bnorm, w.betam, w.alpha, w.beta, w.z, w.g, w.active, w.next, w.iters, w.kact, w.knext, w.count};
+    CgScalars s;
+    const size_t pm = (size_t)np * mp;
+    s.rnorm[0] = w.scalars;
+    s.rnorm[1] = w.scalars + mp;
+    s.bnorm = w.scalars + 2 * mp;
+    s.betam = w.scalars + 3 * mp;
+    s.alpha0 = w.scalars + 4 * mp;
+    s.beta0 = w.scalars + 5 * mp;
+    s.z = w.shifts;
+    s.g = w.shifts + pm;
+    s.cb = w.shifts + 2 * pm;
+    s.al = s.cb + kCgBatch * pm;
+    s.gg = s.al + kCgBatch * pm;
+    s.active = w.flags;
+    s.next = w.flags + mp;
+    s.iters = w.flags + 2 * mp;
+    s.kact = w.flags + 3 * mp;
+    s.knext = w.flags + 4 * mp;
+    s.steps = w.flags + 5 * mp;
+    s.count = w.flags + 6 * mp;
+    int *const count = s.count;
     cudaMemcpyAsync(w.dz, co.d, sizeof(double) * np, cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(w.bz, co.b, sizeof(double) * np, cudaMemcpyHostToDevice, stream);
 
     const int chunks = cg_chunks(L, n_mb, sm_count), sq_chunks = cg_square_chunks(L);
+    const bool fold = sq_chunks > 2 * kDotChunks;
+    double *const rr_part = w.part, *const pap_part = rr_part + (size_t)kDotChunks * mp;
+    double *const pap_fold = pap_part + (size_t)sq_chunks * mp;
     const dim3 vblock(kModeBlock, kCgWarps), vgrid(n_mb, chunks);
-    mscg_init_vectors_kernel<<<vgrid, vblock, 0, stream>>>(phi, r, p, chi, L.V, n, np, w.part, mp);
-    cudaMemsetAsync(w.count, 0, sizeof(int) * 2, stream);
-    cg_init_scalars_kernel<<<n_mb, vblock, 0, stream>>>(s, w.part, chunks, n_modes, mp, np, co.cg_tol);
+    // the residual of slot j is r[j]; the iteration of slot 0 starts from the last slot
+    mscg_init_vectors_kernel<<<vgrid, vblock, 0, stream>>>(phi, r + (size_t)(kCgBatch - 1) * n, p0, p, chi, L.V, n, np, rr_part,
+                                                           mp);
+    cudaMemsetAsync(count, 0, sizeof(int) * 2, stream);
+    cg_init_scalars_kernel<<<n_mb, vblock, 0, stream>>>(s, rr_part, chunks, n_modes, mp, np, co.cg_tol);
     int launches = 2;
     // The count of modes still active is read back one iteration late, while
     // the next iteration is already queued: the GPU does not wait for the host,
     // and the one iteration queued past the end finds no active mode (two
     // stencil passes, no vector changes).
     auto read_count = [&](int slot) {
-        cudaMemcpyAsync(w.host_count + slot, w.count + slot, sizeof(int), cudaMemcpyDeviceToHost, stream);
+        cudaMemcpyAsync(w.host_count + slot, count + slot, sizeof(int), cudaMemcpyDeviceToHost, stream);
         cudaEventRecord(w.counted[slot], stream);
     };
     auto counted = [&](int slot) {
         cudaEventSynchronize(w.counted[slot]);
         return w.host_count[slot];
     };
+    auto update_shifts = [&]() {
+        shift_update_kernel<<<dim3(n_mb, 2 * chunks), dim3(kModeBlock, kShiftWarps), 0, stream>>>(s, chi, p, r, L.V, n, np, mp);
+        launches++;
+    };
     read_count(0);
     int iterations = 0;
     for (int it = 0;; it++) {
+        const int slot = it % kCgBatch, par = it & 1;
+        cpx<double> *rin = r + (size_t)((slot + kCgBatch - 1) % kCgBatch) * n, *rout = r + (size_t)slot * n;
         // q = h_W^2 p0 + d0 p0 = -D(D p0) + d0 p0
-        s.count = w.count + ((it + 1) & 1);
-        launch_wilson<double>(U, u1, p, w.t, L, 0, n_mb, amass, 0.0, false, stream);
-        launch_cg_square(U, u1, w.t, p, q, L, n_mb, amass, co.d[0], w.part, mp, stream);
-        cg_scalars_beta_kernel<<<n_mb, vblock, 0, stream>>>(s, w.part, sq_chunks, w.dz, mp);
-        residual_kernel<<<vgrid, vblock, 0, stream>>>(r, q, w.beta, s.active, L.V, w.part, mp);
-        cg_scalars_alpha_kernel<<<n_mb, vblock, 0, stream>>>(s, w.part, chunks, mp, co.cg_tol, co.cg_max_iter);
-        shift_update_kernel<<<vgrid, vblock, 0, stream>>>(chi, p, r, w.beta, w.alpha, w.g, w.bz, s.active, s.kact, L.V, n,
-                                                          mp);
-        launches += 6;
+        s.count = count + (par ^ 1);
+        launch_wilson<double>(U, u1, p0, w.t, L, 0, n_mb, amass, 0.0, false, stream);
+        launch_cg_square(U, u1, w.t, p0, q, L, n_mb, amass, co.d[0], pap_part, mp, stream);
+        if (fold) cg_fold_kernel<<<dim3(n_mb, kDotChunks / kCgWarps), vblock, 0, stream>>>(pap_part, sq_chunks, pap_fold, mp);
+        residual_kernel<<<vgrid, vblock, 0, stream>>>(s, par, fold ? pap_fold : pap_part, fold ? kDotChunks : sq_chunks, rin,
+                                                      rout, q, L.V, rr_part, mp);
+        cg_advance_kernel<<<dim3(n_mb, chunks + 1), vblock, 0, stream>>>(s, par, slot, rr_part, chunks, w.dz, w.bz, np,
+                                                                         co.cg_tol, co.cg_max_iter, p0, rout, L.V, mp);
+        launches += fold ? 5 : 4;
         std::swap(s.active, s.next);
-        std::swap(s.kact, s.knext);
-        read_count((it + 1) & 1);
-        if (counted(it & 1) == 0) break;  // no mode was active before this iteration
-        iterations++;
-        if (iterations > co.cg_max_iter + 1) break;  // every mode stops by then
+        read_count(par ^ 1);
+        const bool over = counted(par) == 0;  // no mode was active before this iteration
+        if (!over) iterations++;
+        const bool stop = over || iterations > co.cg_max_iter + 1;  // every mode stops by then
+        if (slot == kCgBatch - 1 || (stop && slot > 0)) update_shifts();
+        if (stop) break;
     }
     launch_wilson<double>(U, u1, chi, w.t, L, 0, n_mb, amass, 0.0, false, stream);
     overlap_finish_kernel<<<grid, 256, 0, stream>>>(phi, t, reinterpret_cast<cpx<double> *>(dst), n, mdw, mf, dt,
@@ -516,7 +592,7 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
         stats->iterations = iterations;
         int mx = 0;
         std::vector<int> it(mp);
-        cudaMemcpyAsync(it.data(), w.iters, sizeof(int) * mp, cudaMemcpyDeviceToHost, stream);
+        cudaMemcpyAsync(it.data(), s.iters, sizeof(int) * mp, cudaMemcpyDeviceToHost, stream);
         cudaStreamSynchronize(stream);
         int capped = 0;
         for (int m = 0; m < n_modes; m++) {
