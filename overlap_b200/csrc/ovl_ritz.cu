@@ -21,6 +21,8 @@
 #include <algorithm>
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 #include "ovl_internal.h"
 #include "ovl_stencil.cuh"
 #include "ovl_su3.cuh"
@@ -427,36 +429,62 @@ __global__ void __launch_bounds__(kRitzThreads)
 }
 
 // ------------------------------------------------- one launch per solve --
-// The whole two-colour iteration in one cooperative launch.  The kernels above
-// take a step in six launches of a few CTAs each, and at the sizes of the
-// spectral bounds a launch is all latency (8^3: 37 us per step, 6.3 us per
-// kernel).  Here two threads own a site, half h the spins h and 3 - h of both
-// colours, and keep x, y = A x, p, z = A p and g of it in registers for the
-// whole solve; only the vectors the stencil reads from neighbours (the raw
-// direction, or x at a restart, and t = D p) go through memory, component by
-// component over the sites.  A step is five phases, each ending in a barrier
-// of the problem's CTAs that also delivers the phase's sums: t = D p; z = -s D t;
-// the rotation; the residual; the new direction (normalised on the way into
-// the next step).  The arithmetic is that of the kernels above, except that D
-// is applied to the raw direction and its result scaled.
+// The whole two-colour iteration in one launch.  The kernels above take a step
+// in six launches of a few CTAs each, and at the sizes of the spectral bounds a
+// launch is all latency (8^3: 37 us per step, 6.3 us per kernel).  Here two
+// threads own a site, half h the spins h and 3 - h of both colours, and keep x,
+// y = A x, p, z = A p and g of it in registers for the whole solve; only the
+// vectors the stencil reads from neighbours (v: the raw direction, or x at a
+// restart; t = D p) are exchanged.  A step is five phases, each ending in a
+// barrier of the problem's CTAs that also delivers the phase's sums: t = D p;
+// z = -s D t; the rotation; the residual; the new direction (normalised on the
+// way into the next step).  The arithmetic is that of the kernels above, except
+// that D is applied to the raw direction and its result scaled.
+//
+// Two ways to exchange and to meet:
+//   RitzCluster  a problem is one thread-block cluster: v and t in distributed
+//                shared memory, the hardware's cluster barrier (up to
+//                16 CTAs x 128 sites)
+//   RitzGrid     a cooperative launch: v and t in global memory, a counter per
+//                problem.  The CTAs wait for one another, so all are resident
+//                and every wait is bounded (1 s of %globaltimer): on expiry the
+//                error word is set, every CTA leaves at its next wait, and the
+//                host reports the solve as failed.
 // One overlap leapfrog step with its two pairs of bounds at 8^3, 256 modes:
-// 91 ms with six launches per Ritz step, 50 ms with one launch per solve.
-// The CTAs wait for one another, so the launch is cooperative (all resident)
-// and every wait is bounded (1 s of %globaltimer): on expiry the error word is
-// set, every CTA leaves at its next wait, and the host reports the solve as failed.
-constexpr int kRitzSites = 32;               // sites per CTA
-constexpr int kRitzOneThreads = 2 * kRitzSites;
-constexpr int kRitzTabStride = 50;           // doubles per site of the link table: 6 x 8 and 2 to spread the banks
+// 91 ms with six launches per Ritz step, 50 ms with the cooperative launch; then,
+// the CG made faster, 42.9 ms with the cooperative launch and 30.8 ms with
+// clusters (8 CTAs of 64 sites per problem).
+constexpr int kRitzTabStride = 50;  // doubles per site of the link table: 6 x 8 and 2 to spread the banks
+constexpr int kRitzGridSites = 32;  // sites per CTA of the cooperative launch
 
 struct RitzOne {
     const double2 *start;  // [V][8]
-    double2 *v, *t;        // [problem][8][V]: the exchanged vectors
-    double *part;          // [2 slots][problem][CTAs][kRitzParts]
-    int *count, *err;      // arrivals per problem; error word
     RitzScalars *st;
     double amass, delitr;
     int max_iter, nrestart;
+    int sites;             // per CTA
+    // RitzGrid
+    double2 *v, *t;        // [problem][8][V]
+    double *part;          // [2 slots][problem][CTAs][kRitzParts]
+    int *count, *err;      // arrivals per problem; error word
 };
+
+using RitzHalf = cpx<double>[2][2];  // [colour][upper, lower component of the half]
+
+// Component (colour c, upper 0 / lower 1) of half h: spin h or 3 - h.
+__device__ __forceinline__ int ritz_comp(int c, int lower, int h) { return c * kSpin + (lower ? 3 - h : h); }
+
+// The warps' sums of nv values in sh (lane 0 of each writes); a barrier of the
+// CTA has to follow before they are read.
+template <int WARPS>
+__device__ __forceinline__ void ritz_warp_sums(int nv, const double (&v)[kRitzParts], double (*sh)[kRitzParts]) {
+    for (int k = 0; k < nv; k++) {
+        double t = v[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][k] = t;
+    }
+}
 
 // One thread waits for the count, polling without a pause (the phases are a
 // few hundred nanoseconds apart); bounded as wait_count.
@@ -473,79 +501,147 @@ __device__ __forceinline__ bool ritz_wait(const int *counter, int target, int *e
     return true;
 }
 
-struct RitzBarrier {
-    double *part;  // this problem's partials of slot 0; slot 1 at + slot_stride
+struct RitzGrid {
+    double2 *vec[2];  // v, t of this problem
+    int V, site, nb[6];
+    bool live;
+    double *part;     // this problem's partials of slot 0; slot 1 at + slot_stride
     size_t slot_stride;
     int *count, *err;
     int nblocks, phase;
-};
+    static constexpr int kWarps = 2 * kRitzGridSites / 32;
 
-// Sums nv values over the problem's CTAs (in the order of the CTAs; every
-// thread gets the same totals) behind a barrier of them: what the CTAs wrote
-// before it is visible after it.  False when a wait ran out.
-__device__ __forceinline__ bool ritz_sum(RitzBarrier &b, int nv, const double (&v)[kRitzParts], double (&out)[kRitzParts]) {
-    __shared__ double sh[kRitzOneThreads / 32][kRitzParts], tot[kRitzParts];
-    __shared__ int ok;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < nv; k++) {
-        double t = v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) sh[warp][k] = t;
+    __device__ __forceinline__ RitzGrid(const RitzOne &a, const Lattice &L, int site_, bool live_, const int (&n)[6])
+        : V(L.V), site(site_), live(live_) {
+        const int prob = blockIdx.y;
+        vec[0] = a.v + (size_t)prob * kComp * V;
+        vec[1] = a.t + (size_t)prob * kComp * V;
+        for (int d = 0; d < 6; d++) nb[d] = n[d];
+        nblocks = gridDim.x;
+        slot_stride = (size_t)2 * gridDim.x * kRitzParts;
+        part = a.part + (size_t)prob * gridDim.x * kRitzParts;
+        count = a.count + prob;
+        err = a.err;
+        phase = 0;
     }
-    __syncthreads();
-    double *slot = b.part + (b.phase & 1) * b.slot_stride;
-    b.phase++;
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < nv; k++) {
-            double t = 0.0;
-            for (int w = 0; w < kRitzOneThreads / 32; w++) t += sh[w][k];
-            __stcg(slot + (size_t)blockIdx.x * kRitzParts + k, t);
-        }
-        red_release_add(b.count, 1);
-        ok = ritz_wait(b.count, b.nblocks * b.phase, b.err) ? 1 : 0;
+    __device__ __forceinline__ void put(int which, int comp, double re, double im) {
+        if (live) __stcg(vec[which] + (size_t)comp * V + site, make_double2(re, im));
     }
-    __syncthreads();
-    if (!ok) return false;
-    if (nv > 0) {
-        if (threadIdx.x < 32) {
-            double t[kRitzParts] = {0.0, 0.0, 0.0, 0.0};
-            for (int i = lane; i < b.nblocks; i += 32)
-                for (int k = 0; k < nv; k++) t[k] += __ldcg(slot + (size_t)i * kRitzParts + k);
+    __device__ __forceinline__ cpx<double> get(int which, int dir, int comp) const {
+        const double2 u = __ldcg(vec[which] + (size_t)comp * V + nb[dir]);
+        return mk<double>(u.x, u.y);
+    }
+    // Sums nv values over the problem's CTAs (in the order of the CTAs; every
+    // thread gets the same totals) behind a barrier of them: what the CTAs wrote
+    // before it is visible after it.  False when a wait ran out.
+    __device__ __forceinline__ bool sum(int nv, const double (&v)[kRitzParts], double (&out)[kRitzParts]) {
+        __shared__ double sh[kWarps][kRitzParts], tot[kRitzParts];
+        __shared__ int ok;
+        const int lane = threadIdx.x & 31;
+        ritz_warp_sums<kWarps>(nv, v, sh);
+        __syncthreads();
+        double *slot = part + (phase & 1) * slot_stride;
+        phase++;
+        if (threadIdx.x == 0) {
             for (int k = 0; k < nv; k++) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
-                if (lane == 0) tot[k] = t[k];
+                double t = 0.0;
+                for (int w = 0; w < kWarps; w++) t += sh[w][k];
+                __stcg(slot + (size_t)blockIdx.x * kRitzParts + k, t);
             }
+            red_release_add(count, 1);
+            ok = ritz_wait(count, nblocks * phase, err) ? 1 : 0;
         }
         __syncthreads();
-        for (int k = 0; k < nv; k++) out[k] = tot[k];
+        if (!ok) return false;
+        if (nv > 0) {
+            if (threadIdx.x < 32) {
+                double t[kRitzParts] = {0.0, 0.0, 0.0, 0.0};
+                for (int i = lane; i < nblocks; i += 32)
+                    for (int k = 0; k < nv; k++) t[k] += __ldcg(slot + (size_t)i * kRitzParts + k);
+                for (int k = 0; k < nv; k++) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+                    if (lane == 0) tot[k] = t[k];
+                }
+            }
+            __syncthreads();
+            for (int k = 0; k < nv; k++) out[k] = tot[k];
+        }
+        __syncthreads();  // sh, tot and ok are reused by the next phase
+        return true;
     }
-    __syncthreads();  // sh, tot and ok are reused by the next phase
-    return true;
+    __device__ __forceinline__ void finish() {}
+};
+
+// The cluster's CTAs hold `sites` consecutive sites each; dynamic shared memory:
+// v [8][sites], t [8][sites], then the link table.
+constexpr int kRitzClusterMax = 16;                                 // CTAs per cluster, at most
+constexpr int kRitzClusterThreads = 256;                            // at most: 255 registers a thread
+constexpr size_t ritz_cluster_smem(int sites) {
+    return (sizeof(double2) * 2 * kComp + sizeof(double) * kRitzTabStride) * (size_t)sites;
 }
 
-// Component (colour c, upper 0 / lower 1) of half h: spin h or 3 - h.
-__device__ __forceinline__ int ritz_comp(int c, int lower, int h) { return c * kSpin + (lower ? 3 - h : h); }
+struct RitzCluster {
+    double2 *own;      // v of this CTA's sites, at this thread's site
+    double2 *at[6];    // v of the neighbours (distributed shared memory)
+    int sites, nranks, phase;
+    static constexpr int kWarps = kRitzClusterThreads / 32;
 
-// The half spinor of D src at the thread's site: own[c][0] spin h, own[c][1]
-// spin 3 - h of src there; the neighbours' components from src [8][V].
+    __device__ __forceinline__ RitzCluster(const RitzOne &a, double2 *smem, int sl, const int (&n)[6])
+        : own(smem + sl), sites(a.sites), phase(0) {
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        nranks = (int)cl.num_blocks();
+        for (int d = 0; d < 6; d++) at[d] = cl.map_shared_rank(smem, n[d] / sites) + n[d] % sites;
+        cl.sync();  // every CTA has started before its memory is written
+    }
+    __device__ __forceinline__ void put(int which, int comp, double re, double im) {
+        own[(size_t)(which * kComp + comp) * sites] = make_double2(re, im);
+    }
+    __device__ __forceinline__ cpx<double> get(int which, int dir, int comp) const {
+        const double2 u = at[dir][(size_t)(which * kComp + comp) * sites];
+        return mk<double>(u.x, u.y);
+    }
+    __device__ __forceinline__ bool sum(int nv, const double (&v)[kRitzParts], double (&out)[kRitzParts]) {
+        __shared__ double sh[kWarps][kRitzParts], all[2][kRitzClusterMax][kRitzParts];
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        const int par = phase & 1;
+        phase++;
+        if (nv > 0) {
+            ritz_warp_sums<kWarps>(nv, v, sh);
+            __syncthreads();
+            // this CTA's sums into every CTA's table
+            for (int i = threadIdx.x; i < nranks * nv; i += blockDim.x) {
+                const int k = i % nv;
+                double t = 0.0;
+                for (int w = 0; w < (int)blockDim.x / 32; w++) t += sh[w][k];
+                cl.map_shared_rank(&all[0][0][0], i / nv)[(par * kRitzClusterMax + (int)cl.block_rank()) * kRitzParts + k] = t;
+            }
+        }
+        cl.sync();
+        for (int k = 0; k < nv; k++) {
+            double t = 0.0;
+            for (int r = 0; r < nranks; r++) t += all[par][r][k];
+            out[k] = t;
+        }
+        return true;
+    }
+    __device__ __forceinline__ void finish() { cooperative_groups::this_cluster().sync(); }  // no CTA leaves while its memory is read
+};
+
+// The half spinor of D w at the thread's site: own[c][0] spin h, own[c][1]
+// spin 3 - h of w there; the neighbours' components through x (vector `which`).
 // The projections and reconstruction of hop() (ovl_stencil.cuh), half by half:
 // h0 and its products belong to half 0, h1 to half 1; in the z hops the lower
 // component rebuilt from one half's product belongs to the other half.
-__device__ __forceinline__ void ritz_half_d(const double *__restrict__ tab, const double2 *src, int V, const Nbrs &n,
-                                            int h, bool live, double amass, const cpx<double> (&own)[2][2],
-                                            cpx<double> (&out)[2][2]) {
+template <class X>
+__device__ __forceinline__ void ritz_half_d(const X &x, int which, const double *tab, int h, double amass,
+                                            const RitzHalf &own, RitzHalf &out) {
     const double sg = h ? -1.0 : 1.0;
-    cpx<double> acc[2][2];
+    RitzHalf acc;
 #pragma unroll
     for (int c = 0; c < 2; c++)
 #pragma unroll
         for (int k = 0; k < 2; k++) acc[c][k] = amass * own[c][k];
-    auto at = [&](int site, int comp) {
-        const double2 u = __ldcg(src + (size_t)comp * V + site);
-        return mk<double>(u.x, u.y);
-    };
     auto link = [&](int dir) {
         const double2 *q = reinterpret_cast<const double2 *>(tab + 8 * dir);
         const double2 a = q[0], b = q[1], c = q[2], d = q[3];
@@ -555,13 +651,12 @@ __device__ __forceinline__ void ritz_half_d(const double *__restrict__ tab, cons
     for (int dir = 0; dir < 6; dir++) {  // +x, +y, +z, -x, -y, -z as in the link table
         const int mu = dir % 3;
         const bool fwd = dir < 3;
-        const int nb = mu == 0 ? (fwd ? n.xp : n.xm) : (mu == 1 ? (fwd ? n.yp : n.ym) : (fwd ? n.zp : n.zm));
         const double s = fwd ? 1.0 : -1.0;
         cpx<double> hh[2], k[2];
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-            const cpx<double> up = at(nb, c * kSpin + h);
-            const cpx<double> lo = at(nb, c * kSpin + (mu == 2 ? 2 + h : 3 - h));
+            const cpx<double> up = x.get(which, dir, c * kSpin + h);
+            const cpx<double> lo = x.get(which, dir, c * kSpin + (mu == 2 ? 2 + h : 3 - h));
             if (mu == 0) hh[c] = mk<double>(fma(-s, lo.im, up.re), fma(s, lo.re, up.im));              // p_h +- i p_{3-h}
             else if (mu == 1) hh[c] = mk<double>(fma(s * sg, lo.re, up.re), fma(s * sg, lo.im, up.im));  // p_h +- sg p_{3-h}
             else hh[c] = mk<double>(fma(-s * sg, lo.im, up.re), fma(s * sg, lo.re, up.im));            // p_h +- sg i p_{2+h}
@@ -582,7 +677,6 @@ __device__ __forceinline__ void ritz_half_d(const double *__restrict__ tab, cons
             }
         }
     }
-    (void)live;
 #pragma unroll
     for (int c = 0; c < 2; c++) {  // -i gamma_0 / 2
         out[c][0] = 0.5 * times_mi(acc[c][0]);
@@ -590,51 +684,40 @@ __device__ __forceinline__ void ritz_half_d(const double *__restrict__ tab, cons
     }
 }
 
+// The CTA's link table: the six dressed links of each of its sites' hops.
 template <bool U1>
-__global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> lk, Lattice L, RitzOne a) {
-    __shared__ double tab_s[kRitzSites * kRitzTabStride];
-    const int prob = blockIdx.y, V = L.V;
-    const int sl = threadIdx.x >> 1, h = threadIdx.x & 1;
-    const int want = blockIdx.x * kRitzSites + sl;
-    const bool live = want < V;
-    const int site = live ? want : 0;  // a padded pair repeats site 0 and adds nothing
-    for (int i = threadIdx.x; i < kRitzSites * 6; i += kRitzOneThreads) {
-        const int s = blockIdx.x * kRitzSites + i / 6, dir = i % 6, mu = dir % 3;
-        if (s < V) {
-            int ls = s;
-            if (dir >= 3) {
-                const Nbrs n = neighbours(L, s);
-                ls = mu == 0 ? n.xm : (mu == 1 ? n.ym : n.zm);
-            }
-            const cmat2<double> M = lk.template get<double>(ls, mu);
-            double2 *o = reinterpret_cast<double2 *>(tab_s + (i / 6) * kRitzTabStride + 8 * dir);
-            o[0] = make_double2(M.m00.re, M.m00.im);
-            o[1] = make_double2(M.m01.re, M.m01.im);
-            o[2] = make_double2(M.m10.re, M.m10.im);
-            o[3] = make_double2(M.m11.re, M.m11.im);
+__device__ __forceinline__ void ritz_fill_links(const LinksF64<U1> &lk, const Lattice &L, int site0, int sites, double *tab) {
+    for (int i = threadIdx.x; i < sites * 6; i += blockDim.x) {
+        const int s = site0 + i / 6, dir = i % 6, mu = dir % 3;
+        if (s >= L.V) continue;
+        int ls = s;
+        if (dir >= 3) {
+            const Nbrs n = neighbours(L, s);
+            ls = mu == 0 ? n.xm : (mu == 1 ? n.ym : n.zm);
         }
+        const cmat2<double> M = lk.template get<double>(ls, mu);
+        double2 *o = reinterpret_cast<double2 *>(tab + (i / 6) * kRitzTabStride + 8 * dir);
+        o[0] = make_double2(M.m00.re, M.m00.im);
+        o[1] = make_double2(M.m01.re, M.m01.im);
+        o[2] = make_double2(M.m10.re, M.m10.im);
+        o[3] = make_double2(M.m11.re, M.m11.im);
     }
     __syncthreads();
-    const double *tab = tab_s + (live ? sl : 0) * kRitzTabStride;
-    const Nbrs n = neighbours(L, site);
+}
+
+// The iteration; x exchanges and sums.  A padded pair (live false) computes on
+// some site and adds nothing.
+template <class X>
+__device__ __forceinline__ void ritz_solve(X &ex, const RitzOne &a, const double *tab, int site, int h, bool live) {
+    const int prob = blockIdx.y;
     const double sign = prob == 0 ? 1.0 : -1.0;
-    double2 *v = a.v + (size_t)prob * kComp * V, *t = a.t + (size_t)prob * kComp * V;
-    RitzBarrier bar;
-    bar.nblocks = gridDim.x;
-    bar.slot_stride = (size_t)2 * gridDim.x * kRitzParts;
-    bar.part = a.part + (size_t)prob * gridDim.x * kRitzParts;
-    bar.count = a.count + prob;
-    bar.err = a.err;
-    bar.phase = 0;
-    using Half = cpx<double>[2][2];
-    auto store = [&](double2 *dst, const Half &f) {
-        if (!live) return;
+    auto store = [&](int which, const RitzHalf &f) {
 #pragma unroll
         for (int c = 0; c < 2; c++)
 #pragma unroll
-            for (int k = 0; k < 2; k++) __stcg(dst + (size_t)ritz_comp(c, k, h) * V + site, make_double2(f[c][k].re, f[c][k].im));
+            for (int k = 0; k < 2; k++) ex.put(which, ritz_comp(c, k, h), f[c][k].re, f[c][k].im);
     };
-    auto dot = [&](const Half &u, const Half &w, double &re, double &im) {
+    auto dot = [&](const RitzHalf &u, const RitzHalf &w, double &re, double &im) {
         if (!live) return;
 #pragma unroll
         for (int c = 0; c < 2; c++)
@@ -645,7 +728,7 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
             }
     };
 #define OVL_RITZ_EACH for (int c = 0; c < 2; c++) for (int k = 0; k < 2; k++)
-    Half x, y, p, z, g, raw;
+    RitzHalf x, y, p, z, g, raw;
     double s[kRitzParts], r[kRitzParts];
     auto clear = [&]() { s[0] = s[1] = s[2] = s[3] = 0.0; };
     // x = start / |start|
@@ -657,7 +740,7 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
     }
     clear();
     dot(x, x, s[0], s[3]);
-    if (!ritz_sum(bar, 1, s, r)) return;
+    if (!ex.sum(1, s, r)) return;
     {
         const double inv = 1.0 / sqrt(r[0]);
 #pragma unroll
@@ -668,18 +751,18 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
     bool stop = false;
     while (!stop) {
         // restart (RitzSolver.cpp:138-166): y = s A x, xy = <x, y>, g = raw direction = y - xy x
-        store(v, x);
-        if (!ritz_sum(bar, 0, s, r)) return;
-        Half w;
-        ritz_half_d(tab, v, V, n, h, live, a.amass, x, w);
-        store(t, w);
-        if (!ritz_sum(bar, 0, s, r)) return;
-        ritz_half_d(tab, t, V, n, h, live, a.amass, w, y);
+        store(0, x);
+        if (!ex.sum(0, s, r)) return;
+        RitzHalf w;
+        ritz_half_d(ex, 0, tab, h, a.amass, x, w);
+        store(1, w);
+        if (!ex.sum(0, s, r)) return;
+        ritz_half_d(ex, 1, tab, h, a.amass, w, y);
 #pragma unroll
         OVL_RITZ_EACH y[c][k] = (-sign) * y[c][k];
         clear();
         dot(x, y, s[0], s[1]);
-        if (!ritz_sum(bar, 2, s, r)) return;
+        if (!ex.sum(2, s, r)) return;
         xy_re = r[0];
         xy_im = r[1];
         clear();
@@ -690,8 +773,8 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
             raw[c][k] = g[c][k];
         }
         dot(g, g, s[0], s[3]);
-        store(v, raw);
-        if (!ritz_sum(bar, 1, s, r)) return;
+        store(0, raw);
+        if (!ex.sum(1, s, r)) return;
         raw2 = r[0];
         double gnormim = raw2;
         for (int itt = 1; itt <= a.nrestart && !stop; itt++) {
@@ -699,19 +782,19 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
             const double pnorm = sqrt(raw2), inv = 1.0 / pnorm;
 #pragma unroll
             OVL_RITZ_EACH p[c][k] = mk<double>(raw[c][k].re / pnorm, raw[c][k].im / pnorm);
-            ritz_half_d(tab, v, V, n, h, live, a.amass, raw, w);
+            ritz_half_d(ex, 0, tab, h, a.amass, raw, w);
 #pragma unroll
             OVL_RITZ_EACH w[c][k] = inv * w[c][k];
-            store(t, w);
-            if (!ritz_sum(bar, 0, s, r)) return;
+            store(1, w);
+            if (!ex.sum(0, s, r)) return;
             // z = s A p; <p, z>, <x, z>
-            ritz_half_d(tab, t, V, n, h, live, a.amass, w, z);
+            ritz_half_d(ex, 1, tab, h, a.amass, w, z);
 #pragma unroll
             OVL_RITZ_EACH z[c][k] = (-sign) * z[c][k];
             clear();
             dot(p, z, s[0], s[1]);
             dot(x, z, s[2], s[3]);
-            if (!ritz_sum(bar, 4, s, r)) return;
+            if (!ex.sum(4, s, r)) return;
             // the rotation in the (x, p) plane (RitzSolver.cpp:176-222)
             const double oxy_re = xy_re;
             double ct, sn;
@@ -725,7 +808,7 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
             clear();
             dot(x, x, s[0], s[3]);
             dot(x, y, s[1], s[2]);
-            if (!ritz_sum(bar, 3, s, r)) return;
+            if (!ex.sum(3, s, r)) return;
             // x normalised, xy, g (RitzSolver.cpp:224-243)
             const double xnorm = 1.0 / sqrt(r[0]);
             xy_re = r[1] * xnorm;
@@ -740,7 +823,7 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
             dot(g, g, s[0], s[3]);
             s[3] = 0.0;
             dot(x, p, s[1], s[2]);
-            if (!ritz_sum(bar, 3, s, r)) return;
+            if (!ex.sum(3, s, r)) return;
             // stopping tests and the new direction (RitzSolver.cpp:245-284)
             gnorm = r[0];
             const double xpr = r[1], xpi = r[2];
@@ -754,19 +837,49 @@ __global__ void __launch_bounds__(kRitzOneThreads) ritz_one_kernel(LinksF64<U1> 
                 raw[c][k] = mk<double>(g[c][k].re + beta * (p[c][k].re - xxp.re), g[c][k].im + beta * (p[c][k].im - xxp.im));
             }
             dot(raw, raw, s[0], s[3]);
-            store(v, raw);
-            if (!ritz_sum(bar, 1, s, r)) return;
+            store(0, raw);
+            if (!ex.sum(1, s, r)) return;
             raw2 = r[0];
             gnormim = gnorm;
         }
     }
 #undef OVL_RITZ_EACH
+    ex.finish();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.st[prob].xy_re = xy_re;
         a.st[prob].xy_im = xy_im;
         a.st[prob].ittot = ittot;
         a.st[prob].done = 1;
     }
+}
+
+template <bool U1>
+__global__ void __launch_bounds__(2 * kRitzGridSites) ritz_grid_kernel(LinksF64<U1> lk, Lattice L, RitzOne a) {
+    __shared__ double tab[kRitzGridSites * kRitzTabStride];
+    const int sl = threadIdx.x >> 1, h = threadIdx.x & 1, want = blockIdx.x * kRitzGridSites + sl;
+    const bool live = want < L.V;
+    const int site = live ? want : 0;  // a padded pair repeats site 0
+    ritz_fill_links(lk, L, blockIdx.x * kRitzGridSites, kRitzGridSites, tab);
+    const Nbrs n = neighbours(L, site);
+    const int nb[6] = {n.xp, n.yp, n.zp, n.xm, n.ym, n.zm};
+    RitzGrid ex(a, L, site, live, nb);
+    ritz_solve(ex, a, tab + (live ? sl : 0) * kRitzTabStride, site, h, live);
+}
+
+template <bool U1>
+__global__ void __launch_bounds__(kRitzClusterThreads) ritz_cluster_kernel(LinksF64<U1> lk, Lattice L, RitzOne a) {
+    extern __shared__ double2 smem[];
+    double *tab = reinterpret_cast<double *>(smem + (size_t)2 * kComp * a.sites);
+    const int sl = threadIdx.x >> 1, h = threadIdx.x & 1, want = blockIdx.x * a.sites + sl;
+    const bool live = want < L.V;
+    const int site = live ? want : 0;  // a padded pair computes on site 0's neighbours and stores to its own slot
+    for (int i = threadIdx.x; i < a.sites * kRitzTabStride; i += blockDim.x) tab[i] = 0.0;  // no link for padded sites
+    __syncthreads();
+    ritz_fill_links(lk, L, blockIdx.x * a.sites, a.sites, tab);
+    const Nbrs n = neighbours(L, site);
+    const int nb[6] = {n.xp, n.yp, n.zp, n.xm, n.ym, n.zm};
+    RitzCluster ex(a, smem, sl, nb);
+    ritz_solve(ex, a, tab + sl * kRitzTabStride, site, h, live);
 }
 
 // Start vector with the reference's distribution (Re, Im uniform in [0, 1),
@@ -809,6 +922,14 @@ struct RitzGraphs {
     }
 };
 
+// How a lattice of V sites is solved: by clusters of `ranks` CTAs of `sites`
+// sites (ranks > 0), by the cooperative launch (grid), or kernel by kernel.
+struct RitzPlan {
+    int ranks = 0, sites = 0;
+    size_t smem = 0;
+    bool grid = false;
+};
+
 struct RitzWork {
     double2 *x = nullptr, *y = nullptr, *z = nullptr, *t = nullptr, *p = nullptr, *praw = nullptr, *g = nullptr;
     double2 *start = nullptr;
@@ -819,6 +940,8 @@ struct RitzWork {
     int V = 0;
     int nc = 2;  // colours: vectors of 4 nc components per site
     RitzGraphs graphs;
+    RitzPlan plan[2];             // without and with a U(1) background
+    bool planned[2] = {false, false};
 };
 
 void *ritz_create(int V, int nc) {
@@ -826,8 +949,8 @@ void *ritz_create(int V, int nc) {
     w->V = V;
     w->nc = nc;
     const size_t vec = sizeof(double2) * 4 * nc * (size_t)V * 2;
-    // partials of the kernel-by-kernel iteration or of the one-launch solve (smaller CTAs)
-    const int nblocks = (V + kRitzSites - 1) / kRitzSites;
+    // partials of the kernel-by-kernel iteration or of the cooperative solve (smaller CTAs)
+    const int nblocks = (V + kRitzGridSites - 1) / kRitzGridSites;
     double2 **bufs[] = {&w->x, &w->y, &w->z, &w->t, &w->p, &w->praw, &w->g};
     bool ok = true;
     for (double2 **b : bufs) ok = ok && cudaMalloc(b, vec) == cudaSuccess;
@@ -1012,43 +1135,96 @@ static cudaError_t ritz_run_nc(RitzWork &w, const double *U, const double *u1, c
     return cudaSuccess;
 }
 
-// Whether the one-launch solve serves a lattice of V sites: its CTAs all fit
-// the GPU at once.  (up to 9472 sites on 148 SMs; beyond that, and for
-// three colours, whose vectors do not fit the registers, the iteration above.)
-template <bool U1> static bool ritz_one_fits(int V) {
+template <bool U1> static RitzPlan ritz_plan(int V) {
+    RitzPlan pl;
     int dev = 0, sms = 0, coop = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ritz_one_kernel<U1>, kRitzOneThreads, 0) != cudaSuccess) {
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return pl;
     }
-    return coop && 2LL * ((V + kRitzSites - 1) / kRitzSites) <= (long long)sms * per_sm;
+    // eight CTAs are the portable cluster size; sixteen halve the sites of a CTA
+    // where the GPU takes them
+    for (int ranks = 8; ranks <= kRitzClusterMax; ranks *= 2) {
+        const int sites = (((V + ranks - 1) / ranks + 15) / 16) * 16;  // whole warps of two threads per site
+        if (2 * sites > kRitzClusterThreads) continue;
+        const size_t smem = ritz_cluster_smem(sites);
+        // the attribute belongs to the kernel, not to this solve: always the largest
+        if (cudaFuncSetAttribute(ritz_cluster_kernel<U1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ritz_cluster_smem(kRitzClusterThreads / 2)) != cudaSuccess ||
+            (ranks > 8 && cudaFuncSetAttribute(ritz_cluster_kernel<U1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                              cudaSuccess)) {
+            cudaGetLastError();
+            continue;
+        }
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = ranks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ranks, 2);
+        cfg.blockDim = dim3(2 * sites);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, ritz_cluster_kernel<U1>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (clusters < 1) continue;
+        pl.ranks = ranks;
+        pl.sites = sites;
+        pl.smem = smem;
+        return pl;
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ritz_grid_kernel<U1>, 2 * kRitzGridSites, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return pl;
+    }
+    pl.grid = coop && 2LL * ((V + kRitzGridSites - 1) / kRitzGridSites) <= (long long)sms * per_sm;
+    return pl;
 }
 
 template <bool U1>
-static cudaError_t ritz_run_one(RitzWork &w, const double *U, const double *u1, const Lattice &L, double amass,
-                                int max_iter, int nrestart, double delitr, double out[2], int iters[2],
+static cudaError_t ritz_run_one(RitzWork &w, const RitzPlan &pl, const double *U, const double *u1, const Lattice &L,
+                                double amass, int max_iter, int nrestart, double delitr, double out[2], int iters[2],
                                 cudaStream_t stream, uint64_t *launches) {
     RitzOne a;
     a.start = w.start;
-    a.v = w.praw;
-    a.t = w.t;
-    a.part = w.part;
-    a.count = w.count;
-    a.err = w.count + 2;
     a.st = w.st;
     a.amass = amass;
     a.delitr = delitr;
     a.max_iter = max_iter;
     a.nrestart = nrestart;
+    a.sites = pl.ranks ? pl.sites : kRitzGridSites;
+    a.v = w.praw;
+    a.t = w.t;
+    a.part = w.part;
+    a.count = w.count;
+    a.err = w.count + 2;
     LinksF64<U1> lk{U, reinterpret_cast<const double2 *>(u1), L.N0 * L.N1};
     Lattice lat = L;
     cudaError_t e = cudaMemsetAsync(w.count, 0, sizeof(int) * 3, stream);
     if (e != cudaSuccess) return e;
-    void *args[] = {&lk, &lat, &a};
-    const dim3 grid((L.V + kRitzSites - 1) / kRitzSites, 2);
-    e = cudaLaunchCooperativeKernel(ritz_one_kernel<U1>, grid, dim3(kRitzOneThreads), args, 0, stream);
+    if (pl.ranks) {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = pl.ranks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(pl.ranks, 2);
+        cfg.blockDim = dim3(2 * pl.sites);
+        cfg.dynamicSmemBytes = pl.smem;
+        cfg.stream = stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, ritz_cluster_kernel<U1>, lk, lat, a);
+    } else {
+        void *args[] = {&lk, &lat, &a};
+        const dim3 grid((L.V + kRitzGridSites - 1) / kRitzGridSites, 2);
+        e = cudaLaunchCooperativeKernel(ritz_grid_kernel<U1>, grid, dim3(2 * kRitzGridSites), args, 0, stream);
+    }
     if (e != cudaSuccess) return e;
     int *err = reinterpret_cast<int *>(w.host + 2);
     if ((e = cudaMemcpyAsync(w.host, w.st, 2 * sizeof(RitzScalars), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
@@ -1074,9 +1250,15 @@ cudaError_t ritz_run(void *work, const double *U, const double *u1, const Lattic
     RitzWork &w = *static_cast<RitzWork *>(work);
     if (w.nc == 3)
         return ritz_run_nc<3>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
-    if (u1 ? ritz_one_fits<true>(L.V) : ritz_one_fits<false>(L.V))
-        return u1 ? ritz_run_one<true>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches)
-                  : ritz_run_one<false>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
+    const int b = u1 ? 1 : 0;
+    if (!w.planned[b]) {  // the work space belongs to one lattice size and device
+        w.plan[b] = u1 ? ritz_plan<true>(L.V) : ritz_plan<false>(L.V);
+        w.planned[b] = true;
+    }
+    const RitzPlan &pl = w.plan[b];
+    if (pl.ranks || pl.grid)
+        return u1 ? ritz_run_one<true>(w, pl, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches)
+                  : ritz_run_one<false>(w, pl, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
     return ritz_run_nc<2>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
 }
 
