@@ -37,7 +37,12 @@ struct ovl_ctx {
     double *partial = nullptr;    // reduction scratch
     size_t partial_doubles = 0;
     double *dev_small = nullptr;  // small device results
-    double *host_small = nullptr; // pinned mirror
+    // page-locked: the results a call waits for are written here by the last
+    // kernel itself (host memory is mapped into the device's address space), no
+    // copy between the kernel and the wait
+    double *host_small = nullptr;
+    double *host_bounce = nullptr; // page-locked, behind host_small: downloads up to bounce_bytes
+    size_t bounce_bytes = 0;
     int *dev_int = nullptr;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
@@ -824,8 +829,11 @@ int ovl_create(const ovl_params *p, ovl_ctx **out) {
         (rc = alloc((void **)&c->dev_small, sizeof(double) * 64, "results")) ||
         (rc = alloc((void **)&c->dev_int, sizeof(int) * 4, "flags")))
         return bail(rc);
-    if (cudaMallocHost(&c->host_small, sizeof(double) * 64) != cudaSuccess)
+    // the currents, links or E of lattices up to 4 MB of them
+    c->bounce_bytes = std::min((size_t)4 << 20, sizeof(double) * std::max({(size_t)ovl::kCurrentsPerSite * (size_t)V, n_link, n_e}));
+    if (cudaMallocHost(&c->host_small, sizeof(double) * 64 + c->bounce_bytes) != cudaSuccess)
         return bail(fail(c, OVL_E_OOM, "ovl_create: pinned host allocation failed"));
+    c->host_bounce = c->host_small + 64;
     if ((rc = alloc(&c->aux_src, field_bytes, "operator input")) || (rc = alloc(&c->aux_dst, field_bytes, "operator output")))
         return bail(rc);
     const size_t n_link32 = c->nc == 3 ? (size_t)ovl::kSu3Link32Floats * 3 * V : n_link;  // padded records
@@ -928,14 +936,25 @@ int ovl_set_links(ovl_ctx *c, const double *links) {
     return OVL_OK;
 }
 
+// n doubles of device memory into host memory, waited for.  Up to bounce_bytes
+// through the context's page-locked buffer: the driver's own staging of a copy
+// to pageable memory costs tens of microseconds a call.
+static int download(ovl_ctx *c, const double *dev, size_t n, double *host, const double **where = nullptr) {
+    const size_t bytes = sizeof(double) * n;
+    const bool bounce = bytes <= c->bounce_bytes;
+    double *to = bounce ? c->host_bounce : host;
+    OVL_CUDA(c, cudaMemcpyAsync(to, dev, bytes, cudaMemcpyDeviceToHost, c->stream));
+    OVL_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (where) *where = to;  // the caller reads it there
+    else if (bounce) std::memcpy(host, to, bytes);
+    return OVL_OK;
+}
+
 int ovl_get_links(ovl_ctx *c, double *links) {
     if (!c || !links) return fail(c, OVL_E_ARG, "ovl_get_links: null argument");
     int rc = set_device(c);
     if (rc) return rc;
-    OVL_CUDA(c, cudaMemcpyAsync(links, c->U, sizeof(double) * c->link_doubles * 3 * c->L.V, cudaMemcpyDeviceToHost,
-                                c->stream));
-    OVL_CUDA(c, cudaStreamSynchronize(c->stream));
-    return OVL_OK;
+    return download(c, c->U, (size_t)c->link_doubles * 3 * c->L.V, links);
 }
 
 int ovl_set_efield(ovl_ctx *c, const double *efield) {
@@ -999,10 +1018,7 @@ int ovl_get_efield(ovl_ctx *c, double *efield) {
     if (!c || !efield) return fail(c, OVL_E_ARG, "ovl_get_efield: null argument");
     int rc = set_device(c);
     if (rc) return rc;
-    OVL_CUDA(c, cudaMemcpyAsync(efield, c->E, sizeof(double) * c->e_comp * 3 * c->L.V, cudaMemcpyDeviceToHost,
-                                c->stream));
-    OVL_CUDA(c, cudaStreamSynchronize(c->stream));
-    return OVL_OK;
+    return download(c, c->E, (size_t)c->e_comp * 3 * c->L.V, efield);
 }
 
 // ---------------------------------------------------------------------------
@@ -1504,13 +1520,14 @@ static int step_observe(ovl_ctx *c, int nsteps, double *out, bool async) {
     if ((rc = coupled_efield(c))) return rc;
     {
         ProfScope ps(c, OVL_PROF_OBS);
-        nl = ovl::launch_obs_finish(c->obs_partial, obs_rows, c->obs_scratch, 1.0 / (2.0 * c->L.V), c->dev_small + 32,
-                                    c->stream);
+        nl = ovl::launch_obs_finish(c->obs_partial, obs_rows, c->obs_scratch, 1.0 / (2.0 * c->L.V),
+                                    (async ? c->dev_small : c->host_small) + 32, c->stream);
     }
     if ((rc = launched(c, nl, "charges (observing step)"))) return rc;
-    OVL_CUDA(c, cudaMemcpyAsync(async ? out : c->host_small + 32, c->dev_small + 32, sizeof(double) * 3,
-                                cudaMemcpyDeviceToHost, c->stream));
-    if (async) return OVL_OK;
+    if (async) {  // the caller's memory may be registered without being mapped at its own address: copied
+        OVL_CUDA(c, cudaMemcpyAsync(out, c->dev_small + 32, sizeof(double) * 3, cudaMemcpyDeviceToHost, c->stream));
+        return OVL_OK;
+    }
     OVL_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int k = 0; k < 3; k++) out[k] = c->host_small[32 + k];
     return OVL_OK;
@@ -1540,13 +1557,14 @@ int ovl_currents(ovl_ctx *c, double *jV, double *jA, double *jVw, double *jAw, d
     if (!c) return OVL_E_ARG;
     int rc = set_device(c);
     if (rc) return rc;
-    if ((rc = run_currents(c))) return rc;
     const int V = c->L.V;
-    std::vector<double> h((size_t)V * ovl::kCurrentsPerSite);
-    OVL_CUDA(c, cudaMemcpyAsync(h.data(), c->per_site, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
-    OVL_CUDA(c, cudaStreamSynchronize(c->stream));
+    const size_t n = (size_t)V * ovl::kCurrentsPerSite;
+    if ((rc = run_currents(c))) return rc;
+    std::vector<double> h(sizeof(double) * n > c->bounce_bytes ? n : 0);
+    const double *sites = nullptr;
+    if ((rc = download(c, c->per_site, n, h.data(), &sites))) return rc;
     for (int s = 0; s < V; s++) {
-        const double *q = h.data() + (size_t)s * ovl::kCurrentsPerSite;
+        const double *q = sites + (size_t)s * ovl::kCurrentsPerSite;
         for (int mu = 0; mu < 4; mu++) {
             if (jV) jV[4 * s + mu] = q[mu];
             if (jA) jA[4 * s + mu] = q[4 + mu];
@@ -1565,30 +1583,29 @@ int ovl_charges(ovl_ctx *c, double out[4]) {
     if (rc) return rc;
     if (overlap(c)) {
         if ((rc = run_currents(c))) return rc;
-        ovl::launch_site_sums(c->per_site, c->L, c->partial, c->dev_small, c->stream);
+        ovl::launch_site_sums(c->per_site, c->L, c->partial, c->host_small, c->stream);
         if ((rc = launched(c, 1, "site sums"))) return rc;
     } else if (su3(c)) {
         ProfScope ps(c, OVL_PROF_OBS);
         if (fp32(c))
             ovl::su3_launch_charges<float>(c->U, c->u1_on ? c->u1 : nullptr, c->psi, c->L, c->n_mb, c->p.n_modes,
-                                           c->p.first_mode, c->p.r_wilson, c->partial, c->dev_small, c->stream);
+                                           c->p.first_mode, c->p.r_wilson, c->partial, c->host_small, c->stream);
         else
             ovl::su3_launch_charges<double>(c->U, c->u1_on ? c->u1 : nullptr, c->psi, c->L, c->n_mb, c->p.n_modes,
-                                            c->p.first_mode, c->p.r_wilson, c->partial, c->dev_small, c->stream);
+                                            c->p.first_mode, c->p.r_wilson, c->partial, c->host_small, c->stream);
     } else {
         ProfScope ps(c, OVL_PROF_OBS);
         if (fp40(c))
             ovl::launch_charges40(c->U, c->u1_on ? c->u1 : nullptr, c->psi, c->psi_lo, c->L, c->n_mb, c->p.n_modes,
-                                  c->p.first_mode, c->p.r_wilson, c->partial, c->dev_small, c->stream);
+                                  c->p.first_mode, c->p.r_wilson, c->partial, c->host_small, c->stream);
         else if (fp32(c))
             ovl::launch_charges<float>(c->U, c->u1_on ? c->u1 : nullptr, c->psi, c->L, c->n_mb, c->p.n_modes, c->p.first_mode, c->p.r_wilson,
-                                       c->partial, c->dev_small, c->stream);
+                                       c->partial, c->host_small, c->stream);
         else
             ovl::launch_charges<double>(c->U, c->u1_on ? c->u1 : nullptr, c->psi, c->L, c->n_mb, c->p.n_modes, c->p.first_mode, c->p.r_wilson,
-                                        c->partial, c->dev_small, c->stream);
+                                        c->partial, c->host_small, c->stream);
     }
     if ((rc = launched(c, 2, "charges"))) return rc;
-    OVL_CUDA(c, cudaMemcpyAsync(c->host_small, c->dev_small, sizeof(double) * 4, cudaMemcpyDeviceToHost, c->stream));
     OVL_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int k = 0; k < 4; k++) out[k] = c->host_small[k];
     return OVL_OK;
@@ -1598,10 +1615,9 @@ int ovl_ncsdot(ovl_ctx *c, double *out) {
     if (!c || !out) return OVL_E_ARG;
     int rc = set_device(c);
     if (rc) return rc;
-    if (su3(c)) ovl::su3_launch_ncsdot(c->U, c->E, c->L, c->partial, c->dev_small, c->stream);
-    else ovl::launch_ncsdot(c->U, c->E, c->L, c->partial, c->dev_small, c->stream);
+    if (su3(c)) ovl::su3_launch_ncsdot(c->U, c->E, c->L, c->partial, c->host_small, c->stream);
+    else ovl::launch_ncsdot(c->U, c->E, c->L, c->partial, c->host_small, c->stream);
     if ((rc = launched(c, 2, "ncsdot"))) return rc;
-    OVL_CUDA(c, cudaMemcpyAsync(c->host_small, c->dev_small, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     OVL_CUDA(c, cudaStreamSynchronize(c->stream));
     *out = c->host_small[0];
     return OVL_OK;
@@ -1623,7 +1639,7 @@ int ovl_ncs_update(ovl_ctx *c, double *delta, double *total) {
     double d = 0.0;
     if (c->have_u_old) {
         // GetDeltaNCs(1): Simpson weights 1, 4, 1 at x = 0, 1/2, 1 (CoolingMethod.cpp:80-125)
-        double *out = c->dev_small;
+        double *out = c->host_small;
         if (su3(c)) {
             ovl::su3_launch_geodesic(c->u_old, c->U, 0.5, c->u_mid, c->e_mid, c->L, c->stream);
             ovl::su3_launch_ncsdot3(c->u_mid, c->u_old, c->U, c->e_mid, c->L, c->partial, out, c->stream);
@@ -1632,7 +1648,6 @@ int ovl_ncs_update(ovl_ctx *c, double *delta, double *total) {
             ovl::launch_ncsdot3(c->u_mid, c->u_old, c->U, c->e_mid, c->L, c->partial, out, c->stream);
         }
         if ((rc = launched(c, 3, "ncs update"))) return rc;
-        OVL_CUDA(c, cudaMemcpyAsync(c->host_small, out, sizeof(double) * 3, cudaMemcpyDeviceToHost, c->stream));
     }
     // the links of this call are the next call's old ones; one wait for the values and the copy
     OVL_CUDA(c, cudaMemcpyAsync(c->u_old, c->U, sizeof(double) * c->link_doubles * 3 * V, cudaMemcpyDeviceToDevice,
@@ -2095,9 +2110,8 @@ int ovl_bulk(ovl_ctx *c, double out[10]) {
     if (!c || !out) return OVL_E_ARG;
     int rc = set_device(c);
     if (rc) return rc;
-    ovl::launch_bulk(c->U, c->E, c->L, c->partial, c->dev_small, c->stream, c->nc);
+    ovl::launch_bulk(c->U, c->E, c->L, c->partial, c->host_small, c->stream, c->nc);
     if ((rc = launched(c, 2, "bulk"))) return rc;
-    OVL_CUDA(c, cudaMemcpyAsync(c->host_small, c->dev_small, sizeof(double) * 10, cudaMemcpyDeviceToHost, c->stream));
     OVL_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int k = 0; k < 10; k++) out[k] = c->host_small[k];
     return OVL_OK;
