@@ -545,10 +545,6 @@ int su3_autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
     uint64_t nl = 0;
     ovl::Su3Links lk = su3_links(c);
     const bool cheb = overlap(c) && c->p.sign_method == OVL_SIGN_CHEBYSHEV;
-    if (cheb) {
-        cudaMemsetAsync(c->cw.b1, 0, c->field_complex * c->elem_bytes, c->stream);
-        cudaMemsetAsync(c->cw.b2, 0, c->field_complex * c->elem_bytes, c->stream);
-    }
     const double lmax = std::pow(0.5 * std::fabs(amass(c->p)) + 3.0, 2);
     auto run = [&](int k) -> uint64_t {
         lk.variant = cand[k];

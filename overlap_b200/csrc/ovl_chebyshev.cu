@@ -95,13 +95,13 @@ __global__ void __launch_bounds__(kModeBlock *kSitesPerCta)
     });
 }
 
-// b_out = factor * (a * (-D w) + beta * b1) - b2 + ck * phi, per mode and site;
+// b_out = factor * (a * (-D w) + beta * b1) - s2 * b2 + ck * phi, per mode and site;
 // -D w is the stencil applied to w (the second half of X = -D^2 / lambda_max).
 template <typename T, class LK, bool TABLE>
 __global__ void __launch_bounds__(kModeBlock *kSitesPerCta)
     clenshaw_kernel(LK lk, const cpx<T> *__restrict__ w, const cpx<T> *__restrict__ b1, const cpx<T> *__restrict__ b2,
                     const cpx<T> *__restrict__ phi, cpx<T> *__restrict__ bout, Lattice L, T amass, T a, T beta,
-                    T factor, T ck, int n_mb, int mblk) {
+                    T factor, T s2, T ck, int n_mb, int mblk) {
     const int lane = threadIdx.x;
     cheb_blocks<T, TABLE>(lk, L, n_mb, mblk, [&](const auto &links, int site, int mb) {
         Spinor<T> acc;
@@ -115,28 +115,38 @@ __global__ void __launch_bounds__(kModeBlock *kSitesPerCta)
                 const cpx<T> dw = finish_component(acc.c[c][s], s);
                 const cpx<T> v1 = ld(b1 + i), v2 = ld(b2 + i), f = ld(phi + i);
                 const cpx<T> tx = mk<T>(-a * dw.re + beta * v1.re, -a * dw.im + beta * v1.im);
-                st(bout + i, mk<T>(factor * tx.re - v2.re + ck * f.re, factor * tx.im - v2.im + ck * f.im));
+                st(bout + i, mk<T>(factor * tx.re - s2 * v2.re + ck * f.re, factor * tx.im - s2 * v2.im + ck * f.im));
             }
     });
 }
 
-// out = M [ -i g0 (1 + m/2) phi + (1 - m/2) dchi ];  dst = out or dst += dt out
-template <typename T>
-__global__ void overlap_finish_t_kernel(const cpx<T> *__restrict__ phi, const cpx<T> *__restrict__ dchi, cpx<T> *dst,
-                                        size_t n, T mdw, T mf, T dt, int accumulate) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int spin = (int)((e / kModeBlock) % kComp) % kSpin;
-        const cpx<T> f = ld(phi + e), d = ld(dchi + e);
-        const T cp = (T)1 + (T)0.5 * mf, cm = (T)1 - (T)0.5 * mf;
-        const cpx<T> g = spin < 2 ? mk<T>(cp * f.im, -cp * f.re) : mk<T>(-cp * f.im, cp * f.re);
-        const cpx<T> o = mk<T>(mdw * (g.re + cm * d.re), mdw * (g.im + cm * d.im));
-        if (accumulate) {
-            const cpx<T> v = ld(dst + e);
-            st(dst + e, mk<T>(v.re + dt * o.re, v.im + dt * o.im));
-        } else {
-            st(dst + e, o);
-        }
-    }
+// out = M [ -i g0 (1 + m/2) phi + (1 - m/2) D chi ];  dst = out or dst += dt out
+template <typename T, class LK, bool TABLE>
+__global__ void __launch_bounds__(kModeBlock *kSitesPerCta)
+    overlap_combine_kernel(LK lk, const cpx<T> *__restrict__ chi, const cpx<T> *__restrict__ phi, cpx<T> *__restrict__ dst,
+                           Lattice L, T amass, T mdw, T mf, T dt, int accumulate, int n_mb, int mblk) {
+    const int lane = threadIdx.x;
+    const T cp = (T)1 + (T)0.5 * mf, cm = (T)1 - (T)0.5 * mf;
+    cheb_blocks<T, TABLE>(lk, L, n_mb, mblk, [&](const auto &links, int site, int mb) {
+        Spinor<T> acc;
+        wilson_site_lk(links, chi, L, site, mb, lane, amass, acc);
+        const size_t base = field_index(L.V, mb, site, 0, lane);
+#pragma unroll
+        for (int c = 0; c < kColours; c++)
+#pragma unroll
+            for (int s = 0; s < kSpin; s++) {
+                const size_t i = base + (c * kSpin + s) * kModeBlock;
+                const cpx<T> d = finish_component(acc.c[c][s], s), f = ld(phi + i);
+                const cpx<T> g = s < 2 ? mk<T>(cp * f.im, -cp * f.re) : mk<T>(-cp * f.im, cp * f.re);
+                const cpx<T> o = mk<T>(mdw * (g.re + cm * d.re), mdw * (g.im + cm * d.im));
+                if (accumulate) {
+                    const cpx<T> v = dst[i];
+                    st(dst + i, mk<T>(v.re + dt * o.re, v.im + dt * o.im));
+                } else {
+                    st(dst + i, o);
+                }
+            }
+    });
 }
 
 // w = D b over all modes: FP32 with hop variant 3 (and the FP32 link copy) in
@@ -157,9 +167,8 @@ static void d_pass(const LK &lk, const HopConfig &hc, const cpx<T> *b, cpx<T> *w
 template <typename T, class LK>
 static void cheb_run(const LK &lk, const HopConfig &hc, ChebyshevWork &w, const void *src, void *dst, const Lattice &L,
                      int n_mb, const double *coeff, int K, double eps, double lambda_max, double amass, double mdw,
-                     double mf, double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches) {
-    const size_t n = (size_t)n_mb * L.V * kComp * kModeBlock;
-    dim3 block(kModeBlock, kSitesPerCta);
+                     double mf, double dt, bool accumulate, cudaStream_t stream, uint64_t *launches) {
+    const dim3 block(kModeBlock, kSitesPerCta);
     const cpx<T> *phi = reinterpret_cast<const cpx<T> *>(src);
     cpx<T> *b[3] = {reinterpret_cast<cpx<T> *>(w.b0), reinterpret_cast<cpx<T> *>(w.b1), reinterpret_cast<cpx<T> *>(w.b2)};
     cpx<T> *tmp = reinterpret_cast<cpx<T> *>(w.w);
@@ -169,16 +178,19 @@ static void cheb_run(const LK &lk, const HopConfig &hc, ChebyshevWork &w, const 
     const T beta = (T)(-(1.0 + eps) / (1.0 - eps));
     const T am = (T)amass;
     uint64_t nl = 0;
-    // b_{K+1} = b_{K+2} = 0
-    cudaMemsetAsync(b[1], 0, n * sizeof(cpx<T>), stream);
-    cudaMemsetAsync(b[2], 0, n * sizeof(cpx<T>), stream);
+    // b_K = c_K phi (b_{K+1} = b_{K+2} = 0) is not formed: the next two terms read
+    // phi with c_K in their coefficients.  That saves one of the K + 1 terms and
+    // clearing two fields.
+    const T cK = (T)(coeff[K] * scale);
     int i1 = 1, i2 = 2, io = 0;  // b_{k+1}, b_{k+2}, b_k
-    for (int k = K; k >= 0; k--) {  // k = 0: y = t(X) b_1 - b_2 + c_0/2 phi (chi, scaled by lambda_max^-1/2)
-        d_pass<T>(lk, hc, b[i1], tmp, L, n_mb, am, stream);
+    for (int k = K - 1; k >= 0; k--) {  // k = 0: y = t(X) b_1 - b_2 + c_0/2 phi (chi, scaled by lambda_max^-1/2)
+        const cpx<T> *b1 = k == K - 1 ? phi : b[i1], *b2 = k >= K - 2 ? phi : b[i2];
+        const T s1 = k == K - 1 ? cK : (T)1, s2 = k == K - 1 ? (T)0 : (k == K - 2 ? cK : (T)1);
+        d_pass<T>(lk, hc, b1, tmp, L, n_mb, am, stream);
         const T factor = (T)(k > 0 ? 2 : 1), ck = (T)((k > 0 ? coeff[k] : 0.5 * coeff[0]) * scale);
         cheb_launch<T>(L, n_mb, [&](auto table, dim3 grid, int m) {
             clenshaw_kernel<T, LK, decltype(table)::value><<<grid, block, 0, stream>>>(
-                lk, tmp, b[i1], b[i2], phi, b[io], L, am, a, beta, factor, ck, n_mb, m);
+                lk, tmp, b1, b2, phi, b[io], L, am, a, beta, s1 * factor, s2, ck, n_mb, m);
         });
         nl += 2;
         const int t = i2;
@@ -186,12 +198,12 @@ static void cheb_run(const LK &lk, const HopConfig &hc, ChebyshevWork &w, const 
         i1 = io;
         io = t;
     }
-    // D chi (chi = b[i1]), then the overlap combination
-    d_pass<T>(lk, hc, b[i1], tmp, L, n_mb, am, stream);
-    size_t blocks = (n + 255) / 256, cap = (size_t)sm_count * 16;
-    overlap_finish_t_kernel<T><<<(int)(blocks < cap ? blocks : cap), 256, 0, stream>>>(
-        phi, tmp, reinterpret_cast<cpx<T> *>(dst), n, (T)mdw, (T)mf, (T)dt, accumulate ? 1 : 0);
-    nl += 2;
+    // D chi (chi = b[i1]) and the overlap combination in one pass
+    cheb_launch<T>(L, n_mb, [&](auto table, dim3 grid, int m) {
+        overlap_combine_kernel<T, LK, decltype(table)::value><<<grid, block, 0, stream>>>(
+            lk, b[i1], phi, reinterpret_cast<cpx<T> *>(dst), L, am, (T)mdw, (T)mf, (T)dt, accumulate ? 1 : 0, n_mb, m);
+    });
+    nl += 1;
     if (launches) *launches += nl;
 }
 
@@ -201,7 +213,7 @@ void chebyshev_apply(ChebyshevWork &w, const HopConfig &hc, const void *src, voi
                      double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches) {
     const int n01 = L.N0 * L.N1;
     auto go = [&](const auto &lk) {
-        cheb_run<T>(lk, hc, w, src, dst, L, n_mb, coeff, K, eps, lambda_max, amass, mdw, mf, dt, accumulate, sm_count,
+        cheb_run<T>(lk, hc, w, src, dst, L, n_mb, coeff, K, eps, lambda_max, amass, mdw, mf, dt, accumulate,
                     stream, launches);
     };
     if (sizeof(T) == 4 && hc.U32 != nullptr) {  // FP32 modes: the FP32 link copy

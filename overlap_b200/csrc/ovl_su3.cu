@@ -142,13 +142,13 @@ void su3_launch_update_links(double *U, const double *E, const Lattice &L, doubl
 }
 
 // --------------------------------------------------------- Chebyshev sign --
-// One Clenshaw term b_out = factor (a (-D w) + beta b1) - b2 + ck phi, -D w
+// One Clenshaw term b_out = factor (a (-D w) + beta b1) - s2 b2 + ck phi, -D w
 // the stencil applied to w = D b1 (ovl_chebyshev.cu, three colours).
 template <typename T, class LK>
 __global__ void __launch_bounds__(kModeBlock *kSites3, Occ3<T>::kMinBlocks)
     su3_clenshaw_kernel(LK lk, const cpx<T> *__restrict__ w, const cpx<T> *__restrict__ b1,
                         const cpx<T> *__restrict__ b2, const cpx<T> *__restrict__ phi, cpx<T> *__restrict__ bout,
-                        Lattice L, T amass, T a, T beta, T factor, T ck) {
+                        Lattice L, T amass, T a, T beta, T factor, T s2, T ck) {
     const int lane = threadIdx.x;
     const int site = blockIdx.x * kSites3 + threadIdx.y;
     const int mb = blockIdx.y;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kModeBlock *kSites3, Occ3<T>::kMinBlocks)
             const cpx<T> dw = (T)0.5 * (s < 2 ? times_mi(v) : times_i(v));
             const cpx<T> v1 = ld(b1 + i), v2 = ld(b2 + i), f = ld(phi + i);
             const cpx<T> tx = mk<T>(-a * dw.re + beta * v1.re, -a * dw.im + beta * v1.im);
-            st(bout + i, mk<T>(factor * tx.re - v2.re + ck * f.re, factor * tx.im - v2.im + ck * f.im));
+            st(bout + i, mk<T>(factor * tx.re - s2 * v2.re + ck * f.re, factor * tx.im - s2 * v2.im + ck * f.im));
         }
 }
 
@@ -201,19 +201,21 @@ static void cheb3(ChebyshevWork &w, const Su3Links &lk, const void *src, void *d
     cpx<T> *tmp = reinterpret_cast<cpx<T> *>(w.w);
     const double scale = 1.0 / std::sqrt(lambda_max);
     const T a = (T)(2.0 / ((1.0 - eps) * lambda_max)), beta = (T)(-(1.0 + eps) / (1.0 - eps)), am = (T)amass;
-    cudaMemsetAsync(b[1], 0, n * sizeof(cpx<T>), stream);
-    cudaMemsetAsync(b[2], 0, n * sizeof(cpx<T>), stream);
     int i1 = 1, i2 = 2, io = 0;
     uint64_t nl = 0;
     // variant 3 (FP32): the D passes in the packed stencil, and the overlap
     // combination fused into the last one
     const bool pk = packed3(lk, sizeof(T));
-    for (int k = K; k >= 0; k--) {
-        const T factor = (T)(k > 0 ? 2 : 1), ck = (T)((k > 0 ? coeff[k] : 0.5 * coeff[0]) * scale);
-        if (pk) packed3_launch<0>(lk, b[i1], tmp, L, n_mb, amass, 0.0, ClenshawArgs{}, stream);
-        else su3_wilson_kernel<T, 0, Links3<F32, U1>><<<grid, block, 0, stream>>>(links, b[i1], tmp, L, 0, am, (T)0);
-        su3_clenshaw_kernel<T, Links3<F32, U1>><<<grid, block, 0, stream>>>(links, tmp, b[i1], b[i2], phi, b[io], L, am,
-                                                                            a, beta, factor, ck);
+    // b_K = c_K phi is not formed (cheb_run, ovl_chebyshev.cu)
+    const T cK = (T)(coeff[K] * scale);
+    for (int k = K - 1; k >= 0; k--) {
+        const cpx<T> *b1 = k == K - 1 ? phi : b[i1], *b2 = k >= K - 2 ? phi : b[i2];
+        const T s1 = k == K - 1 ? cK : (T)1, s2 = k == K - 1 ? (T)0 : (k == K - 2 ? cK : (T)1);
+        const T factor = s1 * (T)(k > 0 ? 2 : 1), ck = (T)((k > 0 ? coeff[k] : 0.5 * coeff[0]) * scale);
+        if (pk) packed3_launch<0>(lk, b1, tmp, L, n_mb, amass, 0.0, ClenshawArgs{}, stream);
+        else su3_wilson_kernel<T, 0, Links3<F32, U1>><<<grid, block, 0, stream>>>(links, b1, tmp, L, 0, am, (T)0);
+        su3_clenshaw_kernel<T, Links3<F32, U1>><<<grid, block, 0, stream>>>(links, tmp, b1, b2, phi, b[io], L, am, a, beta,
+                                                                            factor, s2, ck);
         nl += 2;
         const int t = i2;
         i2 = i1;
