@@ -10,7 +10,9 @@
 // needs one application of X per term, X b = -D(D b) / lambda_max with
 // D = -i h_W.  Each term is two stencil launches: w = D b_{k+1}, then one
 // kernel that applies D to w and forms b_k in its epilogue (reads w with its
-// neighbours, b_{k+1}, b_{k+2}, phi; writes b_k).  The result
+// neighbours, b_{k+1}, b_{k+2}, phi; writes b_k).  Where the lattice fits on chip
+// for a few modes at a time the whole series is one launch (ovl_resident.cuh).
+// The result
 //   out = M [ -i g0 (1 + m/2) phi + (1 - m/2) D chi ],  chi = lambda_max^(-1/2) y
 // is the reference's overlap evolution operator (OverlapU.cpp:188-202) with the
 // Chebyshev approximation of the inverse square root; its error against the
@@ -20,6 +22,7 @@
 #include <vector>
 
 #include "ovl_internal.h"
+#include "ovl_resident.cuh"
 #include "ovl_stencil.cuh"
 
 namespace ovl {
@@ -212,6 +215,19 @@ void chebyshev_apply(ChebyshevWork &w, const HopConfig &hc, const void *src, voi
                      const double *coeff, int K, double eps, double lambda_max, double amass, double mdw, double mf,
                      double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches) {
     const int n01 = L.N0 * L.N1;
+    auto resident = [&](auto u1, const void *links, const void *phases) {
+        auto with = [&](auto... caps) {
+            return resident_apply<2, T, decltype(u1)::value, decltype(caps)...>(
+                w.resident, links, phases, src, dst, L, n_mb, w.b0, coeff, K, eps, lambda_max, amass, mdw, mf, dt,
+                accumulate, stream, launches);
+        };
+        if constexpr (sizeof(T) == 4) return with(ResidentCap<LanePair, 512>{});
+        else return with(ResidentCap<LaneOne<double>, 384>{});
+    };
+    if (sizeof(T) == 8 ? (hc.u1 ? resident(std::true_type{}, hc.U, hc.u1) : resident(std::false_type{}, hc.U, nullptr))
+                       : hc.U32 != nullptr && (hc.u1_32 ? resident(std::true_type{}, hc.U32, hc.u1_32)
+                                                        : resident(std::false_type{}, hc.U32, nullptr)))
+        return;
     auto go = [&](const auto &lk) {
         cheb_run<T>(lk, hc, w, src, dst, L, n_mb, coeff, K, eps, lambda_max, amass, mdw, mf, dt, accumulate,
                     stream, launches);

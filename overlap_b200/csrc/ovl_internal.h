@@ -279,10 +279,26 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
 // Chebyshev form of the overlap sign function (ovl_chebyshev.cu).
 constexpr int kMaxChebDegree = 1024;
 void chebyshev_inverse_sqrt(int K, double eps, double *c);
+struct ResidentShape {
+    int planes;  // per CTA (the last CTA of a cluster may hold fewer)
+    int groups;  // sets of modes per cluster: a CTA has groups x sites threads
+    int ranks;   // CTAs per cluster
+};
+
+// How a lattice is laid out on the chip, if it fits at all.
+struct ResidentPlan {
+    bool ok = false, u1 = false;
+    int modes = 0;          // the plan is for this many (0: none made yet)
+    int kernel = 0;         // index of the capacity
+    ResidentShape sh{};
+    size_t smem = 0;
+    double rate = 0.0;      // what it was chosen by
+};
 // Clenshaw vectors b0, b1, b2 and the temporary w = D b (one field each, mode
 // precision).
 struct ChebyshevWork {
     void *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *w = nullptr;
+    ResidentPlan resident;
 };
 // The overlap operator with the Chebyshev series on all mode blocks; FP32 modes
 // take the FP32 link copy when hc.U32 is set.

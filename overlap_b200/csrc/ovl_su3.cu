@@ -11,6 +11,7 @@
 #include "ovl_bilinears.cuh"
 #include "ovl_internal.h"
 #include "ovl_loops.cuh"
+#include "ovl_resident.cuh"
 #include "ovl_su3.cuh"
 #include "ovl_su3_packed.cuh"
 
@@ -192,6 +193,10 @@ template <typename T, bool F32, bool U1>
 static void cheb3(ChebyshevWork &w, const Su3Links &lk, const void *src, void *dst, const Lattice &L, int n_mb,
                   const double *coeff, int K, double eps, double lambda_max, double amass, double mdw, double mf,
                   double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches) {
+    if (resident_apply<3, T, U1, ResidentCap<LaneOne<T>, F32 ? 512 : 256>, ResidentCap<LaneOne<T>, F32 ? 576 : 224>>(
+            w.resident, F32 ? (const void *)lk.U32 : (const void *)lk.U, F32 ? (const void *)lk.u1_32 : (const void *)lk.u1,
+            src, dst, L, n_mb, w.b0, coeff, K, eps, lambda_max, amass, mdw, mf, dt, accumulate, stream, launches))
+        return;
     const size_t n = (size_t)n_mb * L.V * kComp3 * kModeBlock;
     const dim3 block(kModeBlock, kSites3), grid((L.V + kSites3 - 1) / kSites3, n_mb);
     Links3<F32, U1> links{F32 ? (const void *)lk.U32 : (const void *)lk.U, F32 ? (const void *)lk.u1_32 : (const void *)lk.u1,
