@@ -33,7 +33,7 @@ static int elem_grid(size_t n, int sm_count) {
 // component) of one mode block, 512 contiguous bytes each, so the CG scalars
 // of its 32 modes are read once per thread.  Grid (mode blocks, chunks of
 // rows), CTAs of kCgWarps warps.
-constexpr int kCgWarps = 8;
+constexpr int kCgWarps = 8, kCgRows = 2;
 
 // The sum of v over the CTA's warps, per lane, in a fixed order; warp 0 writes
 // it to part[chunk][mode].
@@ -322,55 +322,85 @@ __global__ void __launch_bounds__(kModeBlock *kCgWarps)
 // solutions is wanted, so the 25 x_k are not kept; per batch the kernel moves
 // 2 kact fields, the residuals of the batch and chi (HBM bound), against 4 x 25 + 1
 // fields per iteration for separate x_k and p_k.
+// The scalars of the batch, three per shift and iteration and mode, are staged in
+// shared memory once per CTA, for kShiftStage shifts at a time; left to L1 they are
+// more than it holds, and their reads from L2 as long as those of the fields.
 // One overlap leapfrog step with its two pairs of bounds at 8^3, 256 modes:
-// 50 ms with the shifts updated in every iteration, 42.9 ms in batches of eight.
-constexpr int kShiftRows = 2, kShiftWarps = 4;
+// 50 ms with the shifts updated in every iteration, 42.9 ms in batches of eight;
+// then, the Ritz solver made faster, 27.3 ms with the scalars left to L1 (508 us
+// per batch, 1.9 TB/s) and 20.1 ms with them staged (147 us, 6.6 TB/s; 160 us with
+// 12 warps, 188 us with 16 warps of one row each).
+constexpr int kShiftRows = 2, kShiftWarps = 16, kShiftStage = 32;
 
-__global__ void __launch_bounds__(kModeBlock *kShiftWarps, 3)
+inline size_t shift_smem(int npoles) {
+    return sizeof(double) * 3 * kCgBatch * kModeBlock * (size_t)std::min(npoles, kShiftStage);
+}
+
+__global__ void __launch_bounds__(kModeBlock *kShiftWarps, 1)
     shift_update_kernel(CgScalars s, cpx<double> *__restrict__ chi, cpx<double> *__restrict__ p,
                         const cpx<double> *__restrict__ r, int V, size_t n, int npoles, int modes_padded) {
+    extern __shared__ double shift_sc[];  // [shift of the stage][iteration][b beta, alpha, g][mode]
     const int lane = threadIdx.x, mb = blockIdx.x, rows = V * kComp, m = mb * kModeBlock + lane;
-    const int nj = s.steps[m];
-    if (nj == 0) return;
-    const int nk = s.kact[m];
+    const int nj = s.steps[m], nk = nj == 0 ? 0 : s.kact[m];
+    if (!__syncthreads_or(nk)) return;
     const size_t base = (size_t)mb * rows * kModeBlock + lane;
     const int step = gridDim.y * kShiftWarps;
-    for (int j0 = blockIdx.y * kShiftWarps + threadIdx.y; j0 < rows; j0 += step * kShiftRows) {
-        cpx<double> rv[kCgBatch][kShiftRows], x[kShiftRows];
-        size_t e[kShiftRows];
-#pragma unroll
-        for (int u = 0; u < kShiftRows; u++) {
-            e[u] = base + (size_t)min(j0 + u * step, rows - 1) * kModeBlock;
-            x[u] = chi[e[u]];
+    for (int k0 = 0; k0 < npoles; k0 += kShiftStage) {
+        const int staged = min(kShiftStage, npoles - k0), k1 = min(nk, k0 + staged);
+        if (k0) __syncthreads();
+        for (int i = threadIdx.y; i < staged * kCgBatch; i += kShiftWarps) {
+            const int k = i / kCgBatch, j = i % kCgBatch;
+            const size_t o = ((size_t)j * npoles + k0 + k) * modes_padded + m;
+            double *d = shift_sc + 3 * i * kModeBlock + lane;
+            d[0] = s.cb[o];
+            d[kModeBlock] = s.al[o];
+            d[2 * kModeBlock] = s.gg[o];
         }
+        __syncthreads();
+        if (k1 <= k0) continue;
+        for (int j0 = blockIdx.y * kShiftWarps + threadIdx.y; j0 < rows; j0 += step * kShiftRows) {
+            cpx<double> rv[kCgBatch][kShiftRows], x[kShiftRows], next[kShiftRows];
+            size_t e[kShiftRows];
 #pragma unroll
-        for (int j = 0; j < kCgBatch; j++)
+            for (int u = 0; u < kShiftRows; u++) {
+                e[u] = base + (size_t)min(j0 + u * step, rows - 1) * kModeBlock;
+                x[u] = chi[e[u]];
+                next[u] = p[(size_t)k0 * n + e[u]];
+            }
 #pragma unroll
-            for (int u = 0; u < kShiftRows; u++) rv[j][u] = j < nj ? ld(r + (size_t)j * n + e[u]) : mk<double>(0.0, 0.0);
-        for (int k = 0; k < nk; k++) {
-            cpx<double> *pk = p + (size_t)k * n;
-            cpx<double> pv[kShiftRows];
+            for (int j = 0; j < kCgBatch; j++)
 #pragma unroll
-            for (int u = 0; u < kShiftRows; u++) pv[u] = pk[e[u]];
+                for (int u = 0; u < kShiftRows; u++)
+                    rv[j][u] = j < nj ? ld(r + (size_t)j * n + e[u]) : mk<double>(0.0, 0.0);
+            for (int k = k0; k < k1; k++) {
+                cpx<double> *pk = p + (size_t)k * n;
+                cpx<double> pv[kShiftRows];
 #pragma unroll
-            for (int j = 0; j < kCgBatch; j++) {
-                if (j < nj) {
-                    const size_t o = ((size_t)j * npoles + k) * modes_padded + m;
-                    const double cb = s.cb[o], ak = s.al[o], gk = s.gg[o];
+                for (int u = 0; u < kShiftRows; u++) {
+                    pv[u] = next[u];
+                    if (k + 1 < k1) next[u] = pk[n + e[u]];  // in flight while this shift is brought up to date
+                }
+                const double *sc = shift_sc + 3 * (k - k0) * kCgBatch * kModeBlock + lane;
 #pragma unroll
-                    for (int u = 0; u < kShiftRows; u++) {
-                        x[u] = mk<double>(x[u].re + cb * pv[u].re, x[u].im + cb * pv[u].im);
-                        pv[u] = mk<double>(pv[u].re * ak + rv[j][u].re * gk, pv[u].im * ak + rv[j][u].im * gk);
+                for (int j = 0; j < kCgBatch; j++) {
+                    if (j < nj) {
+                        const double cb = sc[3 * j * kModeBlock], ak = sc[(3 * j + 1) * kModeBlock],
+                                     gk = sc[(3 * j + 2) * kModeBlock];
+#pragma unroll
+                        for (int u = 0; u < kShiftRows; u++) {
+                            x[u] = mk<double>(x[u].re + cb * pv[u].re, x[u].im + cb * pv[u].im);
+                            pv[u] = mk<double>(pv[u].re * ak + rv[j][u].re * gk, pv[u].im * ak + rv[j][u].im * gk);
+                        }
                     }
                 }
+#pragma unroll
+                for (int u = 0; u < kShiftRows; u++)
+                    if (j0 + u * step < rows) st(pk + e[u], pv[u]);
             }
 #pragma unroll
             for (int u = 0; u < kShiftRows; u++)
-                if (j0 + u * step < rows) st(pk + e[u], pv[u]);
+                if (j0 + u * step < rows) st(chi + e[u], x[u]);
         }
-#pragma unroll
-        for (int u = 0; u < kShiftRows; u++)
-            if (j0 + u * step < rows) st(chi + e[u], x[u]);
     }
 }
 
@@ -491,7 +521,7 @@ int cg_square_chunks(const Lattice &L) { return (L.V + kSitesPerCta - 1) / kSite
 // Chunks of rows of the vector kernels: at least four CTAs per SM where the
 // rows allow it, at most kDotChunks.
 static int cg_chunks(const Lattice &L, int n_mb, int sm_count) {
-    const int most = std::min(kDotChunks, (L.V * kComp + kCgWarps * kShiftRows - 1) / (kCgWarps * kShiftRows));
+    const int most = std::min(kDotChunks, (L.V * kComp + kCgWarps * kCgRows - 1) / (kCgWarps * kCgRows));
     return std::max(1, std::min(most, (8 * sm_count + n_mb - 1) / n_mb));
 }
 
@@ -556,8 +586,13 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
         cudaEventSynchronize(w.counted[slot]);
         return w.host_count[slot];
     };
+    // a CTA per SM and one wave of them, or four CTAs per mode block where there are more blocks than SMs
+    const int shift_ctas = std::max(1, std::min(n_mb > sm_count ? 4 : sm_count / n_mb,
+                                                (L.V * kComp + kShiftWarps * kShiftRows - 1) / (kShiftWarps * kShiftRows)));
+    cudaFuncSetAttribute(shift_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shift_smem(kShiftStage));
     auto update_shifts = [&]() {
-        shift_update_kernel<<<dim3(n_mb, 2 * chunks), dim3(kModeBlock, kShiftWarps), 0, stream>>>(s, chi, p, r, L.V, n, np, mp);
+        shift_update_kernel<<<dim3(n_mb, shift_ctas), dim3(kModeBlock, kShiftWarps), shift_smem(np), stream>>>(s, chi, p, r, L.V,
+                                                                                                          n, np, mp);
         launches++;
     };
     read_count(0);
