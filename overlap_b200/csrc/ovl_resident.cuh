@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(CAP, 1)
 #pragma unroll
         for (int a = 0; a < kSpin; a++) b2[c][a] = {vsplat<V>((T)0), vsplat<V>((T)0)};
     if (live) {
-        const V cK = vsplat<V>(A.c[A.K]);
+        const V cK = vsplat<V>(A.K & 2 ? -A.c[A.K] : A.c[A.K]);  // signed as below
         const Slot *in = reinterpret_cast<const Slot *>(A.phi) + base;
 #pragma unroll
         for (int c = 0; c < NC; c++)
@@ -459,18 +459,20 @@ __global__ void __launch_bounds__(CAP, 1)
         wait();
         if (live) {
             outer(1, acc);
-            // b_k = factor (a (-D w) + beta b_{k+1}) - b_{k+2} + c_k phi
+            // b_k = factor (a (-D w) + beta b_{k+1}) - b_{k+2} + c_k phi, three roundings.
+            // The fields hold s_k b_k with s = +, +, -, -, ... from k = 0, so that
+            // b_{k+2} is added and every sign is in a coefficient.
             const Slot *q = res_here(phi);
-            const T factor = (T)(k > 0 ? 2 : 1);
-            const V fa = vsplat<V>(-factor * A.a), fb = vsplat<V>(factor * A.beta), ck = vsplat<V>(A.c[k]);
+            const T factor = (T)(k & 1 ? -2 : k > 0 ? 2 : 1);
+            const V fa = vsplat<V>(-factor * A.a), fb = vsplat<V>(factor * A.beta), ck = vsplat<V>(k & 2 ? -A.c[k] : A.c[k]);
 #pragma unroll
             for (int c = 0; c < NC; c++)
 #pragma unroll
                 for (int a = 0; a < kSpin; a++) {
                     const vcpx<V> d = finish(acc[c][a], a), v1 = slot_get(buf[(size_t)(c * kSpin + a) * CAP + me]),
                                   f = phi_at(q, c * kSpin + a);
-                    acc[c][a].re = vfma(ck, f.re, vsub(vfma(fb, v1.re, vmul(fa, d.re)), b2[c][a].re));
-                    acc[c][a].im = vfma(ck, f.im, vsub(vfma(fb, v1.im, vmul(fa, d.im)), b2[c][a].im));
+                    acc[c][a].re = vfma(fa, d.re, vfma(fb, v1.re, vfma(ck, f.re, b2[c][a].re)));
+                    acc[c][a].im = vfma(fa, d.im, vfma(fb, v1.im, vfma(ck, f.im, b2[c][a].im)));
                     b2[c][a] = v1;
                 }
             publish(0, acc);
