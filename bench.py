@@ -187,6 +187,14 @@ def _ref_worker(args):
     return m, secs
 
 
+def have_reference() -> bool:
+    """Whether the reference was compiled here (its sources may be absent)."""
+    sys.path.insert(0, str(ROOT / "tests"))
+    from _oracle import have_reference as built
+
+    return built("wilson")
+
+
 def reference_cpu(wl, steps: int, warmup: int, max_procs: int | None = None):
     """Aggregate MSU/s of the reference hot path on this host: one process per
     core, each an emulated MPI rank (MPI/ModePartition.cpp:12-24) holding
@@ -726,7 +734,9 @@ def main():
               "l2": "inputs larger than L2 (no flush)", "parallelism": f"replicas x{world}"}
 
     if args.impl == "reference":
-        if rank == 0:
+        if rank == 0 and not have_reference():
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not on this machine"}), flush=True)
+        elif rank == 0:
             # the GPU arm's step and warm-up counts; a step is one leapfrog step of
             # every process's 64-mode slice (about 0.15 s per process at N=16)
             steps, warmup = max(1, args.steps), max(3, args.warmup)
@@ -741,7 +751,7 @@ def main():
         return
 
     cpu = None
-    if rank == 0 and not args.no_cpu_baseline:
+    if rank == 0 and not args.no_cpu_baseline and have_reference():
         # before any CUDA call (spawned workers)
         # about 2.5 s per process: 12 steps of a 64-mode slice at N=16, 60 at N=8
         cpu = reference_cpu(wl, steps=12 if args.workload == "n16" else 60, warmup=0, max_procs=64)
