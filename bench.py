@@ -625,10 +625,13 @@ def su3_overlap_leg(steps, warmup, device, modes=0):
     # term reads b_{k+1} and b_{k+2} and writes b_k once, 3 K elements per
     # mode-site, plus 6 for phi, D chi and the combination into the destination)
     alg = field * (3 * K + 6)
-    # the field passes the kernels make as built: 7 per term (w = D b: read b,
-    # write w; term: read w, b_1, b_2, phi, write b_0), K + 1 terms, then D chi
-    # (2) and the combination into the destination (4); two memsets (2)
-    built = field * (7 * (K + 1) + 8)
+    # the field passes the kernels make as built.  On chip (one launch for the
+    # whole operator): phi read and laid out again, the destination read and
+    # written (phi's reads in every term come from L2).  Through memory: 7 per term
+    # (w = D b: read b, write w; term: read w, b_1, b_2, phi, write b_0), K terms,
+    # then D chi and the combination into the destination (read chi, phi and the
+    # destination, write it)
+    built = field * (4 if launches / steps < K else 7 * K + 4)
     half_ms = ms / (2 * steps)
     peak, peak_kind = measured_peaks()
     return {"config": f"SU(3), N=12^3, overlap (Chebyshev degree {K}, [eps, 1] = [{eps}, 1]), Wilson kernel mass -1, "
