@@ -532,7 +532,7 @@ int autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
 // stencil (variant 3), timed on the operator buffer as the context uses the
 // stencil (the fused half step for Wilson contexts; for overlap contexts a
 // Chebyshev series of degree 3, whose D passes and final combination differ
-// between the variants); the state is not touched.
+// between the variants where it goes through memory); the state is not touched.
 int su3_autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
     if (ms_out)
         for (int v = 0; v < ovl::kHopVariants; v++) ms_out[v] = 0.0;

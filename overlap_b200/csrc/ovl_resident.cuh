@@ -16,7 +16,7 @@
 // is two phases, each ending in a barrier of the cluster that is waited for only
 // where the half spinors are read.
 // One overlap step, through memory and here: 8^3, two colours, 4096 FP32 modes,
-// degree 64: 23.7 and 10.1 ms (one CTA; L1 data pipe 89 % busy); 12^3, three
+// degree 64: 23.7 and 10.1 ms (one CTA; L1 data pipe 92 % busy); 12^3, three
 // colours, 1536 FP32 modes, degree 96: 71.0 and 58.3 ms (six CTAs; 65.0 ms reading
 // whole spinors from the other CTAs, 53.0 ms if nothing had to come from them).
 #pragma once
