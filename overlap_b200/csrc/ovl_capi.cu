@@ -861,10 +861,10 @@ int ovl_create(const ovl_params *p, ovl_ctx **out) {
     if (p->fermion == OVL_FERMION_OVERLAP && p->sign_method == OVL_SIGN_ZOLOTAREV) {
         ovl::OverlapWork &w = c->ow;
         const size_t mp = (size_t)c->n_mb * ovl::kModeBlock, np = (size_t)p->zolo_poles;
-        if ((rc = alloc(&w.r, field_bytes * ovl::kCgBatchSlots, "CG residuals")) ||
+        if ((rc = alloc(&w.r, field_bytes * ovl::cg_batch_slots(p->zolo_poles), "CG residuals")) ||
             (rc = alloc(&w.q, field_bytes, "CG direction image")) || (rc = alloc(&w.p0, field_bytes, "CG direction")) ||
             (rc = alloc(&w.t, field_bytes, "CG temporary")) || (rc = alloc(&w.x, field_bytes, "shifted solutions")) ||
-            (rc = alloc(&w.p, field_bytes * np, "shifted directions")) ||
+            (np > 1 && (rc = alloc(&w.p, field_bytes * np, "shifted directions"))) ||
             (rc = alloc((void **)&w.part, sizeof(double) * ovl::cg_partial_chunks(c->L) * mp, "dot partials")) ||
             (rc = alloc((void **)&w.scalars, sizeof(double) * mp * ovl::kCgModeScalars, "CG scalars")) ||
             (rc = alloc((void **)&w.shifts, sizeof(double) * mp * np * (2 + 3 * ovl::kCgBatchSlots), "shift scalars")) ||

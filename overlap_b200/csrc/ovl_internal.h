@@ -249,11 +249,17 @@ struct OverlapCoeffs {
 };
 
 // Device work space of the batched multi-shift CG (all FP64, mode-block layout).
-constexpr int kCgBatchSlots = 8;  // iterations between two updates of the shifted vectors
+constexpr int kCgBatchSlots = 8;  // iterations between two updates of the shifted vectors, at most
+// With few poles the batches are shorter, so that the residuals kept never take
+// more fields than the npoles solutions x_k would: slots + 4 + npoles <= 3 + 2 npoles
+// (one pole: its direction shares t, below).
+inline int cg_batch_slots(int npoles) {
+    return npoles <= 2 ? 1 : (npoles > kCgBatchSlots ? kCgBatchSlots : npoles - 1);
+}
 struct OverlapWork {
-    void *r = nullptr;                              // kCgBatchSlots fields: the residuals of a batch
+    void *r = nullptr;                              // cg_batch_slots fields: the residuals of a batch
     void *q = nullptr, *t = nullptr, *p0 = nullptr, *x = nullptr;  // one field each (x: chi)
-    void *p = nullptr;                              // npoles fields
+    void *p = nullptr;                              // npoles fields; null for one pole
     double *part = nullptr;                         // cg_partial_chunks x modes
     double *scalars = nullptr;                      // kCgModeScalars x modes
     double *shifts = nullptr;                       // (2 + 3 kCgBatchSlots) x npoles x modes

@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(kModeBlock *kCgWarps)
 
 // beta_0 = rnorm / <p0, q> (OverlapU.cpp:71-75) from the partial sums of <p0, q>,
 // rout = rin - beta_0 q for active modes, and the partial sums of |rout|^2.
-// Clears this iteration's count.
+// INPLACE: rin is rout (a batch of one iteration).  Clears this iteration's count.
+template <bool INPLACE>
 __global__ void __launch_bounds__(kModeBlock *kCgWarps)
     residual_kernel(CgScalars s, int parity, const double *__restrict__ pap_part, int pap_chunks,
                     const cpx<double> *__restrict__ rin, cpx<double> *__restrict__ rout, const cpx<double> *__restrict__ q,
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kModeBlock *kCgWarps)
     if (act)
         for (int j = blockIdx.y * kCgWarps + threadIdx.y; j < rows; j += gridDim.y * kCgWarps) {
             const size_t e = base + (size_t)j * kModeBlock;
-            const cpx<double> a = ld(rin + e), y = ld(q + e);
+            const cpx<double> a = INPLACE ? rout[e] : ld(rin + e), y = ld(q + e);
             const cpx<double> v = mk<double>(a.re - b * y.re, a.im - b * y.im);
             st(rout + e, v);
             t += v.re * v.re + v.im * v.im;
@@ -246,10 +247,13 @@ constexpr double kShiftDone = 1e-20;
 // (OverlapU.cpp:71-88), alpha_k and g_k as the shift loop of :95-106 computes
 // them (alpha_0 is rewritten at k = 0 before the other shifts read it) -- then
 // betam = beta_0, the iteration count and the stopping test (:56, 110-117).
+// keep (or null): receives p0 of before the step, the direction that a single
+// shift's update needs after it.
 __global__ void __launch_bounds__(kModeBlock *kCgWarps)
     cg_advance_kernel(CgScalars s, int parity, int slot, const double *__restrict__ part, int chunks,
                       const double *__restrict__ dz, const double *__restrict__ bz, int npoles, double cgerr, int max_iter,
-                      cpx<double> *__restrict__ p0, const cpx<double> *__restrict__ r, int V, int modes_padded) {
+                      cpx<double> *__restrict__ p0, const cpx<double> *__restrict__ r, cpx<double> *__restrict__ keep,
+                      int V, int modes_padded) {
     const int lane = threadIdx.x, mb = blockIdx.x, m = mb * kModeBlock + lane;
     const double rr = cg_total(part, chunks, m, modes_padded);
     const bool active = s.active[m] != 0;
@@ -263,6 +267,7 @@ __global__ void __launch_bounds__(kModeBlock *kCgWarps)
         for (int j = (blockIdx.y - 1) * kCgWarps + threadIdx.y; j < rows; j += (gridDim.y - 1) * kCgWarps) {
             const size_t e = base + (size_t)j * kModeBlock;
             const cpx<double> pv = p0[e], rv = ld(r + e);
+            if (keep) st(keep + e, pv);
             st(p0 + e, mk<double>(pv.re * a0 + rv.re, pv.im * a0 + rv.im));
         }
         return;
@@ -538,7 +543,11 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
     const cpx<double> *phi = reinterpret_cast<const cpx<double> *>(src);
     cpx<double> *r = reinterpret_cast<cpx<double> *>(w.r), *q = reinterpret_cast<cpx<double> *>(w.q);
     cpx<double> *t = reinterpret_cast<cpx<double> *>(w.t), *p0 = reinterpret_cast<cpx<double> *>(w.p0);
-    cpx<double> *chi = reinterpret_cast<cpx<double> *>(w.x), *p = reinterpret_cast<cpx<double> *>(w.p);
+    cpx<double> *chi = reinterpret_cast<cpx<double> *>(w.x);
+    // One pole: its direction at the start of a batch of one is p0 before the
+    // step, kept in t, which is free between two applications of D.
+    cpx<double> *const keep = np == 1 ? t : nullptr, *const p = np == 1 ? t : reinterpret_cast<cpx<double> *>(w.p);
+    const int slots = cg_batch_slots(np);
     CgScalars s;
     const size_t pm = (size_t)np * mp;
     s.rnorm[0] = w.scalars;
@@ -569,7 +578,7 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
     double *const pap_fold = pap_part + (size_t)sq_chunks * mp;
     const dim3 vblock(kModeBlock, kCgWarps), vgrid(n_mb, chunks);
     // the residual of slot j is r[j]; the iteration of slot 0 starts from the last slot
-    mscg_init_vectors_kernel<<<vgrid, vblock, 0, stream>>>(phi, r + (size_t)(kCgBatch - 1) * n, p0, p, chi, L.V, n, np, rr_part,
+    mscg_init_vectors_kernel<<<vgrid, vblock, 0, stream>>>(phi, r + (size_t)(slots - 1) * n, p0, p, chi, L.V, n, np, rr_part,
                                                            mp);
     cudaMemsetAsync(count, 0, sizeof(int) * 2, stream);
     cg_init_scalars_kernel<<<n_mb, vblock, 0, stream>>>(s, rr_part, chunks, n_modes, mp, np, co.cg_tol);
@@ -598,24 +607,24 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
     read_count(0);
     int iterations = 0;
     for (int it = 0;; it++) {
-        const int slot = it % kCgBatch, par = it & 1;
-        cpx<double> *rin = r + (size_t)((slot + kCgBatch - 1) % kCgBatch) * n, *rout = r + (size_t)slot * n;
+        const int slot = it % slots, par = it & 1;
+        cpx<double> *rin = r + (size_t)((slot + slots - 1) % slots) * n, *rout = r + (size_t)slot * n;
         // q = h_W^2 p0 + d0 p0 = -D(D p0) + d0 p0
         s.count = count + (par ^ 1);
         launch_wilson<double>(U, u1, p0, w.t, L, 0, n_mb, amass, 0.0, false, stream);
         launch_cg_square(U, u1, w.t, p0, q, L, n_mb, amass, co.d[0], pap_part, mp, stream);
         if (fold) cg_fold_kernel<<<dim3(n_mb, kDotChunks / kCgWarps), vblock, 0, stream>>>(pap_part, sq_chunks, pap_fold, mp);
-        residual_kernel<<<vgrid, vblock, 0, stream>>>(s, par, fold ? pap_fold : pap_part, fold ? kDotChunks : sq_chunks, rin,
-                                                      rout, q, L.V, rr_part, mp);
+        (slots > 1 ? residual_kernel<false> : residual_kernel<true>)<<<vgrid, vblock, 0, stream>>>(
+            s, par, fold ? pap_fold : pap_part, fold ? kDotChunks : sq_chunks, rin, rout, q, L.V, rr_part, mp);
         cg_advance_kernel<<<dim3(n_mb, chunks + 1), vblock, 0, stream>>>(s, par, slot, rr_part, chunks, w.dz, w.bz, np,
-                                                                         co.cg_tol, co.cg_max_iter, p0, rout, L.V, mp);
+                                                                         co.cg_tol, co.cg_max_iter, p0, rout, keep, L.V, mp);
         launches += fold ? 5 : 4;
         std::swap(s.active, s.next);
         read_count(par ^ 1);
         const bool over = counted(par) == 0;  // no mode was active before this iteration
         if (!over) iterations++;
         const bool stop = over || iterations > co.cg_max_iter + 1;  // every mode stops by then
-        if (slot == kCgBatch - 1 || (stop && slot > 0)) update_shifts();
+        if (slot == slots - 1 || (stop && slot > 0)) update_shifts();
         if (stop) break;
     }
     launch_wilson<double>(U, u1, chi, w.t, L, 0, n_mb, amass, 0.0, false, stream);

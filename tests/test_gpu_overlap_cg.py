@@ -98,3 +98,53 @@ def test_cg_batches_match_the_reference_loop(max_iter, poles):
     assert abs(stats["max_mode_iterations"] - max(its)) <= 1
     if max_iter == 1000:
         assert len(set(its)) > 3 and stats["not_converged"] == 0
+
+
+# Few poles: batches of one (1 and 2 poles; with one its direction shares a temporary), 2, 3 and 7 iterations
+@pytest.mark.parametrize("poles,max_iter", [(1, 1), (1, 1000), (2, 5), (2, 1000), (3, 3), (3, 1000), (4, 7), (8, 15)])
+def test_cg_with_few_poles_matches_the_reference_loop(poles, max_iter):
+    N = (3, 4, 3)
+    U = random_links(N, 0.5, 11)
+    D = dense_d(N, U)
+    lam = np.linalg.eigvalsh(-(D @ D))
+    lo, hi = 0.95 * lam[0], 1.05 * lam[-1]
+    b, d, _ = zolotarev(lo, hi, npoles=poles)
+    phi = random_modes(35, N, 12)
+    phi *= 10.0 ** np.linspace(-7, 3, 35)[:, None, None, None]
+    with Context(N=N, n_modes=35, fermion="overlap", precision="fp64", m_fermion=M, m_dw=MDW, cg_max_iter=max_iter,
+                 zolo_poles=poles) as ctx:
+        ctx.set_links(U)
+        ctx.set_spectral_bounds([(lo, hi)])
+        out = ctx.apply(phi)
+    # sum_k sqrt(l) b_k / (l + d_k) at the eigenvalues l: 1 for many poles, at most this for few
+    sign = max(np.sum(np.sqrt(l) * b / (l + d)) for l in lam)
+    for m in range(35):
+        want, it = overlap_u(D, phi[m].ravel(), b, d, 1e-16, max_iter)
+        tol = 1e-11 * np.max(np.abs(want))
+        if it < max_iter:  # the bound of the test above
+            tol += 2 * MDW * (1.0 - 0.5 * M) * sign * np.sqrt(1e-16 * np.linalg.norm(phi[m]))
+        assert np.max(np.abs(out[m].ravel() - want)) < tol, (m, it)
+
+
+@pytest.mark.parametrize("poles", [1, 2, 4, 9, 25])
+def test_cg_workspace_fields(poles):
+    """The work space of a Zolotarev context takes no more fields than the five
+    vectors and the two per pole of separate x_k and p_k: 3 + 2 poles."""
+    import torch
+
+    N, modes = (16, 16, 16), 64
+    kw = dict(N=N, n_modes=modes, precision="fp64", m_fermion=M, m_dw=MDW)
+
+    def taken(**more):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        with Context(**kw, **more) as ctx:
+            ctx.synchronize()
+            return before - torch.cuda.mem_get_info()[0]
+
+    taken(), taken(fermion="overlap", zolo_poles=poles)  # what the first of either loads
+    field = volume(N) * 8 * 16 * modes
+    extra = taken(fermion="overlap", zolo_poles=poles) - taken()
+    # the scalars, the dot products' partial sums (one double per mode and 8 sites, and 128) and
+    # what allocations round up to stay below a field
+    assert extra < (3 + 2 * poles + 1) * field
