@@ -240,6 +240,14 @@ int ovl_zolotarev(double lambda_min, double lambda_max, double tol, int npoles, 
  * the same iteration runs on the three-colour h_W^2, start [V][3][4]). */
 int ovl_ritz_bounds(ovl_ctx *ctx, const double *start, double out[2], double raw[2], int iters[2]);
 
+/* Failure-detection self-test of the Ritz solver's cooperative launch (two
+ * colours, more than 2048 sites, as many as are resident at once): its CTAs
+ * wait for a count that nothing reaches, give up after their bounded wait (1 s)
+ * and the solve is made again by kernels that wait for nothing.  *code =
+ * OVL_E_TIMEOUT when the waits ran out; raw and start as ovl_ritz_bounds.
+ * Other lattices: OVL_E_UNSUPPORTED. */
+int ovl_ritz_selftest(ovl_ctx *ctx, const double *start, double raw[2], int *code);
+
 /* Statistics of the last overlap application.  Zolotarev: out[0] = lockstep
  * CG iterations, out[1] = largest per-mode iteration count, out[2] = modes
  * stopped by cg_max_iter (the reference prints a warning and keeps the

@@ -374,15 +374,25 @@ class Context:
         mode [V, Nc, 4] complex (None: drawn from the context's generator)."""
         out, raw = np.empty(2), np.empty(2)
         it = (C.c_int * 2)()
-        sp = None
-        if start is not None:
-            start = np.ascontiguousarray(start, dtype=np.complex128)
-            if start.size != 4 * self.nc * volume(self.params.N):
-                raise ValueError(f"start must hold one mode (V x {self.nc} x 4 complex)")
-            sp = _dp(start.view(np.float64))
-        self._check(self._L.ovl_ritz_bounds(self._ctx, sp, _dp(out), _dp(raw), it))
+        start = self._ritz_start(start)
+        self._check(self._L.ovl_ritz_bounds(self._ctx, start, _dp(out), _dp(raw), it))
         return {"bounds": (float(out[0]), float(out[1])), "raw": (float(raw[0]), float(raw[1])),
                 "iters": (int(it[0]), int(it[1]))}
+
+    def _ritz_start(self, start):
+        if start is None:
+            return None
+        start = np.ascontiguousarray(start, dtype=np.complex128)
+        if start.size != 4 * self.nc * volume(self.params.N):
+            raise ValueError(f"start must hold one mode (V x {self.nc} x 4 complex)")
+        return _dp(start.view(np.float64))
+
+    def ritz_selftest(self, start: np.ndarray | None = None) -> tuple[int, tuple[float, float]]:
+        """ovl_ritz_selftest: (the status of the waits made to run out, OVL_E_TIMEOUT = 4
+        when they did; the eigenvalues as solved after them)."""
+        raw, code = np.empty(2), C.c_int(0)
+        self._check(self._L.ovl_ritz_selftest(self._ctx, self._ritz_start(start), _dp(raw), C.byref(code)))
+        return code.value, (float(raw[0]), float(raw[1]))
 
     def color_force(self) -> np.ndarray:
         """dH_F/dtheta^a_mu(x) as [V, 3 (mu), Nc^2 - 1 (a)] (Wilson fermions)."""

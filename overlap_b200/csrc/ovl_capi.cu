@@ -200,7 +200,9 @@ double wilson_norm_bound2(const ovl_params &p) {
 // ComputeRitzEigenvalues (OverlapUpdate.cpp:61-97): MinEValue = 0.95 lambda_min,
 // MaxEValue = 1.05 lambda_max, with MaximumIterations 2000, NumberOfRestarts 100,
 // NormRatio 1e-16 (:53-58).
-int ritz_bounds(ovl_ctx *c, const double *start, double out[2], double raw[2], int iters[2]) {
+// stall, expired: ritz_run's self-test.
+int ritz_bounds(ovl_ctx *c, const double *start, double out[2], double raw[2], int iters[2], bool stall = false,
+                bool *expired = nullptr) {
     if (!c->ritz && !(c->ritz = ovl::ritz_create(c->L.V, c->nc))) return fail(c, OVL_E_OOM, "Ritz solver: work space");
     const size_t n = (size_t)c->L.V * 4 * c->nc;
     if (start)
@@ -215,9 +217,11 @@ int ritz_bounds(ovl_ctx *c, const double *start, double out[2], double raw[2], i
     {
         ProfScope ps(c, OVL_PROF_OBS);
         e = ovl::ritz_run(c->ritz, c->U, c->u1_on ? c->u1 : nullptr, c->L, amass(c->p), 2000, 100, 1e-16, r, it,
-                          c->stream, &nl);
+                          c->stream, &nl, stall, expired);
     }
     c->launches += nl;
+    if (e == cudaErrorNotSupported && stall)
+        return fail(c, OVL_E_UNSUPPORTED, "ovl_ritz_selftest: the solve of this lattice has no waits between CTAs");
     if (e != cudaSuccess) return cuda_fail(c, e, "Ritz solver");
     const double lmin = r[0], lmax = -r[1];
     if (!(lmin > 0.0) || !(lmax > lmin) || !std::isfinite(lmax))
@@ -2140,6 +2144,17 @@ int ovl_ritz_bounds(ovl_ctx *c, const double *start, double out[2], double raw[2
     int rc = set_device(c);
     if (rc) return rc;
     return ritz_bounds(c, start, out, raw, iters);
+}
+
+int ovl_ritz_selftest(ovl_ctx *c, const double *start, double raw[2], int *code) {
+    if (!c || !raw || !code) return OVL_E_ARG;
+    int rc = set_device(c);
+    if (rc) return rc;
+    double out[2];
+    bool expired = false;
+    rc = ritz_bounds(c, start, out, raw, nullptr, true, &expired);
+    *code = expired ? OVL_E_TIMEOUT : OVL_OK;
+    return rc;
 }
 
 int ovl_set_spectral_bounds(ovl_ctx *c, const double *pairs, int count) {

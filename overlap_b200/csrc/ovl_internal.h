@@ -155,13 +155,16 @@ void launch_fermion_energy(const void *psi, const void *dpsi, const Lattice &L, 
 // Ritz solver for the overlap spectral bounds (ovl_ritz.cu): work space for a
 // lattice of V sites, the start vector buffer (compact [V][8] double2), a
 // seeded uniform start vector, and the run: out = {lambda_min, -lambda_max}.
+// stall (self-test): the one-launch solve's bounded waits run out before the
+// run; *expired tells whether they did; cudaErrorNotSupported where the solve
+// has no such waits.
 void *ritz_create(int V, int nc);
 void ritz_destroy(void *work);
 double2 *ritz_start_buffer(void *work);
 void launch_ritz_random_start(void *work, uint64_t seed, uint64_t call, cudaStream_t stream);
 cudaError_t ritz_run(void *work, const double *U, const double *u1, const Lattice &L, double amass, int max_iter,
                      int nrestart, double delitr, double out[2], int iters[2], cudaStream_t stream,
-                     uint64_t *launches);
+                     uint64_t *launches, bool stall = false, bool *expired = nullptr);
 // The same observables on 40-bit storage (hi words + extension bytes).
 void launch_currents40(const double *U, const double *u1, const void *hi, const void *lo, const Lattice &L, int n_mb,
                        int n_modes, int first_mode, double r_wilson, double *partial, double *per_site,

@@ -449,7 +449,9 @@ __global__ void __launch_bounds__(kRitzThreads)
 //                problem.  The CTAs wait for one another, so all are resident
 //                and every wait is bounded (1 s of %globaltimer): on expiry the
 //                error word is set, every CTA leaves at its next wait, and the
-//                host reports the solve as failed.
+//                host solves again with the kernels above, which wait for
+//                nothing (the second also passes while the GPU runs another
+//                process's work, so an expired wait is not yet a failed solve).
 // One overlap leapfrog step with its two pairs of bounds at 8^3, 256 modes:
 // 91 ms with six launches per Ritz step, 50 ms with the cooperative launch; then,
 // the CG made faster, 42.9 ms with the cooperative launch and 30.8 ms with
@@ -1186,10 +1188,12 @@ template <bool U1> static RitzPlan ritz_plan(int V) {
     return pl;
 }
 
+// stall: the arrival counters start where no phase's count reaches (the bounded
+// waits of the cooperative launch then run out).
 template <bool U1>
 static cudaError_t ritz_run_one(RitzWork &w, const RitzPlan &pl, const double *U, const double *u1, const Lattice &L,
                                 double amass, int max_iter, int nrestart, double delitr, double out[2], int iters[2],
-                                cudaStream_t stream, uint64_t *launches) {
+                                cudaStream_t stream, uint64_t *launches, bool stall) {
     RitzOne a;
     a.start = w.start;
     a.st = w.st;
@@ -1206,6 +1210,7 @@ static cudaError_t ritz_run_one(RitzWork &w, const RitzPlan &pl, const double *U
     LinksF64<U1> lk{U, reinterpret_cast<const double2 *>(u1), L.N0 * L.N1};
     Lattice lat = L;
     cudaError_t e = cudaMemsetAsync(w.count, 0, sizeof(int) * 3, stream);
+    if (e == cudaSuccess && stall) e = cudaMemsetAsync(w.count, 0x80, sizeof(int) * 2, stream);  // -2.1e9
     if (e != cudaSuccess) return e;
     if (pl.ranks) {
         cudaLaunchAttribute at;
@@ -1226,6 +1231,7 @@ static cudaError_t ritz_run_one(RitzWork &w, const RitzPlan &pl, const double *U
         e = cudaLaunchCooperativeKernel(ritz_grid_kernel<U1>, grid, dim3(2 * kRitzGridSites), args, 0, stream);
     }
     if (e != cudaSuccess) return e;
+    if (launches) *launches += 1;
     int *err = reinterpret_cast<int *>(w.host + 2);
     if ((e = cudaMemcpyAsync(w.host, w.st, 2 * sizeof(RitzScalars), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(err, a.err, sizeof(int), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
@@ -1236,7 +1242,6 @@ static cudaError_t ritz_run_one(RitzWork &w, const RitzPlan &pl, const double *U
         out[k] = w.host[k].xy_re;
         if (iters) iters[k] = w.host[k].ittot;
     }
-    if (launches) *launches += 1;
     return cudaSuccess;
 }
 
@@ -1246,8 +1251,9 @@ static cudaError_t ritz_run_one(RitzWork &w, const RitzPlan &pl, const double *U
 // per problem.  Returns a CUDA error or cudaSuccess; *launches counts kernels.
 cudaError_t ritz_run(void *work, const double *U, const double *u1, const Lattice &L, double amass, int max_iter,
                      int nrestart, double delitr, double out[2], int iters[2], cudaStream_t stream,
-                     uint64_t *launches) {
+                     uint64_t *launches, bool stall, bool *expired) {
     RitzWork &w = *static_cast<RitzWork *>(work);
+    if (stall && w.nc == 3) return cudaErrorNotSupported;
     if (w.nc == 3)
         return ritz_run_nc<3>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
     const int b = u1 ? 1 : 0;
@@ -1255,10 +1261,19 @@ cudaError_t ritz_run(void *work, const double *U, const double *u1, const Lattic
         w.plan[b] = u1 ? ritz_plan<true>(L.V) : ritz_plan<false>(L.V);
         w.planned[b] = true;
     }
-    const RitzPlan &pl = w.plan[b];
-    if (pl.ranks || pl.grid)
-        return u1 ? ritz_run_one<true>(w, pl, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches)
-                  : ritz_run_one<false>(w, pl, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
+    RitzPlan &pl = w.plan[b];
+    if (stall && !pl.grid) return cudaErrorNotSupported;
+    if (pl.ranks || pl.grid) {
+        const cudaError_t e =
+            u1 ? ritz_run_one<true>(w, pl, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches, stall)
+               : ritz_run_one<false>(w, pl, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches, stall);
+        if (expired) *expired = e == cudaErrorLaunchTimeout;
+        if (e == cudaSuccess) return e;
+        // The launch was refused or a wait ran out: from here on kernel by kernel
+        // (an error of the device itself shows up there again).
+        cudaGetLastError();
+        if (!stall) pl = RitzPlan{};
+    }
     return ritz_run_nc<2>(w, U, u1, L, amass, max_iter, nrestart, delitr, out, iters, stream, launches);
 }
 

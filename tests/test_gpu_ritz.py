@@ -93,6 +93,30 @@ def test_ritz_at_the_edges_of_its_launch_shapes(N, u1):
     assert r["raw"] == again["raw"] and r["iters"] == again["iters"]  # fixed summation order
 
 
+def test_ritz_solves_again_when_a_wait_runs_out():
+    """Failure detection without a GPU fault: the cooperative solve's CTAs wait
+    for a count that nothing reaches and give up; the bounds still come out, from
+    the kernels that wait for nothing, and later solves run as before."""
+    from overlap_b200 import OvlError
+
+    N = (13, 13, 13)
+    rng = np.random.default_rng(431)
+    start = rng.uniform(0, 1, (volume(N), 2, 4)) + 1j * rng.uniform(0, 1, (volume(N), 2, 4))
+    with Context(N=N, n_modes=1, fermion="overlap", sign_method="chebyshev", m_fermion=0.05, m_dw=1.4) as ctx:
+        ctx.set_links(random_links(N, 0.3, 421))
+        before = ctx.ritz_bounds(start)
+        code, raw = ctx.ritz_selftest(start)
+        after = ctx.ritz_bounds(start)
+    assert code == 4  # OVL_E_TIMEOUT
+    for k in range(2):  # another summation order, stopped at round-off
+        assert abs(raw[k] - before["raw"][k]) <= 1e-11 * before["raw"][k]
+    assert after == before
+    with Context(N=(4, 4, 4), n_modes=1, fermion="overlap", m_dw=1.4) as ctx:
+        ctx.set_links(random_links((4, 4, 4), 0.3, 1))
+        with pytest.raises(OvlError):  # a cluster: no waits on a count
+            ctx.ritz_selftest()
+
+
 @pytest.mark.skipif(not have_reference("overlap"), reason="reference overlap build not present")
 def test_overlap_leapfrog_with_gpu_ritz_bounds_matches_reference():
     N = (4, 4, 4)
