@@ -9,6 +9,7 @@
 #pragma once
 
 #include "ovl_device.cuh"
+#include "ovl_rules.h"
 
 namespace ovl {
 
@@ -124,33 +125,6 @@ __device__ __forceinline__ Nbrs neighbours(const Lattice &L, int site) {
     return n;
 }
 
-// The six FP64 link matrices of one site's hops, gathered once per CTA in
-// shared memory and reused over the CTA's mode blocks: entries 0..2 the links
-// U_mu(site), 3..5 the links U_mu(site - mu) (the backward hop takes their
-// dagger itself), each as LK delivers it (dressed with the U(1) phase when one
-// is set).  get() is called by the stencil with the site itself for the
-// forward hops and with its backward neighbours, which differ from the site on
-// every lattice the library accepts (N >= 3).
-// Mode blocks per CTA of a stencil launch that gathers its sites' links once per
-// CTA (link tables, packed link records): `tiles` CTAs along the sites, n_mb mode
-// blocks.  kLinkBlocks, halved while the launch would hold fewer than `least`
-// CTAs: then a finer split occupies idle SMs and is worth the extra gathering.
-// Beyond that larger is better, even where the last wave is nearly empty: a
-// context on its own would gain from filling it (FP32 packed kernel, 16^3 x 256
-// modes: 112 us per step with 8, 100 with 4), but several contexts on their own
-// streams fill each other's, and there the gathering costs (the same, three
-// contexts in turn: 80 us with 8, 87 with 2; 8^3 x 1024 modes 39 against 44).
-constexpr int kLinkBlocks = 8;
-inline int mode_blocks_per_cta(int tiles, int n_mb, int least) {
-    int m = kLinkBlocks;
-    while (m > 1 && (long long)tiles * ((n_mb + m - 1) / m) < least) m /= 2;
-    return m;
-}
-// The FP64 stencils, two CTAs of 8 warps per SM: one per SM at least.  (Four per
-// SM, as a first rule had it, gave 1 per CTA at 10 x 13 x 9 x 256 modes, 55 us per
-// step against 47 with 8, and 4 at 1024 modes, 187 us against 184; three
-// contexts in turn.)  1 selects the stencil without the table.
-inline int link_blocks(int site_ctas, int n_mb, int sm_count) { return mode_blocks_per_cta(site_ctas, n_mb, sm_count); }
 // SMs of the current device (cached per device).
 inline int current_sm_count() {
     static int cache[64] = {};
@@ -164,6 +138,13 @@ inline int current_sm_count() {
     return cache[dev];
 }
 
+// The six FP64 link matrices of one site's hops, gathered once per CTA in
+// shared memory and reused over the CTA's mode blocks: entries 0..2 the links
+// U_mu(site), 3..5 the links U_mu(site - mu) (the backward hop takes their
+// dagger itself), each as LK delivers it (dressed with the U(1) phase when one
+// is set).  get() is called by the stencil with the site itself for the
+// forward hops and with its backward neighbours, which differ from the site on
+// every lattice the library accepts (N >= 3).
 struct LinksTable {
     const cmat2<double> *t;
     int site;

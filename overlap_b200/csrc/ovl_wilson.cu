@@ -188,9 +188,11 @@ __global__ void __launch_bounds__(kModeBlock *kPkWarps, kPkMinBlocks)
 // CTAs of the packed launch along the sites, and mode blocks per CTA.
 static int packed_tiles(const Lattice &L) { return (L.V + kPkCtaSites - 1) / kPkCtaSites; }
 static int packed_mblk(const Lattice &L, int n_mb) {
-    // three quarters of a CTA per SM, of the three that run on one: at 8^3 x 256
-    // modes 64 CTAs with 8 took 15.9 us per step, 256 with 2 12.0 (three contexts in
-    // turn); at 12^3 x 256 216 with 8 33.0, 432 with 4 33.6
+    // three quarters of a CTA per SM, of the three that run on one (us per step of a
+    // context on its own / with three in turn): 8^3 x 256 modes 64 CTAs with 8 37/15,
+    // 256 with 2 25/12; 8^3 x 1024 49/36 and 49/40; 12^3 x 512 76/57 and 81/64.  Between
+    // one and four CTAs per SM a context on its own would gain from 2 what several
+    // lose by it: 12^3 x 256 49/29 with 8, 41/33 with 2; 16^3 x 256 113/71 and 94/75.
     return mode_blocks_per_cta(packed_tiles(L), n_mb, 3 * current_sm_count() / 4) == kPkBlocks ? kPkBlocks : kPkFewBlocks;
 }
 
