@@ -638,7 +638,7 @@ def su3_overlap_leg(steps, warmup, device, modes=0):
                       f"{M} plane-wave modes FP32, FP64 links reunitarised, random links sigma 0.5, E sigma 0.1",
             "value": M * V * steps / (ms / 1e3), "unit": METRIC, "steps": steps, "ms_per_step": ms / steps,
             "launches_per_step": launches / steps,
-            "hop_variant": variant,
+            "hop_variant": variant if variant >= 0 else None,  # -1: no hop kernel ran (on chip)
             "overlap_application": {"ms": half_ms, "algorithmic_bytes": alg, "achieved_GBs": alg / (half_ms / 1e3) / 1e9,
                                     "frac_of_peak": alg / (half_ms / 1e3) / 1e9 / peak, "peak_source": peak_kind,
                                     "bytes_as_built": built,

@@ -217,7 +217,8 @@ int ovl_autotune(ovl_ctx *ctx, int *variant, double ms[OVL_HOP_VARIANTS]);
 int ovl_pipeline_selftest(ovl_ctx *ctx, int *code);
 
 /* The hop variant and mode grouping in use (after the autotuner ran, or as
- * set in ovl_params); -1 before either is known. */
+ * set in ovl_params); -1 before either is known, and for the variant while no
+ * hop kernel has run (a three-colour overlap operator held on chip). */
 int ovl_tuning(const ovl_ctx *ctx, int *variant, int *mode_group);
 
 /* Zolotarev coefficients of the overlap sign function for spectral bounds

@@ -289,7 +289,10 @@ int run_overlap(ovl_ctx *c, const void *src, void *dst, int n_mb, int n_modes, b
         double lo, hi;
         int rc = take_bounds(c, consume, lo, hi);
         if (rc) return rc;
-        if (su3(c) && c->hop_variant < 0 && (rc = su3_autotune(c, nullptr))) return rc;
+        // on chip there is no stencil to choose, and the variant stays open
+        if (su3(c) && c->hop_variant < 0 && !ovl::su3_chebyshev_on_chip<float>(c->cw, su3_links(c), c->L, n_mb) &&
+            (rc = su3_autotune(c, nullptr)))
+            return rc;
         ProfScope ps(c, OVL_PROF_HOP);
         uint64_t nl = 0;
         if (su3(c) && fp32(c))
@@ -535,8 +538,8 @@ int autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
 // Three colours, FP32: the scalar stencil (variant 0) against the packed-pair
 // stencil (variant 3), timed on the operator buffer as the context uses the
 // stencil (the fused half step for Wilson contexts; for overlap contexts a
-// Chebyshev series of degree 3, whose D passes and final combination differ
-// between the variants where it goes through memory); the state is not touched.
+// Chebyshev series of degree 3 through memory, whose D passes and final
+// combination differ between the variants); the state is not touched.
 int su3_autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
     if (ms_out)
         for (int v = 0; v < ovl::kHopVariants; v++) ms_out[v] = 0.0;
@@ -552,7 +555,7 @@ int su3_autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
     const double lmax = std::pow(0.5 * std::fabs(amass(c->p)) + 3.0, 2);
     auto run = [&](int k) -> uint64_t {
         lk.variant = cand[k];
-        if (cheb) {  // a Chebyshev series of degree 3 (four terms and the combination), psi -> aux_dst
+        if (cheb) {  // a Chebyshev series of degree 3 (three terms and the combination), psi -> aux_dst
             uint64_t n = 0;
             ovl::su3_chebyshev_apply<float>(c->cw, lk, c->psi, c->aux_dst, c->L, c->n_mb, c->cheb.data(),
                                             std::min(3, c->p.cheb_degree), c->p.cheb_eps, lmax, amass(c->p), c->p.m_dw,
@@ -564,7 +567,10 @@ int su3_autotune(ovl_ctx *c, double ms_out[ovl::kHopVariants]) {
                                    c->stream);
         return 1;
     };
-    if (!time_candidates(c->stream, 2, run, ms, nl)) return fail(c, OVL_E_CUDA, "autotune: events");
+    c->cw.through_memory = true;
+    const bool timed = time_candidates(c->stream, 2, run, ms, nl);
+    c->cw.through_memory = false;
+    if (!timed) return fail(c, OVL_E_CUDA, "autotune: events");
     c->hop_variant = ms[1] < ms[0] ? cand[1] : cand[0];
     if (ms_out) {
         ms_out[0] = ms[0];

@@ -217,8 +217,8 @@ void chebyshev_apply(ChebyshevWork &w, const HopConfig &hc, const void *src, voi
     const int n01 = L.N0 * L.N1;
     auto resident = [&](auto u1, const void *links, const void *phases) {
         auto with = [&](auto... caps) {
-            return resident_apply<2, T, decltype(u1)::value, decltype(caps)...>(
-                w.resident, links, phases, src, dst, L, n_mb, w.b0, coeff, K, eps, lambda_max, amass, mdw, mf, dt,
+            return resident_apply<2, T, decltype(u1)::value>(
+                ResidentCaps<decltype(caps)...>{}, w.resident, links, phases, src, dst, L, n_mb, w.b0, coeff, K, eps, lambda_max, amass, mdw, mf, dt,
                 accumulate, stream, launches);
         };
         if constexpr (sizeof(T) == 4) return with(ResidentCap<LanePair, 512>{});

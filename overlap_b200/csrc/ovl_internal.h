@@ -308,6 +308,7 @@ struct ResidentPlan {
 struct ChebyshevWork {
     void *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *w = nullptr;
     ResidentPlan resident;
+    bool through_memory = false;  // leave the plan aside (timing the kernels that go through memory)
 };
 // The overlap operator with the Chebyshev series on all mode blocks; FP32 modes
 // take the FP32 link copy when hc.U32 is set.
@@ -348,6 +349,9 @@ template <typename T>
 void su3_chebyshev_apply(ChebyshevWork &w, const Su3Links &lk, const void *src, void *dst, const Lattice &L, int n_mb,
                          const double *coeff, int K, double eps, double lambda_max, double amass, double mdw, double mf,
                          double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches);
+// Whether that runs on chip (ovl_resident.cuh), where lk.variant plays no part.
+template <typename T>
+bool su3_chebyshev_on_chip(ChebyshevWork &w, const Su3Links &lk, const Lattice &L, int n_mb);
 // The charges and the per-site Wilson currents of three-colour modes (ovl_modes.cu; scratch sizes as for two).
 template <typename T>
 void su3_launch_currents(const double *U, const double *u1, const void *psi, const Lattice &L, int n_mb, int n_modes,

@@ -609,13 +609,12 @@ static cudaError_t resident_launch(const ResidentPlan &pl, const ResidentArgs<ty
     return cudaLaunchKernelEx(&cfg, resident_cheb_kernel<NC, typename Cap::Lane, U1, false, Cap::kCap>, a);
 }
 
-// The operator on chip, if the lattice fits with one of the capacities.  The
-// plan is the context's: it holds sizes only, and is made again when they change.
-template <int NC, typename T, bool U1, class... Caps>
-static bool resident_apply(ResidentPlan &pl, const void *U, const void *u1, const void *src, void *dst, const Lattice &L,
-                           int n_mb, void *scratch, const double *coeff, int K, double eps, double lambda_max,
-                           double amass, double mdw, double mf, double dt, bool accumulate, cudaStream_t stream,
-                           uint64_t *launches) {
+template <class... Caps> struct ResidentCaps {};
+
+// The plan for n_mb mode blocks with one of the capacities.  It is the context's:
+// it holds sizes only, and is made again when they change.  Whether there is one.
+template <int NC, bool U1, class... Caps>
+static bool resident_plan(ResidentCaps<Caps...>, ResidentPlan &pl, const Lattice &L, int n_mb) {
     const int modes = n_mb * kModeBlock;
     if (pl.modes != modes || pl.u1 != U1) {
         pl = ResidentPlan{};
@@ -624,7 +623,17 @@ static bool resident_apply(ResidentPlan &pl, const void *U, const void *u1, cons
         int i = 0;
         (resident_offer<NC, U1, Caps>(L, i++, modes, pl), ...);
     }
-    if (!pl.ok) return false;
+    return pl.ok;
+}
+
+// The operator on chip, if there is a plan for it.
+template <int NC, typename T, bool U1, class... Caps>
+static bool resident_apply(ResidentCaps<Caps...> caps, ResidentPlan &pl, const void *U, const void *u1, const void *src,
+                           void *dst, const Lattice &L, int n_mb, void *scratch, const double *coeff, int K, double eps,
+                           double lambda_max, double amass, double mdw, double mf, double dt, bool accumulate,
+                           cudaStream_t stream, uint64_t *launches) {
+    const int modes = n_mb * kModeBlock;
+    if (!resident_plan<NC, U1>(caps, pl, L, n_mb)) return false;
     ResidentArgs<T> a;
     a.U = U;
     a.u1 = u1;

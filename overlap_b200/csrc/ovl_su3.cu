@@ -189,12 +189,23 @@ __global__ void su3_overlap_finish_kernel(const cpx<T> *__restrict__ phi, const 
     }
 }
 
+template <typename T>
+using Caps3 = ResidentCaps<ResidentCap<LaneOne<T>, sizeof(T) == 4 ? 512 : 256>, ResidentCap<LaneOne<T>, sizeof(T) == 4 ? 576 : 224>>;
+
+template <typename T>
+bool su3_chebyshev_on_chip(ChebyshevWork &w, const Su3Links &lk, const Lattice &L, int n_mb) {
+    const bool u1 = sizeof(T) == 4 ? lk.u1_32 != nullptr : lk.u1 != nullptr;
+    return u1 ? resident_plan<3, true>(Caps3<T>{}, w.resident, L, n_mb) : resident_plan<3, false>(Caps3<T>{}, w.resident, L, n_mb);
+}
+template bool su3_chebyshev_on_chip<float>(ChebyshevWork &, const Su3Links &, const Lattice &, int);
+
 template <typename T, bool F32, bool U1>
 static void cheb3(ChebyshevWork &w, const Su3Links &lk, const void *src, void *dst, const Lattice &L, int n_mb,
                   const double *coeff, int K, double eps, double lambda_max, double amass, double mdw, double mf,
                   double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches) {
-    if (resident_apply<3, T, U1, ResidentCap<LaneOne<T>, F32 ? 512 : 256>, ResidentCap<LaneOne<T>, F32 ? 576 : 224>>(
-            w.resident, F32 ? (const void *)lk.U32 : (const void *)lk.U, F32 ? (const void *)lk.u1_32 : (const void *)lk.u1,
+    if (!w.through_memory &&
+        resident_apply<3, T, U1>(
+            Caps3<T>{}, w.resident, F32 ? (const void *)lk.U32 : (const void *)lk.U, F32 ? (const void *)lk.u1_32 : (const void *)lk.u1,
             src, dst, L, n_mb, w.b0, coeff, K, eps, lambda_max, amass, mdw, mf, dt, accumulate, stream, launches))
         return;
     const size_t n = (size_t)n_mb * L.V * kComp3 * kModeBlock;

@@ -320,6 +320,22 @@ def test_autotune_chooses_between_the_three_colour_stencils(fermion):
         assert v == 0
 
 
+def test_on_chip_overlap_operator_times_no_stencil():
+    """Where the FP32 Chebyshev operator of a context runs on chip its first
+    application launches that operator only, and the hop variant stays open; a
+    plane too large for a CTA goes through memory and tunes between the stencils."""
+    for shape, modes, on_chip in (((4, 4, 4), 64, True), ((25, 24, 3), 32, False)):
+        V = int(np.prod(shape))
+        kw = dict(_overlap_kw("fp32"), N=shape, n_modes=modes, n_colours=3, cheb_degree=24)
+        with Context(**kw) as ctx:
+            ctx.set_links(random_links_su3(shape, 0.5, 41))
+            before = ctx.launch_count
+            ctx.apply(np.ones((modes, V, 3, 4), complex))
+            launches = ctx.launch_count - before
+            assert (ctx.tuning()[0] == -1) == on_chip
+            assert (launches < 24) == on_chip, launches
+
+
 def test_three_colour_limits_are_reported():
     for kw in (dict(precision="fp40"), dict(fermion="overlap", sign_method="zolotarev"), dict(n_colours=4)):
         with pytest.raises(OvlError):
