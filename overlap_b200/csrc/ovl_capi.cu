@@ -290,7 +290,7 @@ int run_overlap(ovl_ctx *c, const void *src, void *dst, int n_mb, int n_modes, b
         int rc = take_bounds(c, consume, lo, hi);
         if (rc) return rc;
         // on chip there is no stencil to choose, and the variant stays open
-        if (su3(c) && c->hop_variant < 0 && !ovl::su3_chebyshev_on_chip<float>(c->cw, su3_links(c), c->L, n_mb) &&
+        if (su3(c) && c->hop_variant < 0 && !ovl::su3_chebyshev_on_chip<float>(c->cw, su3_links(c), c->L, n_mb, c->p.cheb_degree) &&
             (rc = su3_autotune(c, nullptr)))
             return rc;
         ProfScope ps(c, OVL_PROF_HOP);

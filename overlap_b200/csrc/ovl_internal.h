@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "ovl_rules.h"
+
 namespace ovl {
 
 struct Lattice;
@@ -288,20 +290,15 @@ void overlap_apply(OverlapWork &w, const double *U, const double *u1, const void
 // Chebyshev form of the overlap sign function (ovl_chebyshev.cu).
 constexpr int kMaxChebDegree = 1024;
 void chebyshev_inverse_sqrt(int K, double eps, double *c);
-struct ResidentShape {
-    int planes;  // per CTA (the last CTA of a cluster may hold fewer)
-    int groups;  // sets of modes per cluster: a CTA has groups x sites threads
-    int ranks;   // CTAs per cluster
-};
 
-// How a lattice is laid out on the chip, if it fits at all.
+// How a lattice is laid out on the chip, if that is the better place for it.
 struct ResidentPlan {
     bool ok = false, u1 = false;
-    int modes = 0;          // the plan is for this many (0: none made yet)
-    int kernel = 0;         // index of the capacity
+    int modes = 0, degree = 0;  // the plan is for these (0: none made yet)
+    int kernel = 0;             // index of the capacity
     ResidentShape sh{};
     size_t smem = 0;
-    double rate = 0.0;      // what it was chosen by
+    double us = 0.0;            // the time it was chosen by
 };
 // Clenshaw vectors b0, b1, b2 and the temporary w = D b (one field each, mode
 // precision).
@@ -351,7 +348,7 @@ void su3_chebyshev_apply(ChebyshevWork &w, const Su3Links &lk, const void *src, 
                          double dt, bool accumulate, int sm_count, cudaStream_t stream, uint64_t *launches);
 // Whether that runs on chip (ovl_resident.cuh), where lk.variant plays no part.
 template <typename T>
-bool su3_chebyshev_on_chip(ChebyshevWork &w, const Su3Links &lk, const Lattice &L, int n_mb);
+bool su3_chebyshev_on_chip(ChebyshevWork &w, const Su3Links &lk, const Lattice &L, int n_mb, int degree);
 // The charges and the per-site Wilson currents of three-colour modes (ovl_modes.cu; scratch sizes as for two).
 template <typename T>
 void su3_launch_currents(const double *U, const double *u1, const void *psi, const Lattice &L, int n_mb, int n_modes,

@@ -28,6 +28,7 @@
 #include <cooperative_groups.h>
 
 #include "ovl_internal.h"
+#include "ovl_rules.h"
 #include "ovl_stencil.cuh"
 #include "ovl_su3.cuh"
 
@@ -515,81 +516,65 @@ template <class LN, int CAP> struct ResidentCap {
     static constexpr int kCap = CAP;
 };
 
-constexpr int kResMaxRanks = 8;  // the portable cluster size
 // Whole warps (capacities are multiples of 32).
 inline int resident_threads(int n) { return (n + 31) / 32 * 32; }
 
-// Offers capacity number `index` to the plan: takes the split into planes of the
-// largest rate.  The rate is share x t / (t + 300), where share is the part of the
-// SMs at work (clusters of six and more CTAs leave a tenth to a third of them
-// without one, and the planes may fall unevenly on a cluster's CTAs) and t the
-// modes x sites of a CTA: its threads hide the latencies of a phase.  The outer
-// planes of the CTAs of a cluster cost planes / (planes + 1/4) for two colours and
-// planes / (planes + 1/2) for three.  One set of modes per CTA (no two threads share
-// the reads of a link) counts 0.9 in a cluster for two colours, 0.9 alone and 0.8 in
-// a cluster for three, 0.75 on rows of less than eight sites, which also meet in
-// the banks where they wrap.  For three colours more than 512 threads count 0.85
-// (their 96 registers spill).  E.g. 10^3, three colours, 512 FP32 modes: 11.3 ms on
-// 2 CTAs of 5 planes, 12.6 on 5 of 2; 12 x 12 x 6: 4.0 on 3 CTAs of 2 planes and
-// two sets, 4.6 on 2 of 3 and one; 6 x 10 x 15, two colours, FP64: 4.2 on 5 of 3 and
-// two sets, 5.1 on 3 of 5 and one.
-// Whether the chip is the better place at all, measured over 26 lattices of 4 to 16
-// sites a side and degree 24, times through memory / times here.  Two colours:
-// 1.04 to 2.4 from a share of 0.76; 0.98 (14^3, FP32) and 0.94 (13^3, FP64) at 0.71
-// and 0.66; hence 0.75.  Three colours, whose links cost as much to read as the
-// spinors of one mode: FP32 1.03 to 1.8 from a share of 0.87, 0.67 to 1.02 below
-// and for three and more CTAs with one set of modes; FP64 0.97 to 2.0 from 0.81
-// with up to three CTAs of 180 threads and more, 0.78 to 1.1 otherwise.
+// Offers capacity number `index` to the plan: the shape of the least time
+// (resident_choose, ovl_rules.h), if it is less than the plan's so far, which
+// starts at the time through memory.
+// Per application at degree 24, through memory / here (us): 8^3, two colours, FP32,
+// 32, 256, 1024 and 4096 modes 306/100, 406/158, 1250/590 and 4220/2160; 5^3 x 64
+// 305/58 (one set of modes in each of 32 CTAs; 147 with four in each of 8);
+// 12 x 11 x 10 x 2048 5440 through memory, which is taken, 6240 here; 8^3, three
+// colours, FP64, 1024: 3500/2810 with two sets on 4 CTAs of 2 planes, 3760 with one on
+// 3 of 3.
+// Over 597 calls (51 pairs of lattice and storage, 32 to 4096 modes, degrees 24 and
+// 96) the choice takes 0.5 to 2 % (geometric mean) more than the best of all shapes
+// and memory, 18 calls over 3 % more than memory, none over 13 %.  A plan for the
+// largest throughput whatever the number of modes took 12 to 17 % more than this one,
+// 45 calls over 2 % and up to 23 % more than memory.  The 224 threads of three colours
+// in FP64 hold planes of 110 to 112 sites in pairs or two sets of modes, which 256 do
+// not: 8 x 14 x 6 x 4096 at degree 96 58.2 ms, 76.0 through memory.
 template <int NC, bool U1, class Cap>
-static void resident_offer(const Lattice &L, int index, int modes, ResidentPlan &pl) {
-    const int n01 = L.N0 * L.N1, slots = modes / Cap::Lane::kModes, sms = current_sm_count();
-    constexpr bool F64 = sizeof(typename Cap::Lane::T) == 8;
+static void resident_offer(const Lattice &L, int index, int modes, int degree, ResidentPlan &pl) {
+    using Lane = typename Cap::Lane;
+    const int n01 = L.N0 * L.N1;
+    const ResidentCall call{NC, sizeof(typename Lane::T) == 8, L.N0, L.N1, L.N2, modes / Lane::kModes, degree};
+    const void *kernels[2] = {(const void *)resident_cheb_kernel<NC, Lane, U1, false, Cap::kCap>,
+                              (const void *)resident_cheb_kernel<NC, Lane, U1, true, Cap::kCap>};
     int dev = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    bool able = cudaGetDevice(&dev) == cudaSuccess &&
+                cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess;
+    for (const void *fn : kernels)
+        able = able && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess;
+    if (!able) {
         cudaGetLastError();
         return;
     }
-    for (int planes = L.N2; planes >= 1; planes--) {
-        const int S = n01 * planes;
-        if (S > Cap::kCap) continue;
-        const ResidentShape sh{planes, std::min(Cap::kCap / S, slots), (L.N2 + planes - 1) / planes};
-        if (sh.ranks > kResMaxRanks) break;
-        const size_t smem = ResidentLayout<NC, typename Cap::Lane>::bytes(Cap::kCap, sh, n01);
-        if (smem > (size_t)optin) continue;
-        const void *fn = sh.ranks > 1 ? (const void *)resident_cheb_kernel<NC, typename Cap::Lane, U1, true, Cap::kCap>
-                                      : (const void *)resident_cheb_kernel<NC, typename Cap::Lane, U1, false, Cap::kCap>;
+    auto fits = [&](const ResidentShape &sh) {
+        const size_t smem = ResidentLayout<NC, Lane>::bytes(Cap::kCap, sh, n01);
+        if (smem > (size_t)optin) return 0;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = sh.ranks;
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sh.ranks);
-        cfg.blockDim = dim3(resident_threads(S * sh.groups));
+        cfg.blockDim = dim3(resident_threads(n01 * sh.planes * sh.groups));
         cfg.dynamicSmemBytes = smem;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernels[sh.ranks > 1], &cfg) != cudaSuccess) {
             cudaGetLastError();
-            continue;
+            return 0;
         }
-        const double share = (double)clusters * L.N2 / ((double)planes * sms);
-        if (share < (NC == 2 ? 0.75 : F64 ? 0.8 : 0.85)) continue;
-        if (NC == 3 && (F64 ? sh.ranks > 3 || S * sh.groups < 180 : sh.ranks > 2 && sh.groups < 2)) continue;
-        const double t = (double)S * sh.groups * Cap::Lane::kModes;
-        double rate = share * t / (t + 300.0);
-        if (sh.ranks > 1) rate *= planes / (planes + (NC == 2 ? 0.25 : 0.5));
-        if (sh.groups < 2) rate *= NC == 2 ? (sh.ranks > 1 ? 0.9 : 1.0) : (L.N0 < 8 ? 0.75 : sh.ranks > 1 ? 0.8 : 0.9);
-        if (NC == 3 && Cap::kCap > 512) rate *= 0.85;
-        if (rate <= pl.rate * 1.0001) continue;
-        pl.ok = true;
-        pl.kernel = index;
-        pl.sh = sh;
-        pl.smem = smem;
-        pl.rate = rate;
-    }
+        return clusters;
+    };
+    if (!resident_choose(call, Cap::kCap, current_sm_count(), fits, pl.sh, pl.us)) return;
+    pl.ok = true;
+    pl.kernel = index;
+    pl.smem = ResidentLayout<NC, Lane>::bytes(Cap::kCap, pl.sh, n01);
 }
 
 template <int NC, bool U1, class Cap>
@@ -611,17 +596,21 @@ static cudaError_t resident_launch(const ResidentPlan &pl, const ResidentArgs<ty
 
 template <class... Caps> struct ResidentCaps {};
 
-// The plan for n_mb mode blocks with one of the capacities.  It is the context's:
-// it holds sizes only, and is made again when they change.  Whether there is one.
-template <int NC, bool U1, class... Caps>
-static bool resident_plan(ResidentCaps<Caps...>, ResidentPlan &pl, const Lattice &L, int n_mb) {
+// The plan for n_mb mode blocks and a series of this degree with one of the
+// capacities.  It is the context's: it holds sizes only, and is made again when they
+// change.  Whether there is one.
+template <int NC, typename T, bool U1, class... Caps>
+static bool resident_plan(ResidentCaps<Caps...>, ResidentPlan &pl, const Lattice &L, int n_mb, int degree) {
     const int modes = n_mb * kModeBlock;
-    if (pl.modes != modes || pl.u1 != U1) {
+    if (pl.modes != modes || pl.degree != degree || pl.u1 != U1) {
         pl = ResidentPlan{};
         pl.modes = modes;
+        pl.degree = degree;
         pl.u1 = U1;
+        const ResidentCall call{NC, sizeof(T) == 8, L.N0, L.N1, L.N2, modes, degree};
+        pl.us = through_memory_us(call, sizeof(cpx<T>) * NC * kSpin * (double)L.V * modes);
         int i = 0;
-        (resident_offer<NC, U1, Caps>(L, i++, modes, pl), ...);
+        (resident_offer<NC, U1, Caps>(L, i++, modes, degree, pl), ...);
     }
     return pl.ok;
 }
@@ -633,7 +622,7 @@ static bool resident_apply(ResidentCaps<Caps...> caps, ResidentPlan &pl, const v
                            double lambda_max, double amass, double mdw, double mf, double dt, bool accumulate,
                            cudaStream_t stream, uint64_t *launches) {
     const int modes = n_mb * kModeBlock;
-    if (!resident_plan<NC, U1>(caps, pl, L, n_mb)) return false;
+    if (!resident_plan<NC, T, U1>(caps, pl, L, n_mb, K)) return false;
     ResidentArgs<T> a;
     a.U = U;
     a.u1 = u1;

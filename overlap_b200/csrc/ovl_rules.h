@@ -55,4 +55,84 @@ inline int link_blocks(int site_ctas, int n_mb, int sm_count) {
     return 1;
 }
 
+// ------------------------------------ the Chebyshev overlap operator on chip --
+// How ovl_resident.cuh lays a lattice out: a cluster of `ranks` CTAs with `planes`
+// z planes each (the last CTA may hold fewer), `groups` sets of modes per cluster; a CTA
+// has groups x sites threads.
+struct ResidentShape {
+    int planes, groups, ranks;
+};
+
+constexpr int kResMaxRanks = 8;  // the portable cluster size
+
+// A call: colours, FP64 or FP32, the lattice, the sets of modes (modes / modes per
+// thread), the degree of the series.
+struct ResidentCall {
+    int nc;
+    bool f64;
+    int N0, N1, N2, slots, degree;
+};
+
+// The time of the operator on chip, in us: clusters at a time on the GPU's sms
+// SMs, waves of them, degree + 4 terms each (the links and phi laid out first and the
+// combination at the end take as long as four).  A term of two phases takes a
+// barrier of the CTA or the cluster and a time per thread on the SM, and more where
+// every CTA hands its outer planes on, where the rows of a plane do not fill 8 lanes
+// (bank conflicts where they wrap), where no two threads share the reads of a link,
+// and with more than 512 threads of three colours (96 registers, spilling).
+// Fitted to 7829 timings (51 pairs of lattice and storage, 4 to 32 sites a side, 32 to
+// 4096 modes, degrees 24 and 96): 5 to 8 % rms, 9 to 16 % at the 95th percentile.
+inline double resident_term_us(const ResidentCall &c, const ResidentShape &sh, int cap, long long ctas_per_sm) {
+    struct Times { double one, one_thread, many, many_thread; };  // us per term: one CTA, several
+    const Times t = c.nc == 2 ? (c.f64 ? Times{0.40, 0.0100, 1.52, 0.0088} : Times{0.50, 0.0089, 1.87, 0.0085})
+                              : (c.f64 ? Times{0.95, 0.0178, 2.47, 0.0151} : Times{1.12, 0.0088, 2.38, 0.0077});
+    const double threads = (double)c.N0 * c.N1 * sh.planes * sh.groups * ctas_per_sm;
+    double term = sh.ranks == 1 ? t.one + t.one_thread * threads
+                                : (t.many + t.many_thread * threads) * (1.0 + 0.12 / sh.planes);
+    if ((c.N0 * sh.groups) % 8 != 0) term *= 1.11;
+    if (sh.groups == 1) term *= 1.09;
+    if (c.nc == 3 && cap > 512) term *= 1.14;
+    return term;
+}
+inline double resident_us(const ResidentCall &c, const ResidentShape &sh, int cap, int clusters, int sms) {
+    const long long need = (c.slots + sh.groups - 1) / sh.groups, waves = (need + clusters - 1) / clusters;
+    const long long ctas_per_sm = (std::min<long long>(need, clusters) * sh.ranks + sms - 1) / sms;
+    return (double)waves * (c.degree + 4) * resident_term_us(c, sh, cap, ctas_per_sm);
+}
+
+// The time of the kernels that go through memory, in us: two launches a term, no
+// faster than 12.3 us, that move seven fields at the rate they reach beyond L2.
+inline double through_memory_us(const ResidentCall &c, double field_bytes) {
+    const double rate = c.f64 ? 4.9e6 : 5.2e6;  // bytes per us
+    return (c.degree + 0.6) * std::max(12.3, 3.5 + 7.0 * field_bytes / rate);
+}
+
+// The best shape for CTAs of `cap` threads, if it takes less than `best` us: then
+// shape and best are set.  fits(shape) is the number of clusters that run at a time
+// (0: it does not fit; never more than two CTAs per SM), asked only where the
+// answer could matter.
+template <class Fits>
+inline bool resident_choose(const ResidentCall &c, int cap, int sms, const Fits &fits, ResidentShape &shape, double &best) {
+    bool found = false;
+    for (int ranks = 1; ranks <= std::min(kResMaxRanks, c.N2); ranks++) {
+        const int planes = (c.N2 + ranks - 1) / ranks;
+        const long long sites = (long long)c.N0 * c.N1 * planes;
+        if ((c.N2 + planes - 1) / planes != ranks || sites > cap) continue;
+        for (int groups = 1; groups <= std::min<long long>(cap / sites, c.slots); groups++) {
+            const ResidentShape sh{planes, groups, ranks};
+            // no less than this, two CTAs per SM that do not slow each other
+            const int most = std::max(1, 2 * sms / ranks), need = (c.slots + groups - 1) / groups;
+            if ((double)((need + most - 1) / most) * (c.degree + 4) * resident_term_us(c, sh, cap, 1) >= best) continue;
+            const int clusters = fits(sh);
+            if (clusters < 1) continue;
+            const double us = resident_us(c, sh, cap, clusters, sms);
+            if (us >= best) continue;
+            best = us;
+            shape = sh;
+            found = true;
+        }
+    }
+    return found;
+}
+
 }  // namespace ovl

@@ -193,11 +193,12 @@ template <typename T>
 using Caps3 = ResidentCaps<ResidentCap<LaneOne<T>, sizeof(T) == 4 ? 512 : 256>, ResidentCap<LaneOne<T>, sizeof(T) == 4 ? 576 : 224>>;
 
 template <typename T>
-bool su3_chebyshev_on_chip(ChebyshevWork &w, const Su3Links &lk, const Lattice &L, int n_mb) {
+bool su3_chebyshev_on_chip(ChebyshevWork &w, const Su3Links &lk, const Lattice &L, int n_mb, int degree) {
     const bool u1 = sizeof(T) == 4 ? lk.u1_32 != nullptr : lk.u1 != nullptr;
-    return u1 ? resident_plan<3, true>(Caps3<T>{}, w.resident, L, n_mb) : resident_plan<3, false>(Caps3<T>{}, w.resident, L, n_mb);
+    return u1 ? resident_plan<3, T, true>(Caps3<T>{}, w.resident, L, n_mb, degree)
+              : resident_plan<3, T, false>(Caps3<T>{}, w.resident, L, n_mb, degree);
 }
-template bool su3_chebyshev_on_chip<float>(ChebyshevWork &, const Su3Links &, const Lattice &, int);
+template bool su3_chebyshev_on_chip<float>(ChebyshevWork &, const Su3Links &, const Lattice &, int, int);
 
 template <typename T, bool F32, bool U1>
 static void cheb3(ChebyshevWork &w, const Su3Links &lk, const void *src, void *dst, const Lattice &L, int n_mb,
