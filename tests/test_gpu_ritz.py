@@ -63,7 +63,9 @@ def test_ritz_random_start_and_u1_background_match_oracle():
 # One-launch solves: clusters of 8 CTAs (64 and 990 sites, the second not filling
 # its CTAs) and of 16 (1716), the cooperative launch (2197), and the iteration
 # kernel by kernel (9600 sites, more than fit the GPU at once; the largest
-# eigenvalue only, the smallest takes the CPU half a minute).
+# eigenvalue only, the smallest takes the CPU half a minute).  The launches tell
+# one-launch solves from the others; that 2197 sites take the cooperative one is
+# what test_ritz_solves_again_when_a_wait_runs_out depends on.
 @pytest.mark.parametrize("N, u1", [((4, 4, 4), True), ((9, 11, 10), False), ((11, 12, 13), True), ((13, 13, 13), False),
                                    ((24, 20, 20), False)])
 def test_ritz_at_the_edges_of_its_launch_shapes(N, u1):
@@ -85,8 +87,11 @@ def test_ritz_at_the_edges_of_its_launch_shapes(N, u1):
     with Context(N=N, n_modes=1, fermion="overlap", sign_method="chebyshev", m_fermion=0.05, m_dw=1.4) as ctx:
         ctx.set_links(U)
         ctx.set_u1(ph)
+        before = ctx.launch_count
         r = ctx.ritz_bounds(start)
+        launches = ctx.launch_count - before
         again = ctx.ritz_bounds(start)
+    assert launches == 1 if V < 9000 else launches > 6 * max(r["iters"]), launches
     # the iteration stops at round-off (the start-vector independence of the test above)
     assert abs(r["raw"][1] - hi) <= 1e-11 * hi
     assert lo is None or abs(r["raw"][0] - lo) <= 1e-11 * lo
