@@ -48,7 +48,8 @@ def rules(tmp_path_factory):
 # context on its own as well as for several in turn
 @pytest.mark.parametrize("N,modes,m", [
     ((12, 12, 12), 128, 1), ((12, 12, 12), 256, 2), ((12, 12, 12), 512, 4), ((6, 6, 6), 1024, 1), ((6, 6, 6), 4096, 4),
-    ((8, 8, 8), 256, 2), ((8, 8, 8), 1024, 8), ((8, 8, 8), 2048, 4), ((8, 8, 8), 4096, 8), ((10, 13, 9), 512, 8)])
+    ((8, 8, 8), 256, 2), ((8, 8, 8), 1024, 8), ((8, 8, 8), 2048, 4), ((8, 8, 8), 4096, 8), ((10, 13, 9), 512, 8),
+    ((16, 16, 16), 64, 1), ((13, 11, 12), 96, 1)])
 def test_mode_blocks_per_cta_of_the_link_table_stencils(rules, N, modes, m):
     sites = (N[0] * N[1] * N[2] + 7) // 8
     assert rules.link(sites, modes // 32, SMS) == m
@@ -64,7 +65,7 @@ def test_mode_blocks_per_cta_over_all_sizes(rules):
 
             def load(k):
                 on = -(-sites * -(-n // k) // SMS)
-                return min(k, n) * (on + (0.5 if on % 2 else 0.0))
+                return min(k, n) * (on + (0.5 if k > 1 and on % 2 else 0.0))
 
             # the gathering counts for 0.15 of a block per CTA: at most 15 % between two choices
             assert load(m) <= 1.06 * 1.15 * min(load(k) for k in (1, 2, 4, 8)) + 1e-9, (sites, n, m)
