@@ -945,10 +945,10 @@ int ovl_set_links(ovl_ctx *c, const double *links) {
 // n doubles of device memory into host memory, waited for.  To pageable memory
 // through the context's page-locked buffer where that is faster than the driver's
 // own staging, which costs tens of microseconds a call: 49 KB 15 against 18 us,
-// 393 KB 35 against 42, 1.3 MB 97 against 110, but 3.1 MB 258 against 203 (the copy
-// out of the buffer).  A caller that reads the buffer itself (where) skips that copy,
+// 393 KB 35 against 42, 1.0 MB 84 against 93, 1.3 MB the same, 3.1 MB 258 against 203
+// (the copy out of the buffer).  A caller that reads the buffer itself (where) skips that copy,
 // so all that fits goes through it.  To page-locked memory directly (3.1 MB: 67 us).
-constexpr size_t kBounceCopyBytes = (size_t)3 << 19;
+constexpr size_t kBounceCopyBytes = (size_t)5 << 18;
 static int download(ovl_ctx *c, const double *dev, size_t n, double *host, const double **where = nullptr) {
     const size_t bytes = sizeof(double) * n;
     const bool bounce = bytes <= c->bounce_bytes && (where || (bytes <= kBounceCopyBytes && !page_locked(host)));

@@ -137,7 +137,7 @@ def test_downloads_to_page_locked_and_pageable_memory():
 
     import torch
 
-    for N in ((5, 6, 7), (26, 25, 24), (32, 32, 32)):  # 20 KB, 1.5 and 3.1 MB of links
+    for N in ((5, 6, 7), (22, 22, 22), (26, 25, 24), (32, 32, 32)):  # 20 KB, 1.0, 1.5 and 3.1 MB of links
         U, E = random_links(N, 0.3, 71), random_efield(N, 0.2, 72)
         with Context(N=N, n_modes=1, precision="fp64", form="fused") as ctx:
             ctx.set_links(U)
